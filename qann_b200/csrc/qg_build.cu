@@ -31,13 +31,43 @@ __global__ void k_row_argmin(const float* __restrict__ scores, size_t ld, int nr
     if (lane == 0) out[warp] = static_cast<uint32_t>(best);
 }
 
+__global__ void k_scatter_u32(const uint32_t* __restrict__ src, const uint32_t* __restrict__ at, size_t n,
+                              uint32_t* __restrict__ out) {
+    const size_t t = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (t < n) out[at[t]] = src[t];
+}
+
+// The rows tile_nearest could not settle, by the exact tiles.
+static void redo_nearest(const float* x_dev, const DevBuf<uint32_t>& redo, size_t m, const float* c_dev, size_t k,
+                         int dim, uint32_t* out_dev, cudaStream_t st) {
+    DevBuf<float> rows(m * dim, st);
+    gather_rows(x_dev, redo.get(), m, dim, rows.get(), st);
+    DevBuf<uint64_t> key(m, st);
+    DevBuf<uint32_t> slot(m, st);
+    // the smallest (score, centroid): the same first-index-on-ties rule
+    flat_candidates(rows.get(), m, c_dev, k, dim, false, 1, nullptr, nullptr, key.get(), slot.get(), st,
+                    /*allow_mm=*/false);
+    k_scatter_u32<<<static_cast<unsigned>(ceil_div(m, 256)), 256, 0, st>>>(slot.get(), redo.get(), m, out_dev);
+    QG_LAUNCH_CHECK();
+}
+
 void assign_nearest(const float* x_dev, size_t n, const float* c_dev, size_t k, int dim, uint32_t* out_dev,
-                    cudaStream_t st) {
+                    cudaStream_t st, const TileQueries* xq) {
     if (n == 0) return;
-    if (use_tensor_filter(n, k, dim, 1)) {
-        // the smallest (score, centroid): the same first-index-on-ties rule
-        DevBuf<uint64_t> key(n, st);
-        flat_candidates(x_dev, n, c_dev, k, dim, false, 1, nullptr, nullptr, key.get(), out_dev, st);
+    if (use_tensor_nearest(n, k, dim)) {
+        TileBase cent;
+        tile_prepare_base(c_dev, k, dim, cent, st);
+        DevBuf<uint32_t> redo;
+        // rows prepared a block at a time unless the caller has them
+        const size_t step = xq ? n : size_t{1} << 20;
+        for (size_t r0 = 0; r0 < n; r0 += step) {
+            const size_t nr = std::min(step, n - r0);
+            TileQueries own;
+            if (!xq) tile_prepare_queries(x_dev + r0 * dim, nr, dim, own, st);
+            const size_t m = tile_nearest(x_dev + r0 * dim, xq ? *xq : own, c_dev, cent, out_dev + r0, redo, st);
+            count_tensor_filter(static_cast<int64_t>(nr), static_cast<int64_t>(m));
+            if (m) redo_nearest(x_dev + r0 * dim, redo, m, c_dev, k, dim, out_dev + r0, st);
+        }
         return;
     }
     const size_t T = std::max<size_t>(1, std::min<size_t>(n, (size_t{512} << 20) / (k * sizeof(float))));

@@ -625,9 +625,11 @@ int qg_set_option(const char* key, int64_t value) {
         } else if (k == "filter_autotune") {
             require(value == 0 || value == 1, "filter_autotune must be 0 or 1");
             set_filter_autotune(static_cast<int>(value));
+            set_tile_autotune(static_cast<int>(value));
         } else if (k == "filter_epilogue_warps") {
             require(value == 0 || value == 8 || value == 16, "filter_epilogue_warps must be 0, 8 or 16");
             set_filter_epilogue_warps(static_cast<int>(value));
+            set_tile_epilogue_warps(static_cast<int>(value));
         } else {
             throw Error(kInvalidArgument, "unknown option: " + k);
         }
@@ -666,7 +668,7 @@ int qg_get_option(const char* key, int64_t* value) {
         else if (k == "scan_last_shape") *value = scan_last_shape();
         else if (k == "tensor_scan") *value = tensor_scan();
         else if (k == "filter_autotune") *value = filter_autotune();
-        else if (k == "filter_tuned_problems") *value = filter_tuned_problems();
+        else if (k == "filter_tuned_problems") *value = filter_tuned_problems() + tile_tuned_problems();
         else if (k == "filter_last_epilogue_warps") *value = filter_last_epilogue_warps();
         else if (k == "filter_epilogue_warps") *value = filter_epilogue_warps();
         else if (k == "mapped_rows_error") *value = mapped_rows_error();

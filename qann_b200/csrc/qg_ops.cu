@@ -118,6 +118,11 @@ void tensor_filter_counts(int64_t* queries, int64_t* redone) {
     *redone = g_filter_redone.load();
 }
 
+void count_tensor_filter(int64_t queries, int64_t redone) {
+    g_filter_queries += queries;
+    g_filter_redone += redone;
+}
+
 void set_tensor_filter(int mode) { g_tensor_filter.store(mode); }
 int tensor_filter() { return g_tensor_filter.load(); }
 
@@ -129,6 +134,16 @@ bool use_tensor_filter(size_t nq, size_t n, int dim, size_t k) {
     const size_t seed = std::max<size_t>(4096, 4 * k);
     return mode > 0 && mm_supported(dim) && k <= 1024 && n > 2 * seed &&
            (mode == 2 || (nq >= 64 && static_cast<double>(nq) * double(n) * dim >= 2e10));
+}
+
+// Nearest-centroid assignment on the tensor cores from 1e8 multiply-adds: the
+// kernels of 3,000 rows against 200 centroids of 64 dims (3.8e7) take 21 us
+// there and 23 us as exact tiles, but wait once for the host; 4,000 against 500
+// of 100 dims (2e8) 25 and 92 us; 500,000 against 4,096 of 128 dims 1.0 and
+// 105 ms.
+bool use_tensor_nearest(size_t n, size_t k, int dim) {
+    const int mode = g_tensor_filter.load();
+    return mode > 0 && tile_supported(dim) && (mode == 2 || static_cast<double>(n) * double(k) * dim >= 1e8);
 }
 
 namespace {

@@ -3,6 +3,7 @@
 #pragma once
 
 #include "qg_index.h"
+#include "qg_tile.h"
 
 namespace qg {
 
@@ -127,8 +128,13 @@ void flat_candidates(const float* q_dev, size_t nq, const float* rows_dev, size_
 
 // Nearest centroid (squared L2, first index on ties) of each row, as the
 // reference's assign_nearest without BLAS (reference src/kmeans.cpp:34-115).
+// xq: the rows prepared for the tensor cores, if the caller keeps them.
 void assign_nearest(const float* x_dev, size_t n, const float* c_dev, size_t k, int dim, uint32_t* out_dev,
-                    cudaStream_t st);
+                    cudaStream_t st, const TileQueries* xq = nullptr);
+// Whether that goes through the tensor cores.
+bool use_tensor_nearest(size_t n, size_t k, int dim);
+// Queries answered by the tensor cores with exact results, and those of them redone exactly.
+void count_tensor_filter(int64_t queries, int64_t redone);
 
 // Drops deleted slots (IndexBase::compact); *reclaimed = slots freed.
 void compact(IndexObj& idx, size_t* reclaimed);

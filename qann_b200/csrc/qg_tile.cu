@@ -1,0 +1,932 @@
+// The tensor-core tile engine. One persistent, warp-specialised kernel forms
+// acc(q, x) = dot of f16 query and base rows, accumulated in FP32 in TMEM, in
+// tiles of 256 queries by 128 base rows, and its epilogue reads them out by
+// mode.
+//
+// Why results taken from it are exact. Query row q is scaled by 2^qe, the
+// base rows by one 2^xe, so that the largest element lies in [2^13, 2^14), and
+// rounded to f16 (unit roundoff u = 2^-11; below 2^-14 the spacing is 2^-24).
+// With s the exact score as the reference computes it (squared L2, or -dot, in
+// float, AVX2 order) and s^ = |q|^2 + |x|^2 - 2 acc 2^-(qe+xe) (or -acc
+// 2^-(qe+xe)) its estimate,
+//   |s^ - s| <= e = c (|q|^2 + |x|^2) + g
+//   c = C for L2, C / 2 for inner product; C = 2^-10 + 2^-13 + d 2^-21
+//   g = 2 a for L2, a for inner product; a = sqrt(d) |q| M 2^-37
+// (2u + u^2) sum|q_i x_i| comes from the relative rounding of both inputs and
+// sum|q_i x_i| <= (|q|^2 + |x|^2) / 2; d 2^-21 covers the tensor cores' FP32
+// accumulation; the 2^-13 the float rounding of the norms, of the bounds and
+// of the reference's own score; a the absolute rounding of elements of a base
+// row that are below 2^-27 of M, the largest magnitude in the base. Squared
+// norms below 2^-100 or not below 2^100 (tile_extreme), where float squares
+// lose relative accuracy, are left out of this: such a query is not settled
+// here, and such a row always passes.
+//
+// Bounds are compared without the query's own terms, which are the same for
+// all rows: lb = xterm(x) - mult acc 2^-(qe+xe) with xterm = (1 - C) |x|^2
+// and mult = 2 for L2, xterm = -C / 2 |x|^2 and mult = 1 for inner product;
+// the upper bound on the same scale is lb + 2 c |x|^2 + (2 c |q|^2 + 2 g).
+#include "qg_device.cuh"
+#include "qg_ops.h"
+#include "qg_sm100.cuh"
+#include "qg_tile.h"
+
+#include <cuda.h>
+#include <cuda_fp16.h>
+
+#include <algorithm>
+#include <atomic>
+#include <cmath>
+#include <map>
+#include <mutex>
+
+namespace qg {
+
+namespace {
+
+constexpr int BM = 256;         // queries per tile: two halves of 128 TMEM lanes
+constexpr int BN = 128;         // base rows per tile (accumulator columns of a half)
+constexpr int KA = 64;          // f16 elements per 128-byte swizzle row (a K block)
+constexpr int kMaxDim = 2048;
+constexpr uint32_t kABlock = BM * 128, kBBlock = BN * 128;   // bytes of one K block
+constexpr uint32_t kPipeBytes = 192 * 1024;                  // query buffers and the ring
+constexpr int kSlots = 7;       // candidates a lane holds before it appends them
+constexpr uint32_t kTmemCols = 512;   // two accumulators of two halves
+constexpr float kOpen = 3.402823466e+38f;   // threshold of a query that has none yet
+constexpr int kNearestCap = 256;            // candidates of a query in nearest mode
+
+// What the epilogue does with an accumulator.
+enum TileMode { kNearest };
+
+struct TileArgs {
+    int nq;
+    int n0;              // first base row of this launch, a multiple of 128; ntiles tiles from there
+    int kblocks;         // 64-element K blocks of the padded rows
+    int ksteps;          // 16-element MMA steps covering d
+    int mtiles, ntiles, group_n;
+    int scout;           // nearest: tiles of each group first read for their bounds alone
+    const float* xterm;      // per base row: its part of the lower bound (+inf: not to be returned), padded
+                             // with +inf to whole tiles
+    const float* run_slack;  // per 32 base rows: 2 c max|x|^2 (+inf when one of them is extreme), padded alike
+    const float* qmul;       // per query: mult 2^-(qe+xe)
+    const float* qslack;     // per query: 2 c |q|^2 + 2 g
+    uint32_t* thr_key;       // per query: key of the smallest upper bound so far
+    uint32_t* cand_count;    // per query
+    uint2* cand;             // per query, cap entries: (lower bound, row)
+    int cap;
+    int* err;
+};
+
+// Where the pipeline's parts lie in shared memory. Up to two K blocks (d <=
+// 128) the query tile is resident, double buffered, and the ring stages one K
+// block of base rows; deeper rows stream both operands through the ring.
+struct TilePipe {
+    bool resident;
+    uint32_t a_bytes, stage_bytes;
+    int stages;
+    __host__ __device__ explicit TilePipe(int kblocks)
+        : resident(kblocks <= 2),
+          a_bytes(resident ? kblocks * kABlock : 0),
+          stage_bytes(resident ? kBBlock : kABlock + kBBlock),
+          stages(static_cast<int>((kPipeBytes - 2 * a_bytes) / stage_bytes)) {}
+};
+constexpr int kMaxStages = 8;
+constexpr int kTermBufs = 8;                          // tiles whose row terms are staged ahead
+constexpr uint32_t kTermBytes = BN * 4, kSlackBytes = BN / 32 * 4;
+constexpr uint32_t kTermStride = (kTermBytes + kSlackBytes + 127) / 128 * 128;
+
+template <int EPI>
+constexpr int tile_threads() { return (3 + EPI) * 32; }
+template <int EPI>
+constexpr size_t tile_smem_bytes() {
+    return 1024 + kPipeBytes + static_cast<size_t>(EPI) * 32 * kSlots * 8 + kTermBufs * kTermStride + 512;
+}
+
+__device__ __forceinline__ bool tile_extreme(float x2) { return (x2 > 0.0f && x2 < 0x1p-100f) || !(x2 < 0x1p100f); }
+
+// Tiles are walked in groups of group_n base tiles, within which the query
+// tile changes slowest: a base tile comes from HBM once and from L2 for every
+// later query tile, and a query tile is loaded once per group. With `scout`
+// there is one group, and each query tile meets its first `scout` base tiles
+// twice, the first time with in_scout set. The walk is a counter per role
+// (divisions only where it starts: finding every tile by division cost the
+// epilogue as many instructions as reading the tile).
+struct TileWalk {
+    int mt, nt, left;   // left: base tiles of this query tile still to come, this one included
+    int base, gsize;    // the group
+    bool in_scout;
+    __device__ __forceinline__ TileWalk(int t, const TileArgs& a) {
+        if (a.scout) {
+            mt = t / (a.ntiles + a.scout);
+            const int rem = t - mt * (a.ntiles + a.scout);
+            base = 0;
+            gsize = a.ntiles;
+            in_scout = rem < a.scout;
+            nt = in_scout ? rem : rem - a.scout;
+        } else {
+            const int group = t / (a.mtiles * a.group_n);
+            const int rem = t - group * a.mtiles * a.group_n;
+            base = group * a.group_n;
+            gsize = min(a.group_n, a.ntiles - base);
+            mt = rem / gsize;
+            nt = base + (rem - mt * gsize);
+            in_scout = false;
+        }
+        left = in_scout ? a.scout - nt : base + gsize - nt;
+    }
+    __device__ __forceinline__ void next(const TileArgs& a) {
+        ++nt;
+        if (--left > 0) return;
+        if (in_scout) {   // the same query tile again, in earnest
+            in_scout = false;
+            nt = base;
+            left = gsize;
+            return;
+        }
+        if (++mt == a.mtiles) {
+            mt = 0;
+            base += gsize;
+            gsize = min(a.group_n, a.ntiles - base);
+        }
+        nt = base;
+        in_scout = a.scout > 0;
+        left = in_scout ? a.scout : gsize;
+    }
+};
+
+__device__ __forceinline__ float min3(float a, float b, float c) {
+    float d;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+
+// (bits, row) into the slot at shared address sp, which then moves on by
+// `step`, when the float of `bits` is at most thr: predicated, no branch.
+__device__ __forceinline__ void keep_below(uint32_t bits, uint32_t row, float thr, uint32_t& sp, uint32_t step) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.le.f32 p, %4, %3;\n\t"
+        "@p st.shared.v2.b32 [%0], {%1, %2};\n\t"
+        "@p add.u32 %0, %0, %5;\n\t}"
+        : "+r"(sp)
+        : "r"(bits), "r"(row), "f"(thr), "f"(__uint_as_float(bits)), "r"(step)
+        : "memory");
+}
+
+// Warp 0 loads by TMA, warps 1 and 2 issue the MMAs of one query half each,
+// the other EPI warps read the accumulators. 256 x 128 tiles: a base row that
+// comes from L2 serves 256 queries (32 KB a tile of 128 dims; a 128 x 256
+// tile needs 64 KB), and four halves fill TMEM, so that the epilogue of one
+// tile runs under the MMAs of the next. Bound by the MMAs and their issue,
+// then by the epilogue's appends: 131,072 queries against 4,096 / 16,384 rows
+// of 128 dims in 248 / 710 us (555 / 774 TFLOP/s counted once, the scout
+// tiles on top), 157 / 572 us with an epilogue that reads nothing; 768 dims
+// 831 us (992 TFLOP/s), there bound by L2, as both operands are streamed.
+template <int EPI, int MODE>
+__global__ void __launch_bounds__(tile_threads<EPI>(), 1)
+    k_tile(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, TileArgs a) {
+    static_assert(EPI == 8 || EPI == 16, "8 or 16 epilogue warps");
+    using namespace sm100;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* base = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
+    const TilePipe pipe(a.kblocks);
+    const int S = pipe.stages;
+    uint8_t* sA = base;                       // resident: two query tiles
+    uint8_t* ring = base + 2 * pipe.a_bytes;
+    uint2* slots = reinterpret_cast<uint2*>(base + kPipeBytes);                        // [kSlots][EPI * 32]
+    uint8_t* terms = reinterpret_cast<uint8_t*>(slots + static_cast<size_t>(EPI) * 32 * kSlots);   // [kTermBufs]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(terms + kTermBufs * kTermStride);
+    uint64_t* full_r = bars;                  // [S] TMA -> MMA
+    uint64_t* empty_r = bars + kMaxStages;    // [S] MMA -> TMA
+    uint64_t* full_a = bars + 2 * kMaxStages;       // [2] TMA -> MMA
+    uint64_t* empty_a = full_a + 2;                 // [2] MMA -> TMA
+    uint64_t* tfull = full_a + 4;                   // [2 accumulators][2 halves] MMA -> epilogue
+    uint64_t* tempty = full_a + 8;                  // [2][2] epilogue -> MMA
+    uint64_t* mma_done = full_a + 12;               // [2] teardown
+    uint64_t* full_x = full_a + 14;                 // [kTermBufs] TMA -> epilogue
+    uint64_t* empty_x = full_x + kTermBufs;         // [kTermBufs] epilogue -> TMA
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(empty_x + kTermBufs);
+    volatile int* abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < S; ++s) {
+            mbar_init(&full_r[s], 1);
+            mbar_init(&empty_r[s], 2);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&full_a[b], 1);
+            mbar_init(&empty_a[b], 2);
+            mbar_init(&mma_done[b], 1);
+        }
+        for (int b = 0; b < 4; ++b) {
+            mbar_init(&tfull[b], 1);
+            mbar_init(&tempty[b], EPI / 2);
+        }
+        for (int b = 0; b < kTermBufs; ++b) {
+            mbar_init(&full_x[b], 1);
+            mbar_init(&empty_x[b], EPI);
+        }
+        *abort = 0;
+        fence_barrier_init();
+    }
+    if (warp == 1) tmem_alloc(tmem_slot, kTmemCols);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    const int total = a.mtiles * (a.ntiles + a.scout);
+    const int per = (total + gridDim.x - 1) / gridDim.x;   // this CTA's tiles: [t_begin, t_end)
+    const int t_begin = min(total, static_cast<int>(blockIdx.x) * per), t_end = min(total, t_begin + per);
+    auto fail = [&] {
+        *abort = 1;
+        atomicExch(a.err, 2);
+    };
+
+    // The loader and the MMA warp are one thread each, and what they do between
+    // two barriers bounds the pipeline: ring positions and parities are carried
+    // (a division by the ring's length per K block held the whole kernel to 1.1k
+    // cycles a block), and matrix descriptors are made once and offset.
+    if (warp == 0) {
+        if (lane == 0) {
+            int s = 0, cur_m = -1, ab = 1;
+            uint32_t rpar = 1, apar = 0;   // parities waited for: a fresh barrier passes the first wait for 1
+            uint32_t loads = 0, aloads = 0, xloads = 0, xpar = 1;
+            int xb = 0;
+            bool ok = true;
+            TileWalk w(t_begin, a);
+            for (int t = t_begin; t < t_end && ok && !*abort; ++t, w.next(a)) {
+                const int mt = w.mt, nt = w.nt;
+                if (pipe.resident && mt != cur_m) {
+                    ab ^= 1;
+                    if (ab == 0) apar ^= 1;   // 1 for the first two loads
+                    if (!mbar_wait(&empty_a[ab], apar, abort)) {
+                        fail();
+                        break;
+                    }
+                    mbar_expect_tx(&full_a[ab], pipe.a_bytes);
+                    for (int kb = 0; kb < a.kblocks; ++kb)
+                        tma_load_2d(&tmA, sA + ab * pipe.a_bytes + kb * kABlock, &full_a[ab], kb * KA, mt * BM);
+                    ++aloads;
+                    cur_m = mt;
+                }
+                {   // the tile's row terms
+                    if (!mbar_wait(&empty_x[xb], xpar, abort)) {
+                        fail();
+                        break;
+                    }
+                    mbar_expect_tx(&full_x[xb], kTermBytes + (MODE == kNearest ? kSlackBytes : 0));
+                    uint8_t* dst = terms + xb * kTermStride;
+                    bulk_load(dst, a.xterm + a.n0 + static_cast<size_t>(nt) * BN, kTermBytes, &full_x[xb]);
+                    if (MODE == kNearest)
+                        bulk_load(dst + kTermBytes, a.run_slack + (a.n0 >> 5) + static_cast<size_t>(nt) * (BN / 32),
+                                  kSlackBytes, &full_x[xb]);
+                    ++xloads;
+                    if (++xb == kTermBufs) {
+                        xb = 0;
+                        xpar ^= 1;
+                    }
+                }
+                for (int kb = 0; kb < a.kblocks; ++kb) {
+                    if (!mbar_wait(&empty_r[s], rpar, abort)) {
+                        fail();
+                        ok = false;
+                        break;
+                    }
+                    mbar_expect_tx(&full_r[s], pipe.stage_bytes);
+                    uint8_t* dst = ring + s * pipe.stage_bytes;
+                    tma_load_2d(&tmB, dst, &full_r[s], kb * KA, a.n0 + nt * BN);
+                    if (!pipe.resident) tma_load_2d(&tmA, dst + kBBlock, &full_r[s], kb * KA, mt * BM);
+                    ++loads;
+                    if (++s == S) {
+                        s = 0;
+                        rpar ^= 1;
+                    }
+                }
+            }
+            // no copy may land after the CTA is gone: wait for the last load of each buffer
+            volatile int never = 0;
+            for (int i = 0; i < S && static_cast<uint32_t>(i) < loads; ++i) {
+                const uint32_t uses = (loads - i + S - 1) / S;   // of stage i
+                mbar_wait(&full_r[i], (uses - 1) & 1, &never);
+            }
+            for (int b = 0; b < 2 && static_cast<uint32_t>(b) < aloads; ++b)
+                mbar_wait(&full_a[b], ((aloads - b + 1) / 2 - 1) & 1, &never);
+            for (int b = 0; b < kTermBufs && static_cast<uint32_t>(b) < xloads; ++b)
+                mbar_wait(&full_x[b], ((xloads - b + kTermBufs - 1) / kTermBufs - 1) & 1, &never);
+        }
+    } else if (warp <= 2) {
+        // one warp per half of the query tile: what a thread does between its
+        // MMAs is not hidden by them (290 ns a K block for 8 MMAs of 33 ns), so
+        // two threads issue
+        if (lane == 0) {
+            const int h = warp - 1;
+            const uint32_t idesc = idesc_f16_f32(128, BN);
+            const uint64_t ring_d = sw128_desc(smem_u32(ring));
+            const uint64_t a_d = sw128_desc(smem_u32(sA) + h * (kABlock / 2));
+            const uint32_t stage_off = pipe.stage_bytes >> 4, abuf_off = pipe.a_bytes >> 4;   // (in descriptor units)
+            int s = 0, cur_m = -1, ab = 1, acc = 0;
+            uint32_t rpar = 0, apar = 1, tpar = 1;
+            bool ok = true;
+            TileWalk w(t_begin, a);
+            for (int t = t_begin; t < t_end && ok && !*abort; ++t, w.next(a)) {
+                const int mt = w.mt;
+                if (pipe.resident && mt != cur_m) {
+                    if (cur_m >= 0) mma_commit(&empty_a[ab]);   // free once its MMAs finish
+                    ab ^= 1;
+                    if (ab == 0) apar ^= 1;   // 0 for the first two
+                    if (!mbar_wait(&full_a[ab], apar, abort)) {
+                        fail();
+                        break;
+                    }
+                    cur_m = mt;
+                }
+                if (!mbar_wait(&tempty[2 * acc + h], tpar, abort)) {
+                    fail();
+                    break;
+                }
+                const bool live = mt * BM + 128 * h < a.nq;   // (a half without queries is left out)
+                const uint32_t td = tmem + acc * 256 + h * 128;
+                for (int kb = 0; kb < a.kblocks; ++kb) {
+                    if (!mbar_wait(&full_r[s], rpar, abort)) {
+                        fail();
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint64_t bd = ring_d + s * stage_off;
+                    const uint64_t ad = pipe.resident ? a_d + ab * abuf_off + kb * (kABlock >> 4)
+                                                      : bd + ((kBBlock + h * (kABlock / 2)) >> 4);
+                    const int ks1 = live ? min(4, a.ksteps - 4 * kb) : 0;
+#pragma unroll
+                    for (int ks = 0; ks < 4; ++ks)   // 32 bytes of K a step
+                        if (ks < ks1) mma_bf16(td, ad + 2 * ks, bd + 2 * ks, idesc, kb > 0 || ks > 0);
+                    mma_commit(&empty_r[s]);
+                    if (++s == S) {
+                        s = 0;
+                        rpar ^= 1;
+                    }
+                }
+                if (!ok) break;
+                mma_commit(&tfull[2 * acc + h]);
+                acc ^= 1;
+                if (acc == 0) tpar ^= 1;
+            }
+            // every MMA done before TMEM is freed
+            volatile int never = 0;
+            mma_commit(&mma_done[h]);
+            mbar_wait(&mma_done[h], 0, &never);
+        }
+    } else {
+        const int ew = warp - 3;      // 0..EPI-1
+        const int quad = warp & 3;    // this warp's TMEM lanes: 32 * quad ..
+        constexpr int kCols = BN / (EPI / 8);   // this warp's columns of its half
+        constexpr int kRuns = kCols / 32;
+        const int half = (ew >> 2) & 1, col0 = (ew >> 3) * kCols;
+        uint2* slot = slots + ew * 32 + lane;   // entry i at slot[i * EPI * 32]
+        constexpr float kInf = __builtin_huge_valf();
+
+        uint32_t sp = smem_u32(slot);                                  // the next free place,
+        const uint32_t room = sp + (kSlots - 3) * EPI * 32 * 8;        // the first with fewer than 4 after it
+        int cur_m = -1, qi = 0;
+        bool live = false;
+        const float none = __int_as_float(0x7fffffff);   // (a lane without a query passes nothing)
+        float qsl = 0.0f, thr = none;
+        float2 mul2 = make_float2(0.0f, 0.0f);
+        auto flush = [&] {
+            const int cnt = static_cast<int>(sp - smem_u32(slot)) / (EPI * 32 * 8);
+            const uint32_t pos = atomicAdd(&a.cand_count[qi], static_cast<uint32_t>(cnt));
+            uint2* to = a.cand + static_cast<size_t>(qi) * a.cap + pos;
+#pragma unroll 1
+            for (int i = 0; i < cnt; ++i)
+                if (pos + i < static_cast<uint32_t>(a.cap)) to[i] = slot[i * EPI * 32];
+            sp = smem_u32(slot);
+        };
+        auto leave = [&] {   // done with the query tile
+            if (sp > smem_u32(slot)) flush();
+            if (MODE == kNearest && live) atomicMin(&a.thr_key[qi], float_key(thr));
+        };
+        TileWalk w(t_begin, a);
+        int acc = 0, xb = 0;
+        uint32_t apar = 0, xpar = 0;
+        for (int t = t_begin; t < t_end; ++t, w.next(a)) {
+            const int mt = w.mt;
+            if (mt != cur_m) {
+                if (cur_m >= 0) leave();
+                cur_m = mt;
+                qi = mt * BM + half * 128 + quad * 32 + lane;
+                live = qi < a.nq;
+                const float mul = live ? -a.qmul[qi] : 0.0f;
+                mul2 = make_float2(mul, mul);
+                qsl = live ? a.qslack[qi] : 0.0f;
+                thr = live ? key_float(*reinterpret_cast<volatile uint32_t*>(a.thr_key + qi)) : none;
+            }
+            const float* sx = reinterpret_cast<const float*>(terms + xb * kTermStride) + col0;
+            const float* sslack = reinterpret_cast<const float*>(terms + xb * kTermStride + kTermBytes) + col0 / 32;
+            const bool ok = __all_sync(0xffffffffu, mbar_wait(&full_x[xb], xpar, abort) &&
+                                                        mbar_wait(&tfull[2 * acc + half], apar, abort));
+            if (!ok) {
+                if (lane == 0) fail();
+                break;
+            }
+            tc_fence_after();
+#pragma unroll 1
+            for (int r = 0; r < kRuns; ++r) {
+                uint32_t v[32];
+                tmem_ld32(tmem + (static_cast<uint32_t>(quad * 32) << 16) +
+                              static_cast<uint32_t>(acc * 256 + half * 128 + col0 + 32 * r),
+                          v);
+                if (r == kRuns - 1) {   // this warp's last read: the accumulator goes back before the work on it
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&tempty[2 * acc + half]);
+                }
+                const float4* s4 = reinterpret_cast<const float4*>(sx + 32 * r);
+                // the lower bounds (over the products), two a packed FMA, and
+                // the smallest of every 4
+                float gm[8];
+#pragma unroll
+                for (int g = 0; g < 8; ++g) {
+                    const float4 x4 = s4[g];
+                    const float2 l01 = __ffma2_rn(mul2, make_float2(__uint_as_float(v[4 * g]), __uint_as_float(v[4 * g + 1])),
+                                                  make_float2(x4.x, x4.y));
+                    const float2 l23 = __ffma2_rn(mul2, make_float2(__uint_as_float(v[4 * g + 2]), __uint_as_float(v[4 * g + 3])),
+                                                  make_float2(x4.z, x4.w));
+                    gm[g] = fminf(min3(l01.x, l01.y, l23.x), l23.y);
+                    v[4 * g] = __float_as_uint(l01.x);
+                    v[4 * g + 1] = __float_as_uint(l01.y);
+                    v[4 * g + 2] = __float_as_uint(l23.x);
+                    v[4 * g + 3] = __float_as_uint(l23.y);
+                }
+                const float low = min3(min3(gm[0], gm[1], gm[2]), min3(gm[3], gm[4], gm[5]), fminf(gm[6], gm[7]));
+                if (MODE == kNearest) {
+                    thr = live ? fminf(thr, __fadd_ru(low, __fadd_ru(sslack[r], qsl))) : none;
+                }
+                if (w.in_scout || !__any_sync(0xffffffffu, low <= thr)) continue;
+                const uint32_t r0 = static_cast<uint32_t>(a.n0 + w.nt * BN + col0 + 32 * r);   // base row of v[0]
+                // the groups in which some lane has one (one reduction: a vote and
+                // a branch per group cost eight latencies)
+                uint32_t groups = 0;
+#pragma unroll
+                for (int g = 0; g < 8; ++g) groups |= gm[g] <= thr ? 1u << g : 0u;
+                groups = __reduce_or_sync(0xffffffffu, groups);
+#pragma unroll
+                for (int g = 0; g < 8; ++g) {
+                    if (!((groups >> g) & 1u)) continue;
+                    if (sp >= room) flush();
+#pragma unroll
+                    for (int j = 4 * g; j < 4 * g + 4; ++j) keep_below(v[j], r0 + j, thr, sp, EPI * 32 * 8);
+                }
+            }
+            acc ^= 1;
+            if (acc == 0) apar ^= 1;
+            __syncwarp();   // the warp's reads of the row terms are done
+            if (lane == 0) mbar_arrive(&empty_x[xb]);
+            if (++xb == kTermBufs) {
+                xb = 0;
+                xpar ^= 1;
+            }
+        }
+        if (cur_m >= 0) leave();
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_free(tmem, kTmemCols);
+    }
+}
+
+// ---- preparing rows ------------------------------------------------------------
+
+// x 2^e rounded to f16 (one exact multiply when 2^e is a normal float)
+__device__ __forceinline__ __half scaled_half(float x, int e) {
+    const float y = (e >= -126 && e <= 127) ? __fmul_rn(x, __int_as_float((e + 127) << 23)) : ldexpf(x, e);
+    return __float2half_rn(y);
+}
+
+// The exponent that puts the largest magnitude m into [2^13, 2^14).
+__device__ __forceinline__ int lift_exp(float m) {
+    int ex = 0;
+    if (m > 0.0f) frexpf(m, &ex);
+    return m > 0.0f ? 14 - ex : 0;
+}
+
+// The largest magnitude below 2^50 (rows holding a larger one are extreme) as
+// its float bits, by one atomic per block.
+__global__ void __launch_bounds__(256) k_tile_amax(const float* __restrict__ x, size_t n, uint32_t* __restrict__ amax) {
+    float m = 0.0f;
+    auto take = [&](float v) {
+        const float b = fabsf(v);
+        if (b < 0x1p50f) m = fmaxf(m, b);
+    };
+    const size_t t = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const size_t step = static_cast<size_t>(gridDim.x) * blockDim.x;
+    const size_t n4 = (reinterpret_cast<uintptr_t>(x) & 15) == 0 ? n / 4 : 0;
+    for (size_t i = t; i < n4; i += step) {
+        const float4 v = reinterpret_cast<const float4*>(x)[i];
+        take(v.x);
+        take(v.y);
+        take(v.z);
+        take(v.w);
+    }
+    for (size_t i = 4 * n4 + t; i < n; i += step) take(x[i]);
+    __shared__ float wm[8];
+    m = warp_max(m);
+    if ((threadIdx.x & 31) == 0) wm[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) m = fmaxf(m, wm[w]);
+        if (m > 0.0f) atomicMax(amax, __float_as_uint(m));   // (non-negative floats order as their bits)
+    }
+}
+
+// Base rows to f16 with the shared exponent, and their squared norms. One warp
+// per row, twice over a row that the first read leaves in L1.
+__global__ void __launch_bounds__(256) k_tile_base(const float* __restrict__ x, size_t n, int d, int dpad,
+                                                   const uint32_t* __restrict__ amax, __half* __restrict__ xh,
+                                                   float* __restrict__ x2) {
+    const size_t r = (static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (r >= n) return;
+    const int e = lift_exp(__uint_as_float(*amax));
+    const float* row = x + r * d;
+    float s = 0.0f;
+    for (int j = lane; j < d; j += 32) s = __fmaf_rn(row[j], row[j], s);
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    const bool zero = tile_extreme(s);
+    for (int j = lane; j < dpad; j += 32)
+        xh[r * dpad + j] = j < d && !zero ? scaled_half(row[j], e) : __float2half_rn(0.0f);
+    if (lane == 0) x2[r] = s;
+}
+
+// Query rows to f16, each with its own exponent, and their squared norms.
+__global__ void __launch_bounds__(256) k_tile_queries(const float* __restrict__ x, size_t n, int d, int dpad,
+                                                      __half* __restrict__ xh, float* __restrict__ x2,
+                                                      int* __restrict__ xe) {
+    const size_t r = (static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (r >= n) return;
+    const float* row = x + r * d;
+    float s = 0.0f, mx = 0.0f;
+    for (int j = lane; j < d; j += 32) {
+        const float v = row[j];
+        s = __fmaf_rn(v, v, s);
+        mx = fmaxf(mx, fabsf(v));
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        s += __shfl_xor_sync(0xffffffffu, s, o);
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    }
+    const bool zero = tile_extreme(s);
+    const int e = zero ? 0 : lift_exp(mx);
+    for (int j = lane; j < dpad; j += 32)
+        xh[r * dpad + j] = j < d && !zero ? scaled_half(row[j], e) : __float2half_rn(0.0f);
+    if (lane == 0) {
+        x2[r] = s;
+        xe[r] = e;
+    }
+}
+
+// The bound's factors (top of the file).
+struct TileBound {
+    float mult;   // of acc
+    float xc;     // xterm = xc |x|^2
+    float c2;     // 2 c
+    float g2;     // 2 g = g2 |q| M
+    TileBound(int d, bool ip) {
+        const double C = std::ldexp(1.0, -10) + std::ldexp(1.0, -13) + d * std::ldexp(1.0, -21);
+        mult = ip ? 1.0f : 2.0f;
+        xc = static_cast<float>(ip ? -0.5 * C : 1.0 - C);
+        c2 = static_cast<float>(ip ? C : 2.0 * C);
+        g2 = static_cast<float>((ip ? 2.0 : 4.0) * std::sqrt(double(d)) * std::ldexp(1.0, -37));
+    }
+};
+
+// Each base row's part of the lower bound (+inf for rows that are refused,
+// -inf for extreme ones, which always pass), and per 32 rows the slack that
+// takes the smallest lower bound among them to an upper bound.
+__global__ void __launch_bounds__(256) k_tile_terms(const float* __restrict__ sq, size_t n, size_t npad, TileBound b,
+                                                    float* __restrict__ xterm, float* __restrict__ run_slack) {
+    const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    constexpr float kInf = __builtin_huge_valf();
+    float s = 0.0f;
+    if (i < n) {
+        const float x2 = sq[i];
+        const bool ex = tile_extreme(x2);
+        xterm[i] = ex ? -kInf : __fmul_rn(b.xc, x2);
+        s = ex ? kInf : __fmul_ru(b.c2, x2);
+    } else if (i < npad) {
+        xterm[i] = kInf;
+    }
+    s = warp_max(s);
+    if ((threadIdx.x & 31) == 0 && i < npad) run_slack[i >> 5] = s;
+}
+
+// Per query: the factor that takes acc to the row's scale, the slack, an open
+// threshold and an empty candidate list. An extreme query's list counts as
+// overflowed from the start.
+__global__ void k_tile_open(const float* __restrict__ q2, const int* __restrict__ qexp, int nq, TileBound b,
+                            const uint32_t* __restrict__ amax, int cap, float* __restrict__ qmul,
+                            float* __restrict__ qslack, uint32_t* __restrict__ thr_key, uint32_t* __restrict__ count) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nq) return;
+    const float s = q2[i], M = __uint_as_float(*amax);
+    const bool ex = tile_extreme(s);
+    qmul[i] = ldexpf(b.mult, -(qexp[i] + lift_exp(M)));
+    qslack[i] = ex ? 0.0f : __fadd_ru(__fmul_ru(b.c2, s), __fmul_ru(b.g2, __fmul_ru(__fsqrt_ru(s), M)));
+    thr_key[i] = float_key(ex ? -kOpen : kOpen);
+    count[i] = ex ? static_cast<uint32_t>(cap) + 1 : 0u;
+}
+
+// One warp per query: of its candidates, those whose lower bound is at most
+// the smallest upper bound. A single one is the nearest row; several are
+// scored exactly, 8 at a time by 4-lane groups (even dim at 8-byte alignment,
+// kG = 4) or 4 at a time by 8-lane groups, and the smallest (score, row) wins.
+// An overflowed list goes to redo.
+template <int kG>
+__global__ void __launch_bounds__(256) k_tile_pick(const float* __restrict__ q, int d, const float* __restrict__ rows,
+                                                   int nq, const uint32_t* __restrict__ count,
+                                                   const uint2* __restrict__ cand, int cap,
+                                                   const uint32_t* __restrict__ thr_key, uint32_t first,
+                                                   uint32_t* __restrict__ label, uint32_t* __restrict__ redo,
+                                                   uint32_t* __restrict__ nredo) {
+    const int qi = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (qi >= nq) return;
+    const uint32_t cnt = count[qi];
+    const float T = key_float(thr_key[qi]);
+    const uint2* c = cand + static_cast<size_t>(qi) * cap;
+    const float* qv = q + static_cast<size_t>(qi) * d;
+    constexpr int kPer = 32 / kG;   // candidates scored together
+    uint64_t best = ~0ull;
+    uint32_t one = 0, passed = 0;
+    if (cnt <= static_cast<uint32_t>(cap)) {
+        for (uint32_t b = 0; b < cnt; b += 32) {
+            const uint2 e = b + lane < cnt ? c[b + lane] : make_uint2(0x7f800000u, 0u);
+            const unsigned in = __ballot_sync(0xffffffffu, b + lane < cnt && __uint_as_float(e.x) <= T);
+            passed += __popc(in);
+            if (in) one = __shfl_sync(0xffffffffu, e.y, __ffs(in) - 1);
+        }
+        for (uint32_t b = 0; passed > 1 && b < cnt; b += 32) {
+            const uint2 e = b + lane < cnt ? c[b + lane] : make_uint2(0x7f800000u, 0u);
+            unsigned in = __ballot_sync(0xffffffffu, b + lane < cnt && __uint_as_float(e.x) <= T);
+            while (in) {
+                // this lane group's candidate: the set bit of its rank
+                unsigned m = in;
+                for (int g = 0; g < lane / kG && m; ++g) m &= m - 1;
+                const bool act = m != 0;
+                const uint32_t row = __shfl_sync(0xffffffffu, e.y, act ? __ffs(m) - 1 : 0);
+                const float* rp = rows + static_cast<size_t>(row) * d;
+                const float s = kG == 4 ? exact_avx2_group4<true>(qv, rp, d) : exact_avx2_group8<true, true>(qv, rp, d);
+                const uint64_t key = act ? (static_cast<uint64_t>(float_key_eq0(s)) << 32) | row : ~0ull;
+                best = key < best ? key : best;
+                for (int g = 0; g < kPer && in; ++g) in &= in - 1;
+            }
+        }
+    }
+    if (passed > 1) {
+        for (int o = 16; o > 0; o >>= 1) {
+            const uint64_t other = __shfl_xor_sync(0xffffffffu, best, o);
+            best = other < best ? other : best;
+        }
+        one = static_cast<uint32_t>(best);
+    }
+    if (lane == 0) {
+        if (passed > 0) label[qi] = one;
+        else redo[atomicAdd(nredo, 1u)] = first + qi;
+    }
+}
+
+// ---- launching ------------------------------------------------------------------
+
+using EncodeTiled = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                 const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                 CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+EncodeTiled encode_fn() {
+    static EncodeTiled fn = nullptr;
+    static std::once_flag once;
+    std::call_once(once, [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q{};
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            fn = reinterpret_cast<EncodeTiled>(p);
+    });
+    require(fn != nullptr, "cuTensorMapEncodeTiled is not available", kCudaError);
+    return fn;
+}
+
+// f16 rows (dpad elements, row stride dpad * 2 bytes) read as boxes of 64 x box_rows, 128-byte swizzle.
+CUtensorMap make_map(const void* ptr, size_t rows, int dpad, int box_rows) {
+    CUtensorMap m;
+    const cuuint64_t dims[2] = {static_cast<cuuint64_t>(dpad), static_cast<cuuint64_t>(rows)};
+    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(dpad) * 2};
+    const cuuint32_t box[2] = {static_cast<cuuint32_t>(KA), static_cast<cuuint32_t>(box_rows)};
+    const cuuint32_t estr[2] = {1, 1};
+    const CUresult r = encode_fn()(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(ptr), dims, strides, box,
+                                   estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    require(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled failed", kCudaError);
+    return m;
+}
+
+// The epilogue's warp count is the schedule choice: 8 (each warp 128 columns
+// of its 32 queries) or 16 (64 columns each). On the first launch of a problem
+// (mode, K blocks, query and base tiles by their power of two) with at least 8
+// tiles per SM, both are timed twice on the launch's own inputs and the faster
+// kept for the rest of the process; reset() puts the launch's outputs back
+// before each timed run, and the last run's are the launch's result. Both give
+// the same results. Launches that must not wait on the host use the problem's
+// pick if there is one, else 16.
+std::mutex g_tune_mu;
+std::map<uint64_t, int> g_tuned;   // problem key -> epilogue warps
+std::atomic<int> g_tune_on{1}, g_tune_last{8}, g_tune_force{0};
+
+template <int EPI, int MODE>
+void launch_epi(const CUtensorMap& tmA, const CUtensorMap& tmB, const TileArgs& a, cudaStream_t st) {
+    allow_large_smem<k_tile<EPI, MODE>>();
+    const int tiles = a.mtiles * (a.ntiles + a.scout);
+    k_tile<EPI, MODE><<<static_cast<unsigned>(std::min(tiles, sm_count())), tile_threads<EPI>(),
+                        tile_smem_bytes<EPI>(), st>>>(tmA, tmB, a);
+    QG_LAUNCH_CHECK();
+}
+
+template <int MODE>
+void launch_as(int epi, const CUtensorMap& tmA, const CUtensorMap& tmB, const TileArgs& a, cudaStream_t st) {
+    if (epi == 16) launch_epi<16, MODE>(tmA, tmB, a, st);
+    else launch_epi<8, MODE>(tmA, tmB, a, st);
+    g_tune_last.store(epi);
+}
+
+template <int MODE, class Reset>
+void launch_tile(const CUtensorMap& tmA, const CUtensorMap& tmB, const TileArgs& a, cudaStream_t st, bool may_tune,
+                 Reset reset) {
+    if (const int f = g_tune_force.load()) {
+        launch_as<MODE>(f, tmA, tmB, a, st);
+        return;
+    }
+    const uint64_t key = (static_cast<uint64_t>(MODE) << 48) | (static_cast<uint64_t>(a.kblocks) << 40) |
+                         (static_cast<uint64_t>(next_pow2(a.mtiles)) << 20) | static_cast<uint64_t>(next_pow2(a.ntiles));
+    {
+        std::lock_guard<std::mutex> g(g_tune_mu);
+        const auto it = g_tuned.find(key);
+        if (it != g_tuned.end()) {
+            launch_as<MODE>(it->second, tmA, tmB, a, st);
+            return;
+        }
+    }
+    if (!may_tune || !g_tune_on.load() || static_cast<long long>(a.mtiles) * a.ntiles < 8ll * sm_count()) {
+        launch_as<MODE>(16, tmA, tmB, a, st);
+        return;
+    }
+    cudaEvent_t e0, e1;
+    QG_CUDA(cudaEventCreate(&e0));
+    QG_CUDA(cudaEventCreate(&e1));
+    constexpr int kCand[2] = {8, 16};
+    float fastest[2] = {0.0f, 0.0f};
+    for (int round = 0; round < 2; ++round)
+        for (int c = 0; c < 2; ++c) {
+            if (round + c > 0) reset();
+            QG_CUDA(cudaEventRecord(e0, st));
+            launch_as<MODE>(kCand[c], tmA, tmB, a, st);
+            QG_CUDA(cudaEventRecord(e1, st));
+            QG_CUDA(cudaEventSynchronize(e1));
+            float ms = 0.0f;
+            QG_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+            if (round == 0 || ms < fastest[c]) fastest[c] = ms;
+        }
+    cudaEventDestroy(e0);
+    cudaEventDestroy(e1);
+    std::lock_guard<std::mutex> g(g_tune_mu);
+    g_tuned[key] = fastest[1] < fastest[0] ? 16 : 8;
+}
+
+unsigned blocks_of(size_t n, size_t per = 256) { return static_cast<unsigned>(ceil_div(std::max<size_t>(1, n), per)); }
+
+} // namespace
+
+void set_tile_autotune(int on) { g_tune_on.store(on); }
+int tile_autotune() { return g_tune_on.load(); }
+int64_t tile_tuned_problems() {
+    std::lock_guard<std::mutex> g(g_tune_mu);
+    return static_cast<int64_t>(g_tuned.size());
+}
+int tile_last_epilogue_warps() { return g_tune_last.load(); }
+void set_tile_epilogue_warps(int warps) { g_tune_force.store(warps); }
+int tile_epilogue_warps() { return g_tune_force.load(); }
+
+bool tile_supported(int dim) { return dim >= 1 && dim <= kMaxDim; }
+
+void tile_prepare_queries(const float* rows, size_t n, int dim, TileQueries& out, cudaStream_t st) {
+    require(tile_supported(dim), "the tensor-core path does not support this dimension", kUnsupported);
+    out.n = n;
+    out.dim = dim;
+    out.dpad = (dim + 7) & ~7;
+    out.f16.alloc(std::max<size_t>(1, n * out.dpad), st);
+    out.sq.alloc(std::max<size_t>(1, n), st);
+    out.exps.alloc(std::max<size_t>(1, n), st);
+    if (n == 0) return;
+    k_tile_queries<<<blocks_of(n * 32), 256, 0, st>>>(rows, n, dim, out.dpad, reinterpret_cast<__half*>(out.f16.get()),
+                                                      out.sq.get(), out.exps.get());
+    QG_LAUNCH_CHECK();
+}
+
+void tile_prepare_base(const float* rows, size_t n, int dim, TileBase& out, cudaStream_t st) {
+    require(tile_supported(dim), "the tensor-core path does not support this dimension", kUnsupported);
+    out.n = n;
+    out.dim = dim;
+    out.dpad = (dim + 7) & ~7;
+    out.f16.alloc(std::max<size_t>(1, n * out.dpad), st);
+    out.sq.alloc(std::max<size_t>(1, n), st);
+    out.amax.alloc(1, st);
+    QG_CUDA(cudaMemsetAsync(out.amax.get(), 0, sizeof(uint32_t), st));
+    if (n == 0) return;
+    k_tile_amax<<<std::min(blocks_of(n * dim, 4096), static_cast<unsigned>(8 * sm_count())), 256, 0, st>>>(
+        rows, n * dim, out.amax.get());
+    QG_LAUNCH_CHECK();
+    k_tile_base<<<blocks_of(n * 32), 256, 0, st>>>(rows, n, dim, out.dpad, out.amax.get(),
+                                                   reinterpret_cast<__half*>(out.f16.get()), out.sq.get());
+    QG_LAUNCH_CHECK();
+}
+
+// One launch over every base row per block of queries: a lane of the epilogue
+// owns one query, keeps its smallest upper bound so far and appends the rows
+// whose lower bound is at most that. Rows in random order give about ln(n)
+// records a query and warp; only those within the bound of the final one are
+// scored exactly.
+size_t tile_nearest(const float* q, const TileQueries& qs, const float* base_rows, const TileBase& base,
+                    uint32_t* label, DevBuf<uint32_t>& redo, cudaStream_t st) {
+    const size_t nq = qs.n, n = base.n;
+    const int d = base.dim;
+    if (nq == 0) return 0;
+    require(n >= 1 && n < (size_t{1} << 31) && nq < (size_t{1} << 31), "too many rows for the tensor-core path",
+            kUnsupported);
+    const TileBound bound(d, false);
+    const size_t npad = ceil_div(n, BN) * BN;
+    DevBuf<float> xterm(npad, st), run_slack(npad / 32, st);
+    k_tile_terms<<<blocks_of(npad), 256, 0, st>>>(base.sq.get(), n, npad, bound, xterm.get(), run_slack.get());
+    QG_LAUNCH_CHECK();
+    const size_t QB = 131072;   // queries per block: 268 MB of candidate lists
+    const size_t qb = std::min(QB, nq);
+    DevBuf<float> qmul(qb, st), qslack(qb, st);
+    DevBuf<uint32_t> thr(qb, st), count(qb, st);
+    DevBuf<uint2> cand(qb * kNearestCap, st);
+    redo.alloc(nq + 2, st);   // the list, its length, and the error flag
+    uint32_t* const nredo = redo.get() + nq;
+    QG_CUDA(cudaMemsetAsync(nredo, 0, 2 * sizeof(uint32_t), st));
+    TileArgs a{};
+    a.kblocks = (base.dpad + KA - 1) / KA;
+    a.ksteps = (d + 15) / 16;
+    a.ntiles = static_cast<int>(ceil_div(n, BN));
+    // a base that stays in L2 is walked whole for each query tile, so that the
+    // running bound meets every row; a larger one in groups
+    // (a quarter of it, at most 16 tiles, for the bound alone, before any row is
+    // appended: 131,072 queries of 128 dims against 4,096 rows took 262 us
+    // with it and 286 us without, against 16,384 rows 710 and 962 us)
+    const bool whole = n * base.dpad * 2 <= (size_t{32} << 20);
+    a.group_n = whole ? a.ntiles : 16;
+    a.scout = whole ? std::min((a.ntiles + 3) / 4, 16) : 0;
+    a.xterm = xterm.get();
+    a.run_slack = run_slack.get();
+    a.qmul = qmul.get();
+    a.qslack = qslack.get();
+    a.thr_key = thr.get();
+    a.cand_count = count.get();
+    a.cand = cand.get();
+    a.cap = kNearestCap;
+    a.err = reinterpret_cast<int*>(nredo + 1);
+    const CUtensorMap tmB = make_map(base.f16.get(), n, base.dpad, BN);
+    const bool g4 = (d & 1) == 0 && (reinterpret_cast<uintptr_t>(q) & 7) == 0 &&
+                    (reinterpret_cast<uintptr_t>(base_rows) & 7) == 0;
+    for (size_t q0 = 0; q0 < nq; q0 += QB) {
+        const int nb = static_cast<int>(std::min(QB, nq - q0));
+        a.nq = nb;
+        a.mtiles = static_cast<int>(ceil_div(static_cast<size_t>(nb), BM));
+        auto open = [&] {
+            k_tile_open<<<blocks_of(nb), 256, 0, st>>>(qs.sq.get() + q0, qs.exps.get() + q0, nb, bound, base.amax.get(),
+                                                       kNearestCap, qmul.get(), qslack.get(), thr.get(), count.get());
+            QG_LAUNCH_CHECK();
+        };
+        open();
+        const CUtensorMap tmA = make_map(qs.f16.get() + q0 * qs.dpad, nb, qs.dpad, BM);
+        {
+            KernelTimer kt("mm_filter", st);
+            launch_tile<kNearest>(tmA, tmB, a, st, /*may_tune=*/true, open);
+        }
+        const unsigned blocks = blocks_of(nb, 8);
+        if (g4)
+            k_tile_pick<4><<<blocks, 256, 0, st>>>(q + q0 * d, d, base_rows, nb, count.get(), cand.get(), kNearestCap,
+                                                   thr.get(), static_cast<uint32_t>(q0), label + q0, redo.get(), nredo);
+        else
+            k_tile_pick<8><<<blocks, 256, 0, st>>>(q + q0 * d, d, base_rows, nb, count.get(), cand.get(), kNearestCap,
+                                                   thr.get(), static_cast<uint32_t>(q0), label + q0, redo.get(), nredo);
+        QG_LAUNCH_CHECK();
+    }
+    uint32_t h[2] = {0, 0};
+    QG_CUDA(cudaMemcpyAsync(h, nredo, sizeof(h), cudaMemcpyDeviceToHost, st));
+    QG_CUDA(cudaStreamSynchronize(st));
+    require(h[1] == 0, "tensor-core filter: a pipeline wait timed out", kRuntimeError);
+    return h[0];
+}
+
+} // namespace qg

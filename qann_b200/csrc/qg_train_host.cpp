@@ -149,6 +149,10 @@ KMeansOut kmeans_lloyd(const float* x_dev, size_t n, int d, int k, size_t iters,
     out.assign.alloc(pn, st);
     DevBuf<uint32_t> order(pn, st), off(static_cast<size_t>(P) * (k + 1), st);
     DevBuf<int> empty(1, st);
+    // the points prepared once for the tensor cores (up to 4 GB), not per iteration
+    TileQueries xq;
+    const bool keep = P == 1 && k > 64 && use_tensor_nearest(n, k, d) && n * static_cast<size_t>(d) * 2 <= size_t{4} << 30;
+    if (keep) tile_prepare_queries(x_dev, n, d, xq, st);
     auto assign_all = [&]() {
         if (k <= 64) {
             assign_small(x_dev, n, d, cent.get(), k, P, out.assign.get(), st);
@@ -156,7 +160,7 @@ KMeansOut kmeans_lloyd(const float* x_dev, size_t n, int d, int k, size_t iters,
         }
         for (int p = 0; p < P; ++p)
             assign_nearest(x_dev + static_cast<size_t>(p) * n * d, n, cent.get() + p * kd, k, d,
-                           out.assign.get() + static_cast<size_t>(p) * n, st);
+                           out.assign.get() + static_cast<size_t>(p) * n, st, keep ? &xq : nullptr);
     };
     for (size_t it = 0; it < iters; ++it) {
         assign_all();
