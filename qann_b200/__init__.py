@@ -79,7 +79,7 @@ def _ids(ids) -> np.ndarray:
 
 
 def set_tensor_filter(mode: int) -> None:
-    """Exact top-k over many rows through the BF16 tensor-core filter and FP32
+    """Exact top-k over many rows through the F16 tensor-core filter and FP32
     recheck: 0 never, 1 when it pays (default), 2 whenever supported. Results
     are identical in every mode."""
     check(_lib.lib.qg_set_option(b"tensor_filter", int(mode)))

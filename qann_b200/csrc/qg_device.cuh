@@ -540,4 +540,56 @@ struct KeyBins {
     }
 };
 
+// A threshold T at or above the k-th smallest (1-based) of the n uint32 keys
+// in shared memory, by one block. 0xFFFFFFFF marks an unbounded key, above
+// every other. [kmin, kmax] is the range of the nfin bounded keys; they are
+// counted into kKeyBins nearly equal key intervals (KeyBins), and T is the last key of the
+// first interval whose running count reaches k, so at least k keys are <= T
+// and T lies within one interval of the k-th smallest. (A T above the k-th
+// smallest only admits more candidates to the exact step.) hist: kKeyHist
+// ints of shared scratch, zero on entry, bin b at b + b / 32 so that the lanes
+// that add up 32 bins each read distinct banks; two barriers.
+inline constexpr int kKeyBins = 1024, kKeyHist = kKeyBins + kKeyBins / 32;
+__device__ __noinline__ static uint32_t block_threshold_u32(const uint32_t* keys, int n, int k, uint32_t kmin,
+                                                            uint32_t kmax, int nfin, int* hist, uint32_t* s_t) {
+    if (nfin < k) return 0xFFFFFFFFu;   // (block-uniform) the k-th smallest is unbounded
+    if (kmax == kmin) return kmin;
+    const KeyBins kb(kmin, static_cast<uint64_t>(kmax - kmin) + 1, kKeyBins);
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const uint32_t key = keys[i];
+        if (key != 0xFFFFFFFFu) {
+            const int b = kb.bin(key);
+            atomicAdd(&hist[b + (b >> 5)], 1);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {   // warp 0: lane l owns bins 32 l .. 32 l + 31
+        const int lane = threadIdx.x;
+        constexpr int kPer = kKeyBins / 32;
+        int own = 0;
+#pragma unroll 8
+        for (int b = 0; b < kPer; ++b) own += hist[(kPer + 1) * lane + b];
+        int incl = own;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += t;
+        }
+        const int excl = incl - own;
+        if (excl < k && k <= incl) {
+            int acc = excl, bin = kPer * lane + kPer - 1;
+            for (int b = 0; b < kPer; ++b) {
+                acc += hist[(kPer + 1) * lane + b];
+                if (acc >= k) {
+                    bin = kPer * lane + b;
+                    break;
+                }
+            }
+            // every key counted in bins <= bin is <= kb.last(bin)
+            *s_t = static_cast<uint32_t>(min(kb.last(bin), static_cast<uint64_t>(kmax)));
+        }
+    }
+    __syncthreads();
+    return *s_t;
+}
+
 } // namespace qg

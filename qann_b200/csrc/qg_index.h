@@ -5,6 +5,7 @@
 #include "qg_cuda.h"
 #include "qg_host.h"
 #include "qg_search.h"
+#include "qg_tile.h"
 
 #include <memory>
 #include <mutex>
@@ -22,9 +23,7 @@ struct DeviceIVF {
     DevBuf<uint4> codes;
     DevBuf<uint64_t> deleted;
     DevBuf<int64_t> labels;   // slot -> id when the ids are not the slots
-    DevBuf<uint16_t> cent_f16;   // scaled f16 centroids for the tensor-core coarse step
-    DevBuf<float> cent_sq;
-    DevBuf<int> cent_exp;
+    TileQueries cent;            // scaled f16 centroids for the tensor-core coarse step
     size_t total_sb = 0;
 };
 

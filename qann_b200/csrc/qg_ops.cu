@@ -127,13 +127,12 @@ void set_tensor_filter(int mode) { g_tensor_filter.store(mode); }
 int tensor_filter() { return g_tensor_filter.load(); }
 
 // The exact top-k either way; the tensor-core filter when the work is large
-// enough to pay for its bf16 copies (or always, in mode 2), the FP32 tiles
+// enough to pay for its f16 copy (or always, in mode 2), the FP32 tiles
 // otherwise.
 bool use_tensor_filter(size_t nq, size_t n, int dim, size_t k) {
     const int mode = g_tensor_filter.load();
-    const size_t seed = std::max<size_t>(4096, 4 * k);
-    return mode > 0 && mm_supported(dim) && k <= 1024 && n > 2 * seed &&
-           (mode == 2 || (nq >= 64 && static_cast<double>(nq) * double(n) * dim >= 2e10));
+    return mode > 0 && tile_supported(dim) && k <= kTileMaxK &&
+           (mode == 2 || (nq >= 64 && static_cast<double>(nq) * double(n) * dim >= 5e8));
 }
 
 // Nearest-centroid assignment on the tensor cores from 1e8 multiply-adds: the
@@ -172,62 +171,68 @@ void tensor_coarse_counts(int64_t* queries, int64_t* redone) {
 // exact path took 92 us and the F16 GEMM and recheck 66 us.
 bool use_tensor_coarse(size_t nq, int nlist, int dim) {
     const int mode = g_tensor_filter.load();
-    return mode > 0 && mm_supported(dim) &&
+    return mode > 0 && tile_supported(dim) &&
            (mode == 2 || static_cast<double>(nq) * nlist * dim >= 2.5e7 ||
             static_cast<double>(nlist) * dim >= 2097152.0);
 }
 
+// lists of k keys and slots back to the queries at[] they belong to
+__global__ void k_put_back(const uint64_t* __restrict__ key, const uint32_t* __restrict__ slot,
+                           const uint32_t* __restrict__ at, size_t m, int k, uint64_t* __restrict__ out_key,
+                           uint32_t* __restrict__ out_slot) {
+    const size_t t = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (t >= m * k) return;
+    const size_t o = static_cast<size_t>(at[t / k]) * k + t % k;
+    out_key[o] = key[t];
+    out_slot[o] = slot[t];
+}
+
 void flat_candidates(const float* q_dev, size_t nq, const float* rows_dev, size_t n, int dim, bool ip, size_t k,
                      const uint64_t* allow_dev, const uint64_t* deny_dev, uint64_t* out_key, uint32_t* out_slot,
-                     cudaStream_t st, bool allow_mm, const MmRows* pre) {
+                     cudaStream_t st, bool allow_mm, const TileBase* pre) {
     if (!allow_mm || !use_tensor_filter(nq, n, dim, k)) {
         flat_candidates_fp32(q_dev, nq, rows_dev, n, dim, ip, k, allow_dev, deny_dev, out_key, out_slot, st);
         return;
     }
-    MmRows tmp;
-    const MmRows* base = pre;
+    TileBase own;
+    const TileBase* base = pre;
     if (!base) {
-        mm_prepare(rows_dev, n, dim, tmp, st);
-        base = &tmp;
+        tile_prepare_base(rows_dev, n, dim, own, st);
+        base = &own;
     }
-    std::vector<int> ovf;
-    mm_topk(q_dev, nq, rows_dev, *base, ip, k, allow_dev, deny_dev, out_key, out_slot, ovf, st);
-    g_filter_queries += static_cast<int64_t>(nq);
-    g_filter_redone += static_cast<int64_t>(ovf.size());
-    if (ovf.empty()) return;
-    // queries whose candidate list overflowed: the exact FP32 tiles over every row
-    const size_t m = ovf.size();
-    DevBuf<uint32_t> idx(m, st);
-    std::vector<uint32_t> hidx(ovf.begin(), ovf.end());
-    QG_CUDA(cudaMemcpyAsync(idx.get(), hidx.data(), m * 4, cudaMemcpyHostToDevice, st));
-    DevBuf<float> qs(m * dim, st);
-    gather_rows(q_dev, idx.get(), m, dim, qs.get(), st);
+    TileQueries qs;
+    tile_prepare_queries(q_dev, nq, dim, qs, st);
+    DevBuf<uint32_t> redo;
+    const size_t m = tile_topk(q_dev, qs, rows_dev, *base, ip, k, allow_dev, deny_dev, out_key, out_slot, redo, st);
+    count_tensor_filter(static_cast<int64_t>(nq), static_cast<int64_t>(m));
+    if (m == 0) return;
+    // queries it could not settle: the exact FP32 tiles over every row
+    DevBuf<float> qr(m * dim, st);
+    gather_rows(q_dev, redo.get(), m, dim, qr.get(), st);
     DevBuf<uint64_t> sk(m * k, st);
     DevBuf<uint32_t> ss(m * k, st);
-    flat_candidates_fp32(qs.get(), m, rows_dev, n, dim, ip, k, allow_dev, deny_dev, sk.get(), ss.get(), st);
-    for (size_t j = 0; j < m; ++j) {
-        QG_CUDA(cudaMemcpyAsync(out_key + static_cast<size_t>(ovf[j]) * k, sk.get() + j * k, k * 8,
-                                cudaMemcpyDeviceToDevice, st));
-        QG_CUDA(cudaMemcpyAsync(out_slot + static_cast<size_t>(ovf[j]) * k, ss.get() + j * k, k * 4,
-                                cudaMemcpyDeviceToDevice, st));
-    }
-    QG_CUDA(cudaStreamSynchronize(st));
+    flat_candidates_fp32(qr.get(), m, rows_dev, n, dim, ip, k, allow_dev, deny_dev, sk.get(), ss.get(), st);
+    k_put_back<<<static_cast<unsigned>(ceil_div(m * k, 256)), 256, 0, st>>>(sk.get(), ss.get(), redo.get(), m,
+                                                                            static_cast<int>(k), out_key, out_slot);
+    QG_LAUNCH_CHECK();
 }
 
-// Flat results in (score, slot) order with ids and the exact score.
+// Flat results in (score, slot) order with ids and the exact score, which its
+// key gives back but for the sign of a zero (formed again).
 __global__ void k_finalize_flat(const float* __restrict__ q, int dim, const float* __restrict__ rows,
-                                const uint32_t* __restrict__ slot, int k, bool ip, const int64_t* __restrict__ labels,
-                                bool cosine, int64_t* __restrict__ out_ids, float* __restrict__ out_d, size_t nq) {
+                                const uint64_t* __restrict__ key, const uint32_t* __restrict__ slot, int k, bool ip,
+                                const int64_t* __restrict__ labels, bool cosine, int64_t* __restrict__ out_ids,
+                                float* __restrict__ out_d, size_t nq) {
     const size_t t = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t >= nq * k) return;
-    const size_t qi = t / k;
     const uint32_t s = slot[t];
     if (s == 0xFFFFFFFFu) {
         out_ids[t] = -1;
         out_d[t] = __int_as_float(0x7f800000);
         return;
     }
-    const float d = exact_score(rows + static_cast<size_t>(s) * dim, q + qi * dim, dim, ip);
+    float d = key_float(static_cast<uint32_t>(key[t] >> 32));
+    if (d == 0.0f) d = exact_score(rows + static_cast<size_t>(s) * dim, q + (t / k) * dim, dim, ip);
     out_ids[t] = labels ? labels[s] : static_cast<int64_t>(s);
     out_d[t] = cosine ? __fmul_rn(d, 0.5f) : d;
 }
@@ -456,8 +461,8 @@ void search(IndexObj& idx, const SearchRequest& r, cudaStream_t st) {
         flat_candidates(p.q.get(), r.nq, o.dev.rows.get(), o.model.idmap.slots(), dim, ip, r.k, p.filter.get(),
                         r.filter ? nullptr : o.dev.deleted.get(), ck.get(), cs.get(), st);
         k_finalize_flat<<<static_cast<unsigned>(ceil_div(r.nq * r.k, 256)), 256, 0, st>>>(
-            p.q.get(), dim, o.dev.rows.get(), cs.get(), static_cast<int>(r.k), ip, o.dev.labels.get(), cosine, out_ids,
-            out_d, r.nq);
+            p.q.get(), dim, o.dev.rows.get(), ck.get(), cs.get(), static_cast<int>(r.k), ip, o.dev.labels.get(), cosine,
+            out_ids, out_d, r.nq);
         QG_LAUNCH_CHECK();
         finish(p);
         return;

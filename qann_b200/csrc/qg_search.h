@@ -130,8 +130,8 @@ void nearest_lists(const IvfView& v, const IvfSearchArgs& s, int nq, int P, uint
 // The k' = s.kp best candidates of each query, as sorted (key64, slot) lists
 // (key64 = key(dist) << 32 | push index; 0xFFFF... marks an empty entry).
 void ivf_candidates(const IvfView& v, const IvfSearchArgs& s, uint64_t* out_key, uint32_t* out_slot, cudaStream_t st);
-// Coarse assignment through the tensor cores (qg_mm.cu): the P nearest lists
-// of each query by exact score, ties by list, from BF16 estimates with an
+// Coarse assignment through the tensor cores (qg_coarse.cu): the P nearest lists
+// of each query by exact score, ties by list, from F16 estimates with an
 // error bound and an exact recheck; queries with too many near-ties are
 // listed in redo_q for the exact path. use_tensor_coarse: whether the batch
 // goes this way (the process-wide tensor-filter mode and the work's size).
@@ -149,10 +149,6 @@ int64_t tensor_coarse_candidates();
 // timeout is flagged in *err_dev for the caller to read with the results.
 void coarse_probes_mm(const IvfView& v, const float* q, int nq, int P, uint32_t* probe, float* pdist,
                       std::vector<int>& redo_q, cudaStream_t st, int* err_dev = nullptr);
-// Rows scaled by powers of two (2^exps) and rounded to f16 (zero-padded to
-// dpad, a multiple of 8), with their float squared norms (unscaled).
-void prepare_f16_rows(const float* rows, size_t n, int dim, DevBuf<uint16_t>& f16, DevBuf<float>& sq,
-                      DevBuf<int>& exps, int& dpad, cudaStream_t st);
 
 // The scan's shape autotuner: on (1, the default) it times the candidate
 // shapes on the first large search of each problem key; off (0) every search

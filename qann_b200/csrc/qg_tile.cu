@@ -55,7 +55,11 @@ constexpr float kOpen = 3.402823466e+38f;   // threshold of a query that has non
 constexpr int kNearestCap = 256;            // candidates of a query in nearest mode
 
 // What the epilogue does with an accumulator.
-enum TileMode { kNearest };
+enum TileMode {
+    kNearest,   // append rows below the running upper bound of each query's nearest
+    kFilter,    // append rows below each query's threshold
+    kStore,     // write the products
+};
 
 struct TileArgs {
     int nq;
@@ -69,11 +73,14 @@ struct TileArgs {
     const float* run_slack;  // per 32 base rows: 2 c max|x|^2 (+inf when one of them is extreme), padded alike
     const float* qmul;       // per query: mult 2^-(qe+xe)
     const float* qslack;     // per query: 2 c |q|^2 + 2 g
-    uint32_t* thr_key;       // per query: key of the smallest upper bound so far
+    uint32_t* thr_key;       // per query: key of its threshold (nearest: the smallest upper bound so far)
     uint32_t* cand_count;    // per query
     uint2* cand;             // per query, cap entries: (lower bound, row)
     int cap;
     int* err;
+    float* store;            // kStore: acc(q, row) at store[q * ld + row - n0], ncols columns
+    size_t ld;
+    int ncols;
 };
 
 // Where the pipeline's parts lie in shared memory. Up to two K blocks (d <=
@@ -176,11 +183,11 @@ __device__ __forceinline__ void keep_below(uint32_t bits, uint32_t row, float th
 // the other EPI warps read the accumulators. 256 x 128 tiles: a base row that
 // comes from L2 serves 256 queries (32 KB a tile of 128 dims; a 128 x 256
 // tile needs 64 KB), and four halves fill TMEM, so that the epilogue of one
-// tile runs under the MMAs of the next. Bound by the MMAs and their issue,
-// then by the epilogue's appends: 131,072 queries against 4,096 / 16,384 rows
-// of 128 dims in 248 / 710 us (555 / 774 TFLOP/s counted once, the scout
-// tiles on top), 157 / 572 us with an epilogue that reads nothing; 768 dims
-// 831 us (992 TFLOP/s), there bound by L2, as both operands are streamed.
+// tile runs under the MMAs of the next. Bound by the epilogue: 131,072 queries
+// against 4,096 / 16,384 rows of 128 dims in 220 / 605 us (624 / 909 TFLOP/s
+// counted once, the scout tiles on top), 156 / 507 us if no row passed and 117
+// / 378 us with an epilogue that reads nothing; 768 dims 786 us (1,050
+// TFLOP/s), there bound by L2, as both operands are streamed.
 template <int EPI, int MODE>
 __global__ void __launch_bounds__(tile_threads<EPI>(), 1)
     k_tile(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, TileArgs a) {
@@ -207,7 +214,7 @@ __global__ void __launch_bounds__(tile_threads<EPI>(), 1)
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(empty_x + kTermBufs);
     volatile int* abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // (warp-uniform)
     if (threadIdx.x == 0) {
         for (int s = 0; s < S; ++s) {
             mbar_init(&full_r[s], 1);
@@ -237,145 +244,153 @@ __global__ void __launch_bounds__(tile_threads<EPI>(), 1)
     const int total = a.mtiles * (a.ntiles + a.scout);
     const int per = (total + gridDim.x - 1) / gridDim.x;   // this CTA's tiles: [t_begin, t_end)
     const int t_begin = min(total, static_cast<int>(blockIdx.x) * per), t_end = min(total, t_begin + per);
+    // What the loader and the MMA warps do between two barriers is not hidden by
+    // the copies and MMAs they issue, so it is kept short: ring positions and
+    // parities are carried (a division by the ring's length per K block held the
+    // whole kernel to 1.1k cycles a block), the warps run converged and one elected
+    // lane issues (addresses and descriptors stay in uniform registers: 179 ns a
+    // K block of 4 MMAs against 310 ns from a branch on the lane index, of which
+    // the MMAs are 136), and each half of the query tile has its own MMA warp.
     auto fail = [&] {
         *abort = 1;
-        atomicExch(a.err, 2);
+        if (lane == 0) atomicExch(a.err, 2);
     };
-
-    // The loader and the MMA warp are one thread each, and what they do between
-    // two barriers bounds the pipeline: ring positions and parities are carried
-    // (a division by the ring's length per K block held the whole kernel to 1.1k
-    // cycles a block), and matrix descriptors are made once and offset.
     if (warp == 0) {
-        if (lane == 0) {
-            int s = 0, cur_m = -1, ab = 1;
-            uint32_t rpar = 1, apar = 0;   // parities waited for: a fresh barrier passes the first wait for 1
-            uint32_t loads = 0, aloads = 0, xloads = 0, xpar = 1;
-            int xb = 0;
-            bool ok = true;
-            TileWalk w(t_begin, a);
-            for (int t = t_begin; t < t_end && ok && !*abort; ++t, w.next(a)) {
-                const int mt = w.mt, nt = w.nt;
-                if (pipe.resident && mt != cur_m) {
-                    ab ^= 1;
-                    if (ab == 0) apar ^= 1;   // 1 for the first two loads
-                    if (!mbar_wait(&empty_a[ab], apar, abort)) {
-                        fail();
-                        break;
-                    }
+        int s = 0, cur_m = -1, ab = 1, xb = 0;
+        uint32_t rpar = 1, apar = 0, xpar = 1;   // parities waited for: a fresh barrier passes the first wait for 1
+        uint32_t loads = 0, aloads = 0, xloads = 0;
+        bool ok = true;
+        TileWalk w(t_begin, a);
+        for (int t = t_begin; t < t_end && ok && !*abort; ++t, w.next(a)) {
+            const int mt = w.mt, nt = w.nt;
+            if (pipe.resident && mt != cur_m) {
+                ab ^= 1;
+                if (ab == 0) apar ^= 1;   // 1 for the first two loads
+                if (!mbar_wait(&empty_a[ab], apar, abort)) {
+                    fail();
+                    break;
+                }
+                if (elect_one()) {
                     mbar_expect_tx(&full_a[ab], pipe.a_bytes);
                     for (int kb = 0; kb < a.kblocks; ++kb)
                         tma_load_2d(&tmA, sA + ab * pipe.a_bytes + kb * kABlock, &full_a[ab], kb * KA, mt * BM);
-                    ++aloads;
-                    cur_m = mt;
                 }
-                {   // the tile's row terms
-                    if (!mbar_wait(&empty_x[xb], xpar, abort)) {
-                        fail();
-                        break;
-                    }
+                __syncwarp();
+                ++aloads;
+                cur_m = mt;
+            }
+            if (MODE != kStore) {   // the tile's row terms
+                if (!mbar_wait(&empty_x[xb], xpar, abort)) {
+                    fail();
+                    break;
+                }
+                if (elect_one()) {
                     mbar_expect_tx(&full_x[xb], kTermBytes + (MODE == kNearest ? kSlackBytes : 0));
                     uint8_t* dst = terms + xb * kTermStride;
                     bulk_load(dst, a.xterm + a.n0 + static_cast<size_t>(nt) * BN, kTermBytes, &full_x[xb]);
                     if (MODE == kNearest)
                         bulk_load(dst + kTermBytes, a.run_slack + (a.n0 >> 5) + static_cast<size_t>(nt) * (BN / 32),
                                   kSlackBytes, &full_x[xb]);
-                    ++xloads;
-                    if (++xb == kTermBufs) {
-                        xb = 0;
-                        xpar ^= 1;
-                    }
                 }
-                for (int kb = 0; kb < a.kblocks; ++kb) {
-                    if (!mbar_wait(&empty_r[s], rpar, abort)) {
-                        fail();
-                        ok = false;
-                        break;
-                    }
+                __syncwarp();
+                ++xloads;
+                if (++xb == kTermBufs) {
+                    xb = 0;
+                    xpar ^= 1;
+                }
+            }
+            for (int kb = 0; kb < a.kblocks; ++kb) {
+                if (!mbar_wait(&empty_r[s], rpar, abort)) {
+                    fail();
+                    ok = false;
+                    break;
+                }
+                if (elect_one()) {
                     mbar_expect_tx(&full_r[s], pipe.stage_bytes);
                     uint8_t* dst = ring + s * pipe.stage_bytes;
                     tma_load_2d(&tmB, dst, &full_r[s], kb * KA, a.n0 + nt * BN);
                     if (!pipe.resident) tma_load_2d(&tmA, dst + kBBlock, &full_r[s], kb * KA, mt * BM);
-                    ++loads;
-                    if (++s == S) {
-                        s = 0;
-                        rpar ^= 1;
-                    }
+                }
+                __syncwarp();
+                ++loads;
+                if (++s == S) {
+                    s = 0;
+                    rpar ^= 1;
                 }
             }
-            // no copy may land after the CTA is gone: wait for the last load of each buffer
-            volatile int never = 0;
-            for (int i = 0; i < S && static_cast<uint32_t>(i) < loads; ++i) {
-                const uint32_t uses = (loads - i + S - 1) / S;   // of stage i
-                mbar_wait(&full_r[i], (uses - 1) & 1, &never);
-            }
-            for (int b = 0; b < 2 && static_cast<uint32_t>(b) < aloads; ++b)
-                mbar_wait(&full_a[b], ((aloads - b + 1) / 2 - 1) & 1, &never);
-            for (int b = 0; b < kTermBufs && static_cast<uint32_t>(b) < xloads; ++b)
-                mbar_wait(&full_x[b], ((xloads - b + kTermBufs - 1) / kTermBufs - 1) & 1, &never);
         }
+        // no copy may land after the CTA is gone: wait for the last load of each buffer
+        volatile int never = 0;
+        for (int i = 0; i < S && static_cast<uint32_t>(i) < loads; ++i) {
+            const uint32_t uses = (loads - i + S - 1) / S;   // of stage i
+            mbar_wait(&full_r[i], (uses - 1) & 1, &never);
+        }
+        for (int b = 0; b < 2 && static_cast<uint32_t>(b) < aloads; ++b)
+            mbar_wait(&full_a[b], ((aloads - b + 1) / 2 - 1) & 1, &never);
+        for (int b = 0; b < kTermBufs && static_cast<uint32_t>(b) < xloads; ++b)
+            mbar_wait(&full_x[b], ((xloads - b + kTermBufs - 1) / kTermBufs - 1) & 1, &never);
     } else if (warp <= 2) {
-        // one warp per half of the query tile: what a thread does between its
-        // MMAs is not hidden by them (290 ns a K block for 8 MMAs of 33 ns), so
-        // two threads issue
-        if (lane == 0) {
-            const int h = warp - 1;
-            const uint32_t idesc = idesc_f16_f32(128, BN);
-            const uint64_t ring_d = sw128_desc(smem_u32(ring));
-            const uint64_t a_d = sw128_desc(smem_u32(sA) + h * (kABlock / 2));
-            const uint32_t stage_off = pipe.stage_bytes >> 4, abuf_off = pipe.a_bytes >> 4;   // (in descriptor units)
-            int s = 0, cur_m = -1, ab = 1, acc = 0;
-            uint32_t rpar = 0, apar = 1, tpar = 1;
-            bool ok = true;
-            TileWalk w(t_begin, a);
-            for (int t = t_begin; t < t_end && ok && !*abort; ++t, w.next(a)) {
-                const int mt = w.mt;
-                if (pipe.resident && mt != cur_m) {
-                    if (cur_m >= 0) mma_commit(&empty_a[ab]);   // free once its MMAs finish
-                    ab ^= 1;
-                    if (ab == 0) apar ^= 1;   // 0 for the first two
-                    if (!mbar_wait(&full_a[ab], apar, abort)) {
-                        fail();
-                        break;
-                    }
-                    cur_m = mt;
-                }
-                if (!mbar_wait(&tempty[2 * acc + h], tpar, abort)) {
+        const int h = warp - 1;
+        const uint32_t idesc = idesc_f16_f32(128, BN);
+        const uint64_t ring_d = sw128_desc(smem_u32(ring));
+        const uint64_t a_d = sw128_desc(smem_u32(sA) + h * (kABlock / 2));
+        const uint32_t stage_off = pipe.stage_bytes >> 4, abuf_off = pipe.a_bytes >> 4;   // (in descriptor units)
+        int s = 0, cur_m = -1, ab = 1, acc = 0;
+        uint32_t rpar = 0, apar = 1, tpar = 1;
+        bool ok = true;
+        TileWalk w(t_begin, a);
+        for (int t = t_begin; t < t_end && ok && !*abort; ++t, w.next(a)) {
+            const int mt = w.mt;
+            if (pipe.resident && mt != cur_m) {
+                if (cur_m >= 0 && elect_one()) mma_commit(&empty_a[ab]);   // free once its MMAs finish
+                __syncwarp();
+                ab ^= 1;
+                if (ab == 0) apar ^= 1;   // 0 for the first two
+                if (!mbar_wait(&full_a[ab], apar, abort)) {
                     fail();
                     break;
                 }
-                const bool live = mt * BM + 128 * h < a.nq;   // (a half without queries is left out)
-                const uint32_t td = tmem + acc * 256 + h * 128;
-                for (int kb = 0; kb < a.kblocks; ++kb) {
-                    if (!mbar_wait(&full_r[s], rpar, abort)) {
-                        fail();
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after();
-                    const uint64_t bd = ring_d + s * stage_off;
-                    const uint64_t ad = pipe.resident ? a_d + ab * abuf_off + kb * (kABlock >> 4)
-                                                      : bd + ((kBBlock + h * (kABlock / 2)) >> 4);
-                    const int ks1 = live ? min(4, a.ksteps - 4 * kb) : 0;
+                cur_m = mt;
+            }
+            if (!mbar_wait(&tempty[2 * acc + h], tpar, abort)) {
+                fail();
+                break;
+            }
+            const bool live = mt * BM + 128 * h < a.nq;   // (a half without queries is left out)
+            const uint32_t td = tmem + acc * 256 + h * 128;
+            for (int kb = 0; kb < a.kblocks; ++kb) {
+                if (!mbar_wait(&full_r[s], rpar, abort)) {
+                    fail();
+                    ok = false;
+                    break;
+                }
+                tc_fence_after();
+                const uint64_t bd = ring_d + s * stage_off;
+                const uint64_t ad = pipe.resident ? a_d + ab * abuf_off + kb * (kABlock >> 4)
+                                                  : bd + ((kBBlock + h * (kABlock / 2)) >> 4);
+                const int ks1 = live ? min(4, a.ksteps - 4 * kb) : 0;
+                if (elect_one()) {
 #pragma unroll
                     for (int ks = 0; ks < 4; ++ks)   // 32 bytes of K a step
-                        if (ks < ks1) mma_bf16(td, ad + 2 * ks, bd + 2 * ks, idesc, kb > 0 || ks > 0);
+                        if (ks < ks1) mma_f16(td, ad + 2 * ks, bd + 2 * ks, idesc, kb > 0 || ks > 0);
                     mma_commit(&empty_r[s]);
-                    if (++s == S) {
-                        s = 0;
-                        rpar ^= 1;
-                    }
+                    if (kb == a.kblocks - 1) mma_commit(&tfull[2 * acc + h]);
                 }
-                if (!ok) break;
-                mma_commit(&tfull[2 * acc + h]);
-                acc ^= 1;
-                if (acc == 0) tpar ^= 1;
+                __syncwarp();
+                if (++s == S) {
+                    s = 0;
+                    rpar ^= 1;
+                }
             }
-            // every MMA done before TMEM is freed
-            volatile int never = 0;
-            mma_commit(&mma_done[h]);
-            mbar_wait(&mma_done[h], 0, &never);
+            if (!ok) break;
+            acc ^= 1;
+            if (acc == 0) tpar ^= 1;
         }
+        // every MMA done before TMEM is freed
+        volatile int never = 0;
+        if (elect_one()) mma_commit(&mma_done[h]);
+        __syncwarp();
+        mbar_wait(&mma_done[h], 0, &never);
     } else {
         const int ew = warp - 3;      // 0..EPI-1
         const int quad = warp & 3;    // this warp's TMEM lanes: 32 * quad ..
@@ -383,14 +398,12 @@ __global__ void __launch_bounds__(tile_threads<EPI>(), 1)
         constexpr int kRuns = kCols / 32;
         const int half = (ew >> 2) & 1, col0 = (ew >> 3) * kCols;
         uint2* slot = slots + ew * 32 + lane;   // entry i at slot[i * EPI * 32]
-        constexpr float kInf = __builtin_huge_valf();
-
         uint32_t sp = smem_u32(slot);                                  // the next free place,
         const uint32_t room = sp + (kSlots - 3) * EPI * 32 * 8;        // the first with fewer than 4 after it
         int cur_m = -1, qi = 0;
         bool live = false;
         const float none = __int_as_float(0x7fffffff);   // (a lane without a query passes nothing)
-        float qsl = 0.0f, thr = none;
+        float qsl = 0.0f, thr = none;   // (lower bounds at or below thr pass)
         float2 mul2 = make_float2(0.0f, 0.0f);
         auto flush = [&] {
             const int cnt = static_cast<int>(sp - smem_u32(slot)) / (EPI * 32 * 8);
@@ -402,6 +415,7 @@ __global__ void __launch_bounds__(tile_threads<EPI>(), 1)
             sp = smem_u32(slot);
         };
         auto leave = [&] {   // done with the query tile
+            if (MODE == kStore) return;
             if (sp > smem_u32(slot)) flush();
             if (MODE == kNearest && live) atomicMin(&a.thr_key[qi], float_key(thr));
         };
@@ -415,30 +429,39 @@ __global__ void __launch_bounds__(tile_threads<EPI>(), 1)
                 cur_m = mt;
                 qi = mt * BM + half * 128 + quad * 32 + lane;
                 live = qi < a.nq;
-                const float mul = live ? -a.qmul[qi] : 0.0f;
+                const float mul = live && MODE != kStore ? -a.qmul[qi] : 0.0f;
                 mul2 = make_float2(mul, mul);
-                qsl = live ? a.qslack[qi] : 0.0f;
-                thr = live ? key_float(*reinterpret_cast<volatile uint32_t*>(a.thr_key + qi)) : none;
+                qsl = live && MODE == kNearest ? a.qslack[qi] : 0.0f;
+                if (MODE != kStore) thr = live ? key_float(*reinterpret_cast<volatile uint32_t*>(a.thr_key + qi)) : none;
             }
             const float* sx = reinterpret_cast<const float*>(terms + xb * kTermStride) + col0;
             const float* sslack = reinterpret_cast<const float*>(terms + xb * kTermStride + kTermBytes) + col0 / 32;
-            const bool ok = __all_sync(0xffffffffu, mbar_wait(&full_x[xb], xpar, abort) &&
+            const bool ok = __all_sync(0xffffffffu, (MODE == kStore || mbar_wait(&full_x[xb], xpar, abort)) &&
                                                         mbar_wait(&tfull[2 * acc + half], apar, abort));
             if (!ok) {
-                if (lane == 0) fail();
+                fail();
                 break;
             }
             tc_fence_after();
-#pragma unroll 1
-            for (int r = 0; r < kRuns; ++r) {
-                uint32_t v[32];
-                tmem_ld32(tmem + (static_cast<uint32_t>(quad * 32) << 16) +
-                              static_cast<uint32_t>(acc * 256 + half * 128 + col0 + 32 * r),
-                          v);
-                if (r == kRuns - 1) {   // this warp's last read: the accumulator goes back before the work on it
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&tempty[2 * acc + half]);
+            // one run of 32 columns: its products in v
+            auto run = [&](int r, uint32_t (&v)[32]) {
+                if constexpr (MODE == kStore) {
+                    const int c0 = w.nt * BN + col0 + 32 * r;
+                    if (live) {
+                        float* dst = a.store + static_cast<size_t>(qi) * a.ld + c0;
+                        if (c0 + 32 <= a.ncols && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+#pragma unroll
+                            for (int j = 0; j < 32; j += 4)
+                                *reinterpret_cast<float4*>(dst + j) =
+                                    make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]),
+                                                __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < 32; ++j)
+                                if (c0 + j < a.ncols) dst[j] = __uint_as_float(v[j]);
+                        }
+                    }
+                    return;
                 }
                 const float4* s4 = reinterpret_cast<const float4*>(sx + 32 * r);
                 // the lower bounds (over the products), two a packed FMA, and
@@ -461,7 +484,7 @@ __global__ void __launch_bounds__(tile_threads<EPI>(), 1)
                 if (MODE == kNearest) {
                     thr = live ? fminf(thr, __fadd_ru(low, __fadd_ru(sslack[r], qsl))) : none;
                 }
-                if (w.in_scout || !__any_sync(0xffffffffu, low <= thr)) continue;
+                if (w.in_scout || !__any_sync(0xffffffffu, low <= thr)) return;
                 const uint32_t r0 = static_cast<uint32_t>(a.n0 + w.nt * BN + col0 + 32 * r);   // base row of v[0]
                 // the groups in which some lane has one (one reduction: a vote and
                 // a branch per group cost eight latencies)
@@ -476,9 +499,41 @@ __global__ void __launch_bounds__(tile_threads<EPI>(), 1)
 #pragma unroll
                     for (int j = 4 * g; j < 4 * g + 4; ++j) keep_below(v[j], r0 + j, thr, sp, EPI * 32 * 8);
                 }
+            };
+            const uint32_t taddr = tmem + (static_cast<uint32_t>(quad * 32) << 16) +
+                                   static_cast<uint32_t>(acc * 256 + half * 128 + col0);
+            auto hand_back = [&] {   // this warp's last read: the accumulator goes back before the work on it
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&tempty[2 * acc + half]);
+            };
+            if constexpr (EPI == 8) {
+                // each run's load goes under the work on the run before it (64
+                // registers, which 8 warps have and 16 do not)
+                uint32_t va[32], vb[32];
+                tmem_ld32_start(taddr, va);
+#pragma unroll 1
+                for (int r = 0; r < kRuns; r += 2) {
+                    tmem_ld32_wait(va);
+                    tmem_ld32_start(taddr + 32 * (r + 1), vb);
+                    run(r, va);
+                    tmem_ld32_wait(vb);
+                    if (r + 2 < kRuns) tmem_ld32_start(taddr + 32 * (r + 2), va);
+                    else hand_back();
+                    run(r + 1, vb);
+                }
+            } else {
+#pragma unroll 1
+                for (int r = 0; r < kRuns; ++r) {
+                    uint32_t v[32];
+                    tmem_ld32(taddr + 32 * r, v);
+                    if (r == kRuns - 1) hand_back();
+                    run(r, v);
+                }
             }
             acc ^= 1;
             if (acc == 0) apar ^= 1;
+            if (MODE == kStore) continue;
             __syncwarp();   // the warp's reads of the row terms are done
             if (lane == 0) mbar_arrive(&empty_x[xb]);
             if (++xb == kTermBufs) {
@@ -594,7 +649,7 @@ struct TileBound {
     float c2;     // 2 c
     float g2;     // 2 g = g2 |q| M
     TileBound(int d, bool ip) {
-        const double C = std::ldexp(1.0, -10) + std::ldexp(1.0, -13) + d * std::ldexp(1.0, -21);
+        const double C = tile_error_factor(d);
         mult = ip ? 1.0f : 2.0f;
         xc = static_cast<float>(ip ? -0.5 * C : 1.0 - C);
         c2 = static_cast<float>(ip ? C : 2.0 * C);
@@ -606,14 +661,18 @@ struct TileBound {
 // -inf for extreme ones, which always pass), and per 32 rows the slack that
 // takes the smallest lower bound among them to an upper bound.
 __global__ void __launch_bounds__(256) k_tile_terms(const float* __restrict__ sq, size_t n, size_t npad, TileBound b,
-                                                    float* __restrict__ xterm, float* __restrict__ run_slack) {
+                                                    const uint64_t* __restrict__ allow,
+                                                    const uint64_t* __restrict__ deny, float* __restrict__ xterm,
+                                                    float* __restrict__ run_slack) {
     const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     constexpr float kInf = __builtin_huge_valf();
     float s = 0.0f;
     if (i < n) {
         const float x2 = sq[i];
         const bool ex = tile_extreme(x2);
-        xterm[i] = ex ? -kInf : __fmul_rn(b.xc, x2);
+        const bool refused = (allow && !((allow[i >> 6] >> (i & 63)) & 1ull)) ||
+                             (deny && ((deny[i >> 6] >> (i & 63)) & 1ull));
+        xterm[i] = refused ? kInf : ex ? -kInf : __fmul_rn(b.xc, x2);
         s = ex ? kInf : __fmul_ru(b.c2, x2);
     } else if (i < npad) {
         xterm[i] = kInf;
@@ -696,6 +755,246 @@ __global__ void __launch_bounds__(256) k_tile_pick(const float* __restrict__ q, 
     }
 }
 
+// ---- the k nearest ----------------------------------------------------------------
+//
+// The first rows' products are stored, and each query's threshold is the k-th
+// smallest upper bound among them; the rows below it open its candidate list.
+// The rows after them are taken in chunks of growing size: the engine appends
+// the rows whose lower bound is below the threshold, and a cut per query takes
+// the threshold to the k-th smallest upper bound of all its candidates and
+// drops those above. Only what is left at the end is scored exactly.
+
+// The k-th smallest upper bound of n candidates as a float on the lower
+// bounds' scale (kOpen when fewer than k are bounded), by one block. key: the
+// upper bounds' keys in shared memory (0xFFFFFFFF: unbounded).
+struct CutScratch {
+    int hist[kKeyHist];
+    uint32_t lo[8], hi[8], t;
+    int fin[8], count;
+};
+__device__ __forceinline__ float cut_threshold(const uint32_t* key, int n, int k, CutScratch& s) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    for (int t = threadIdx.x; t < kKeyHist; t += blockDim.x) s.hist[t] = 0;
+    if (threadIdx.x == 0) s.count = 0;
+    uint32_t lo = 0xFFFFFFFFu, hi = 0;
+    int fin = 0;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const uint32_t u = key[i];
+        if (u != 0xFFFFFFFFu) {
+            lo = min(lo, u);
+            hi = max(hi, u);
+            ++fin;
+        }
+    }
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    fin = __reduce_add_sync(0xffffffffu, fin);
+    if (lane == 0) {
+        s.lo[warp] = lo;
+        s.hi[warp] = hi;
+        s.fin[warp] = fin;
+    }
+    __syncthreads();
+    fin = 0;
+    for (int w = 0; w < nw; ++w) {
+        lo = min(lo, s.lo[w]);
+        hi = max(hi, s.hi[w]);
+        fin += s.fin[w];
+    }
+    const uint32_t T = block_threshold_u32(key, n, k, lo, hi, fin, s.hist, &s.t);
+    return T == 0xFFFFFFFFu ? kOpen : fminf(key_float(T), kOpen);
+}
+
+__device__ __forceinline__ uint32_t upper_key(float lb, float x2, float c2, float qslack) {
+    // (an extreme row's lower bound says nothing about where it is)
+    return tile_extreme(x2) ? 0xFFFFFFFFu : float_key(__fadd_ru(lb, __fadd_ru(__fmul_ru(c2, x2), qslack)));
+}
+
+// One block per query over the stored products of the first ncols rows: its
+// threshold and the rows at or below it. lbs, keys: ncols words of shared memory each.
+__global__ void __launch_bounds__(256) k_tile_seed(const float* __restrict__ acc, size_t ld, int ncols,
+                                                   const float* __restrict__ xterm, const float* __restrict__ sq,
+                                                   float c2, const float* __restrict__ qmul,
+                                                   const float* __restrict__ qslack, int k, int cap,
+                                                   uint32_t* __restrict__ thr_key, uint32_t* __restrict__ count,
+                                                   uint2* __restrict__ cand) {
+    extern __shared__ __align__(16) uint8_t sm_raw[];
+    __shared__ CutScratch s;
+    const int qi = blockIdx.x;
+    if (count[qi] > static_cast<uint32_t>(cap)) return;   // an extreme query
+    float* lbs = reinterpret_cast<float*>(sm_raw);
+    uint32_t* keys = reinterpret_cast<uint32_t*>(lbs + ncols);
+    const float* row = acc + static_cast<size_t>(qi) * ld;
+    const float mul = -qmul[qi], qs = qslack[qi];
+    for (int j = threadIdx.x; j < ncols; j += blockDim.x) {
+        const float lb = __fmaf_rn(mul, row[j], xterm[j]);
+        lbs[j] = lb;
+        // (refused rows: +inf)
+        keys[j] = lb <= kOpen ? upper_key(lb, sq[j], c2, qs) : 0xFFFFFFFFu;
+    }
+    __syncthreads();
+    const float T = cut_threshold(keys, ncols, k, s);
+    const int lane = threadIdx.x & 31;
+    for (int j0 = 0; j0 < ncols; j0 += blockDim.x) {   // (trip count block-uniform)
+        const int j = j0 + threadIdx.x;
+        const float lb = j < ncols ? lbs[j] : __builtin_huge_valf();
+        const unsigned in = __ballot_sync(0xffffffffu, lb <= T);
+        if (in == 0) continue;
+        int at = 0;
+        if (lane == 0) at = atomicAdd(&s.count, __popc(in));
+        at = __shfl_sync(0xffffffffu, at, 0) + __popc(in & ((1u << lane) - 1));
+        if (lb <= T && at < cap)
+            cand[static_cast<size_t>(qi) * cap + at] = make_uint2(__float_as_uint(lb), static_cast<uint32_t>(j));
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        count[qi] = static_cast<uint32_t>(s.count);
+        thr_key[qi] = float_key(s.count > cap ? -kOpen : T);   // (an overflowed list takes no more)
+    }
+}
+
+// The candidates of one query at or below their k-th smallest upper bound,
+// compacted to the front of list[] in shared memory (by one block; n of them
+// on entry); returns how many, and the threshold in T. key: n words of scratch.
+__device__ __forceinline__ int cut_list(uint2* list, uint32_t* key, int n, int k, const float* __restrict__ sq,
+                                        float c2, float qs, CutScratch& s, float& T) {
+    for (int i = threadIdx.x; i < n; i += blockDim.x)
+        key[i] = upper_key(__uint_as_float(list[i].x), sq[list[i].y], c2, qs);
+    __syncthreads();
+    T = cut_threshold(key, n, k, s);
+    const int lane = threadIdx.x & 31;
+    int kept = 0;
+    for (int i0 = 0; i0 < n; i0 += blockDim.x) {   // (trip count block-uniform)
+        const int i = i0 + threadIdx.x;
+        const uint2 e = i < n ? list[i] : make_uint2(0x7f800000u, 0u);
+        const bool in = i < n && __uint_as_float(e.x) <= T;
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        __syncthreads();   // this round's entries are read before any is overwritten
+        int at = 0;
+        if (lane == 0 && m) at = atomicAdd(&s.count, __popc(m));
+        at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1));
+        if (in) list[at] = e;   // (at < i0 + blockDim.x: only read entries)
+    }
+    __syncthreads();
+    kept = s.count;
+    return kept;
+}
+
+// After a chunk, one block per query: the list cut, its threshold lowered.
+__global__ void __launch_bounds__(128) k_tile_cut(const float* __restrict__ sq, float c2,
+                                                  const float* __restrict__ qslack, int k, int cap,
+                                                  uint32_t* __restrict__ thr_key, uint32_t* __restrict__ count,
+                                                  uint2* __restrict__ cand) {
+    extern __shared__ __align__(16) uint8_t sm_raw[];
+    __shared__ CutScratch s;
+    const int qi = blockIdx.x;
+    const uint32_t cnt = count[qi];
+    if (cnt > static_cast<uint32_t>(cap)) {   // overflowed: it takes no more
+        if (threadIdx.x == 0) thr_key[qi] = float_key(-kOpen);
+        return;
+    }
+    const int n = static_cast<int>(cnt);
+    uint2* list = reinterpret_cast<uint2*>(sm_raw);
+    uint32_t* key = reinterpret_cast<uint32_t*>(list + cap);
+    uint2* mine = cand + static_cast<size_t>(qi) * cap;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) list[i] = mine[i];
+    __syncthreads();
+    float T;
+    const int kept = cut_list(list, key, n, k, sq, c2, qslack[qi], s, T);
+    for (int i = threadIdx.x; i < kept; i += blockDim.x) mine[i] = list[i];
+    if (threadIdx.x == 0) {
+        count[qi] = static_cast<uint32_t>(kept);
+        thr_key[qi] = float_key(T);
+    }
+}
+
+// At the end, one block per query: the list cut, the rows left scored exactly
+// (a lane group of kG per row: 4 for an even dim at 8-byte alignment, else 8), and
+// the k smallest by (score, row) written in order. Up to 512 keys are ranked
+// over per-warp register-sorted runs (one barrier), more sorted by the block.
+template <int kG>
+__global__ void __launch_bounds__(256) k_tile_finish(const float* __restrict__ q, int d, const float* __restrict__ rows,
+                                                     bool ip, const float* __restrict__ sq, float c2,
+                                                     const float* __restrict__ qslack, int k, int cap,
+                                                     const uint32_t* __restrict__ count,
+                                                     const uint2* __restrict__ cand, uint32_t first,
+                                                     uint64_t* __restrict__ out_key, uint32_t* __restrict__ out_slot,
+                                                     uint32_t* __restrict__ redo, uint32_t* __restrict__ nredo) {
+    extern __shared__ __align__(16) uint8_t sm_raw[];
+    __shared__ CutScratch s;
+    const int qi = blockIdx.x;
+    const uint32_t cnt = count[qi];
+    if (cnt > static_cast<uint32_t>(cap)) {
+        if (threadIdx.x == 0) redo[atomicAdd(nredo, 1u)] = first + qi;
+        return;
+    }
+    const int n = static_cast<int>(cnt);
+    uint2* list = reinterpret_cast<uint2*>(sm_raw);
+    uint32_t* key = reinterpret_cast<uint32_t*>(list + cap);
+    const uint2* mine = cand + static_cast<size_t>(qi) * cap;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) list[i] = mine[i];
+    __syncthreads();
+    float T;
+    const int m = cut_list(list, key, n, k, sq, c2, qslack[qi], s, T);
+    // exact keys over the list, entry by entry (a group reads its row first)
+    uint64_t* ekey = reinterpret_cast<uint64_t*>(list);
+    const float* qv = q + static_cast<size_t>(qi) * d;
+    const int ngrp = blockDim.x / kG, grp = threadIdx.x / kG;
+    for (int i0 = 0; i0 < m; i0 += ngrp) {   // (block-uniform)
+        const int i = i0 + grp;
+        const bool act = i < m;
+        const uint32_t row = act ? list[i].y : 0u;   // idle groups score row 0 unused
+        const float* rp = rows + static_cast<size_t>(row) * d;
+        float sc;
+        if constexpr (kG == 4) sc = ip ? -exact_avx2_group4<false>(qv, rp, d) : exact_avx2_group4<true>(qv, rp, d);
+        else sc = ip ? -exact_avx2_group8<false, true>(qv, rp, d) : exact_avx2_group8<true, true>(qv, rp, d);
+        __syncwarp();
+        if (act && threadIdx.x % kG == 0) ekey[i] = (static_cast<uint64_t>(float_key_eq0(sc)) << 32) | row;
+    }
+    uint64_t* ok = out_key + static_cast<size_t>(qi) * k;
+    uint32_t* os = out_slot + static_cast<size_t>(qi) * k;
+    const int got = min(m, k);
+    for (int i = got + threadIdx.x; i < k; i += blockDim.x) {
+        ok[i] = ~0ull;
+        os[i] = 0xFFFFFFFFu;
+    }
+    __syncthreads();
+    if (m <= 512) {   // (block-uniform)
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        const int n_w = max(0, min(64, m - 64 * warp));
+        if (n_w > 0) warp_sort_keys_reg<2>(ekey + 64 * warp, n_w);
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int e = 32 * i + lane;
+            if (e >= n_w) continue;
+            const uint64_t kk = ekey[64 * warp + e];
+            int rank = 0;
+            for (int w = 0; 64 * w < m; ++w) {
+                const int len = min(64, m - 64 * w);
+                const uint64_t* rw = ekey + 64 * w;
+                int pos = 0;
+#pragma unroll
+                for (int step = 64; step > 0; step >>= 1)
+                    if (pos + step <= len && rw[pos + step - 1] < kk) pos += step;
+                rank += pos;
+            }
+            if (rank < k) {
+                ok[rank] = kk;
+                os[rank] = static_cast<uint32_t>(kk);
+            }
+        }
+        return;
+    }
+    const int np = next_pow2(m);   // (at most the list's power-of-two cap)
+    for (int i = m + threadIdx.x; i < np; i += blockDim.x) ekey[i] = ~0ull;
+    bitonic_sort_keys(ekey, np);
+    for (int i = threadIdx.x; i < got; i += blockDim.x) {
+        ok[i] = ekey[i];
+        os[i] = static_cast<uint32_t>(ekey[i]);
+    }
+}
+
 // ---- launching ------------------------------------------------------------------
 
 using EncodeTiled = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -734,10 +1033,10 @@ CUtensorMap make_map(const void* ptr, size_t rows, int dpad, int box_rows) {
 // of its 32 queries) or 16 (64 columns each). On the first launch of a problem
 // (mode, K blocks, query and base tiles by their power of two) with at least 8
 // tiles per SM, both are timed twice on the launch's own inputs and the faster
-// kept for the rest of the process; reset() puts the launch's outputs back
-// before each timed run, and the last run's are the launch's result. Both give
-// the same results. Launches that must not wait on the host use the problem's
-// pick if there is one, else 16.
+// kept for the rest of the process; save() keeps what the launch changes,
+// reset() puts it back before each further run, and the last run's is the
+// launch's result. Both give the same results. Launches that must not wait on
+// the host use the problem's pick if there is one, else 16.
 std::mutex g_tune_mu;
 std::map<uint64_t, int> g_tuned;   // problem key -> epilogue warps
 std::atomic<int> g_tune_on{1}, g_tune_last{8}, g_tune_force{0};
@@ -758,9 +1057,9 @@ void launch_as(int epi, const CUtensorMap& tmA, const CUtensorMap& tmB, const Ti
     g_tune_last.store(epi);
 }
 
-template <int MODE, class Reset>
+template <int MODE, class Save, class Reset>
 void launch_tile(const CUtensorMap& tmA, const CUtensorMap& tmB, const TileArgs& a, cudaStream_t st, bool may_tune,
-                 Reset reset) {
+                 Save save, Reset reset) {
     if (const int f = g_tune_force.load()) {
         launch_as<MODE>(f, tmA, tmB, a, st);
         return;
@@ -779,6 +1078,7 @@ void launch_tile(const CUtensorMap& tmA, const CUtensorMap& tmB, const TileArgs&
         launch_as<MODE>(16, tmA, tmB, a, st);
         return;
     }
+    save();
     cudaEvent_t e0, e1;
     QG_CUDA(cudaEventCreate(&e0));
     QG_CUDA(cudaEventCreate(&e1));
@@ -815,6 +1115,8 @@ int tile_last_epilogue_warps() { return g_tune_last.load(); }
 void set_tile_epilogue_warps(int warps) { g_tune_force.store(warps); }
 int tile_epilogue_warps() { return g_tune_force.load(); }
 
+double tile_error_factor(int dim) { return std::ldexp(1.0, -10) + std::ldexp(1.0, -13) + dim * std::ldexp(1.0, -21); }
+
 bool tile_supported(int dim) { return dim >= 1 && dim <= kMaxDim; }
 
 void tile_prepare_queries(const float* rows, size_t n, int dim, TileQueries& out, cudaStream_t st) {
@@ -849,6 +1151,25 @@ void tile_prepare_base(const float* rows, size_t n, int dim, TileBase& out, cuda
     QG_LAUNCH_CHECK();
 }
 
+void tile_store(const TileQueries& qs, const uint16_t* base_f16, size_t n, int dpad, float* store, size_t ld, int* err,
+                bool may_tune, cudaStream_t st) {
+    if (qs.n == 0 || n == 0) return;
+    TileArgs a{};
+    a.nq = static_cast<int>(qs.n);
+    a.kblocks = (dpad + KA - 1) / KA;
+    a.ksteps = (qs.dim + 15) / 16;
+    a.mtiles = static_cast<int>(ceil_div(qs.n, BM));
+    a.ntiles = static_cast<int>(ceil_div(n, BN));
+    a.group_n = 16;
+    a.err = err;
+    a.store = store;
+    a.ld = ld;
+    a.ncols = static_cast<int>(n);
+    const CUtensorMap tmA = make_map(qs.f16.get(), qs.n, qs.dpad, BM);
+    const CUtensorMap tmB = make_map(base_f16, n, dpad, BN);
+    launch_tile<kStore>(tmA, tmB, a, st, may_tune, [] {}, [] {});
+}
+
 // One launch over every base row per block of queries: a lane of the epilogue
 // owns one query, keeps its smallest upper bound so far and appends the rows
 // whose lower bound is at most that. Rows in random order give about ln(n)
@@ -864,7 +1185,8 @@ size_t tile_nearest(const float* q, const TileQueries& qs, const float* base_row
     const TileBound bound(d, false);
     const size_t npad = ceil_div(n, BN) * BN;
     DevBuf<float> xterm(npad, st), run_slack(npad / 32, st);
-    k_tile_terms<<<blocks_of(npad), 256, 0, st>>>(base.sq.get(), n, npad, bound, xterm.get(), run_slack.get());
+    k_tile_terms<<<blocks_of(npad), 256, 0, st>>>(base.sq.get(), n, npad, bound, nullptr, nullptr,
+                                                   xterm.get(), run_slack.get());
     QG_LAUNCH_CHECK();
     const size_t QB = 131072;   // queries per block: 268 MB of candidate lists
     const size_t qb = std::min(QB, nq);
@@ -881,8 +1203,7 @@ size_t tile_nearest(const float* q, const TileQueries& qs, const float* base_row
     // a base that stays in L2 is walked whole for each query tile, so that the
     // running bound meets every row; a larger one in groups
     // (a quarter of it, at most 16 tiles, for the bound alone, before any row is
-    // appended: 131,072 queries of 128 dims against 4,096 rows took 262 us
-    // with it and 286 us without, against 16,384 rows 710 and 962 us)
+    // appended: without it every query's first runs append)
     const bool whole = n * base.dpad * 2 <= (size_t{32} << 20);
     a.group_n = whole ? a.ntiles : 16;
     a.scout = whole ? std::min((a.ntiles + 3) / 4, 16) : 0;
@@ -911,7 +1232,7 @@ size_t tile_nearest(const float* q, const TileQueries& qs, const float* base_row
         const CUtensorMap tmA = make_map(qs.f16.get() + q0 * qs.dpad, nb, qs.dpad, BM);
         {
             KernelTimer kt("mm_filter", st);
-            launch_tile<kNearest>(tmA, tmB, a, st, /*may_tune=*/true, open);
+            launch_tile<kNearest>(tmA, tmB, a, st, /*may_tune=*/true, [] {}, open);
         }
         const unsigned blocks = blocks_of(nb, 8);
         if (g4)
@@ -921,6 +1242,122 @@ size_t tile_nearest(const float* q, const TileQueries& qs, const float* base_row
             k_tile_pick<8><<<blocks, 256, 0, st>>>(q + q0 * d, d, base_rows, nb, count.get(), cand.get(), kNearestCap,
                                                    thr.get(), static_cast<uint32_t>(q0), label + q0, redo.get(), nredo);
         QG_LAUNCH_CHECK();
+    }
+    uint32_t h[2] = {0, 0};
+    QG_CUDA(cudaMemcpyAsync(h, nredo, sizeof(h), cudaMemcpyDeviceToHost, st));
+    QG_CUDA(cudaStreamSynchronize(st));
+    require(h[1] == 0, "tensor-core filter: a pipeline wait timed out", kRuntimeError);
+    return h[0];
+}
+
+// The exact k nearest rows of each query (see "the k nearest" above).
+size_t tile_topk(const float* q, const TileQueries& qs, const float* base_rows, const TileBase& base, bool ip, size_t k,
+                 const uint64_t* allow, const uint64_t* deny, uint64_t* out_key, uint32_t* out_slot,
+                 DevBuf<uint32_t>& redo, cudaStream_t st) {
+    const size_t nq = qs.n, n = base.n;
+    const int d = base.dim;
+    if (nq == 0 || k == 0) return 0;
+    require(n >= 1 && n < (size_t{1} << 31) && nq < (size_t{1} << 31), "too many rows for the tensor-core path",
+            kUnsupported);
+    require(k <= kTileMaxK, "k too large for the tensor-core path", kUnsupported);
+    const TileBound bound(d, ip);
+    const size_t npad = ceil_div(n, BN) * BN;
+    DevBuf<float> xterm(npad, st), run_slack(npad / 32, st);
+    k_tile_terms<<<blocks_of(npad), 256, 0, st>>>(base.sq.get(), n, npad, bound, allow, deny, xterm.get(),
+                                                   run_slack.get());
+    QG_LAUNCH_CHECK();
+    // the candidate list: about 8 times what is wanted, so that a chunk of rows
+    // far from their average order does not overflow it
+    const int cap = std::clamp(next_pow2(static_cast<int>(8 * k)), 2048, 8192);
+    // the seed: enough rows that the first chunk's threshold lets few pass
+    const size_t seed = std::min<size_t>(n, std::clamp<size_t>(ceil_div(16 * k, BN) * BN, 2048, 8192));
+    const size_t ld = ceil_div(seed, 4) * 4;
+    // queries per block: the lists within 512 MB, the stored products within 256 MB
+    const size_t QB = std::min<size_t>({(size_t{512} << 20) / (cap * 8), (size_t{256} << 20) / (ld * 4), nq});
+    DevBuf<float> acc(QB * ld, st), qmul(QB, st), qslack(QB, st);
+    DevBuf<uint32_t> thr(QB, st), count(QB, st);
+    DevBuf<uint2> cand(QB * cap, st);
+    redo.alloc(nq + 2, st);   // the list, its length, and the error flag
+    uint32_t* const nredo = redo.get() + nq;
+    QG_CUDA(cudaMemsetAsync(nredo, 0, 2 * sizeof(uint32_t), st));
+    TileArgs a{};
+    a.kblocks = (base.dpad + KA - 1) / KA;
+    a.ksteps = (d + 15) / 16;
+    a.xterm = xterm.get();
+    a.run_slack = run_slack.get();
+    a.qmul = qmul.get();
+    a.qslack = qslack.get();
+    a.thr_key = thr.get();
+    a.cand_count = count.get();
+    a.cand = cand.get();
+    a.cap = cap;
+    a.err = reinterpret_cast<int*>(nredo + 1);
+    a.store = acc.get();
+    a.ld = ld;
+    const CUtensorMap tmB = make_map(base.f16.get(), n, base.dpad, BN);
+    const size_t seed_smem = seed * 8, cut_smem = static_cast<size_t>(cap) * 12;
+    allow_large_smem<k_tile_seed>();
+    allow_large_smem<k_tile_cut>();
+    allow_large_smem<k_tile_finish<4>>();
+    allow_large_smem<k_tile_finish<8>>();
+    const bool g4 = (d & 1) == 0 && (reinterpret_cast<uintptr_t>(q) & 7) == 0 &&
+                    (reinterpret_cast<uintptr_t>(base_rows) & 7) == 0;
+    // chunks grow so that about 320 rows pass in each, of a list of at least
+    // 2,048 (10,000 queries against 2M x 96, k = 100: the chunks and cuts of
+    // growth 3, 4 and 6 took 6.35, 6.32 and 6.52 ms)
+    const size_t growth = std::clamp<size_t>(1 + 320 / k, 2, 8);
+    for (size_t q0 = 0; q0 < nq; q0 += QB) {
+        const int nb = static_cast<int>(std::min(QB, nq - q0));
+        a.nq = nb;
+        a.mtiles = static_cast<int>(ceil_div(static_cast<size_t>(nb), BM));
+        k_tile_open<<<blocks_of(nb), 256, 0, st>>>(qs.sq.get() + q0, qs.exps.get() + q0, nb, bound, base.amax.get(), cap,
+                                                   qmul.get(), qslack.get(), thr.get(), count.get());
+        QG_LAUNCH_CHECK();
+        const CUtensorMap tmA = make_map(qs.f16.get() + q0 * qs.dpad, nb, qs.dpad, BM);
+        a.n0 = 0;
+        a.ncols = static_cast<int>(seed);
+        a.ntiles = static_cast<int>(ceil_div(seed, BN));
+        a.group_n = a.ntiles;
+        {
+            KernelTimer kt("mm_filter", st);
+            launch_tile<kStore>(tmA, tmB, a, st, /*may_tune=*/false, [] {}, [] {});
+        }
+        k_tile_seed<<<nb, 256, seed_smem, st>>>(acc.get(), ld, static_cast<int>(seed), xterm.get(), base.sq.get(),
+                                                bound.c2, qmul.get(), qslack.get(), static_cast<int>(k), cap, thr.get(),
+                                                count.get(), cand.get());
+        QG_LAUNCH_CHECK();
+        for (size_t n0 = seed; n0 < n;) {
+            const size_t n1 = std::min(n, std::min(n0 * growth, n0 + (size_t{1} << 22)));
+            a.n0 = static_cast<int>(n0);
+            a.ntiles = static_cast<int>(ceil_div(n1 - n0, BN));
+            a.group_n = 16;
+            {
+                KernelTimer kt("mm_filter", st);
+                // (a timed run's appends go over those of the run before it)
+                DevBuf<uint32_t> before;
+                launch_tile<kFilter>(
+                    tmA, tmB, a, st, /*may_tune=*/true,
+                    [&] {
+                        before.alloc(nb, st);
+                        QG_CUDA(cudaMemcpyAsync(before.get(), count.get(), nb * 4, cudaMemcpyDeviceToDevice, st));
+                    },
+                    [&] { QG_CUDA(cudaMemcpyAsync(count.get(), before.get(), nb * 4, cudaMemcpyDeviceToDevice, st)); });
+            }
+            n0 = n1;
+            if (n0 == n) break;
+            k_tile_cut<<<nb, 128, cut_smem, st>>>(base.sq.get(), bound.c2, qslack.get(), static_cast<int>(k), cap,
+                                                  thr.get(), count.get(), cand.get());
+            QG_LAUNCH_CHECK();
+        }
+        auto finish = [&](auto kernel) {
+            kernel<<<nb, 256, cut_smem, st>>>(q + q0 * d, d, base_rows, ip, base.sq.get(), bound.c2, qslack.get(),
+                                              static_cast<int>(k), cap, count.get(), cand.get(),
+                                              static_cast<uint32_t>(q0), out_key + q0 * k, out_slot + q0 * k, redo.get(),
+                                              nredo);
+            QG_LAUNCH_CHECK();
+        };
+        if (g4) finish(k_tile_finish<4>);
+        else finish(k_tile_finish<8>);
     }
     uint32_t h[2] = {0, 0};
     QG_CUDA(cudaMemcpyAsync(h, nredo, sizeof(h), cudaMemcpyDeviceToHost, st));

@@ -44,6 +44,24 @@ void tile_prepare_base(const float* rows, size_t n, int dim, TileBase& out, cuda
 size_t tile_nearest(const float* q, const TileQueries& qs, const float* base_rows, const TileBase& base,
                     uint32_t* label, DevBuf<uint32_t>& redo, cudaStream_t st);
 
+// The exact k nearest base rows of each query by (score, row), -0 == +0:
+// out_key[nq][k] (key_eq0(score) << 32 | row, ~0 when there are fewer) and
+// out_slot[nq][k], sorted. ip: the score is -(q . x), else squared L2. allow /
+// deny: bitmaps over the rows, or null. redo as above. k at most kTileMaxK.
+inline constexpr size_t kTileMaxK = 1024;
+size_t tile_topk(const float* q, const TileQueries& qs, const float* base_rows, const TileBase& base, bool ip, size_t k,
+                 const uint64_t* allow, const uint64_t* deny, uint64_t* out_key, uint32_t* out_slot,
+                 DevBuf<uint32_t>& redo, cudaStream_t st);
+
+// The raw products of the queries with n base rows (f16 rows of dpad
+// elements), row after row of `store` (ld apart). *err is set if a pipeline
+// wait times out; with may_tune false nothing waits on the host.
+void tile_store(const TileQueries& qs, const uint16_t* base_f16, size_t n, int dpad, float* store, size_t ld, int* err,
+                bool may_tune, cudaStream_t st);
+
+// C of the error bound (qg_tile.cu).
+double tile_error_factor(int dim);
+
 // The epilogue-warp autotuner: on or off, problems tuned, the last launch's pick.
 // force: 0 the autotuner's pick; 8 or 16 that epilogue on every launch.
 void set_tile_autotune(int on);

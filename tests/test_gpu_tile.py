@@ -77,3 +77,96 @@ def test_nearest_data(kind, warps, d):
     qb.set_tensor_filter(2)
     qb.set_filter_options(epilogue_warps=warps)
     assert lloyd(x, 500) == exact
+
+
+def both(fn):
+    qb.set_tensor_filter(0)
+    exact = fn()
+    qb.set_tensor_filter(2)
+    got, queries, redone = tensor_redone(fn)
+    np.testing.assert_array_equal(exact[0], got[0])
+    assert exact[1].tobytes() == got[1].tobytes()
+    return queries, redone
+
+
+@pytest.mark.parametrize("d", [1, 7, 63, 65, 96, 128, 129, 300, 768, 2048])
+@pytest.mark.parametrize("metric", [0, 1, 2])
+def test_flat_tile_edges(d, metric):
+    """Row counts around the seed and the tiles, queries around a half tile, k from 1 to the engine's largest."""
+    for n, nq, k in ((100, 3, 100), (2047, 129, 10), (2049, 256, 1), (9000, 257, 40), (9001, 5, 1024)):
+        idx = qb.FlatIndex(d, metric=qb.Metric(metric))
+        idx.add(rows_of("normal", d + n, n, d))
+        q = rows_of("normal", d + n + 1, nq, d)
+        queries, redone = both(lambda: idx.batch_query(q, k))
+        assert queries == nq
+        if d >= 96:
+            assert redone == 0
+
+
+@pytest.mark.parametrize("kind", ["mixture", "duplicates", "positive", "scales", "tiny", "huge", "odd_rows"])
+@pytest.mark.parametrize("metric", [0, 2])
+@pytest.mark.parametrize("warps", [8, 16])
+def test_flat_data(kind, metric, warps):
+    d, n = 100, 20_000
+    idx = qb.FlatIndex(d, metric=qb.Metric(metric))
+    idx.add(rows_of(kind, 8, n, d))
+    q = rows_of(kind, 9, 200, d)
+    qb.set_filter_options(epilogue_warps=warps)
+    for k in (1, 10, 100):
+        both(lambda: idx.batch_query(q, k))
+    idx.remove(np.arange(0, n, 5))
+    both(lambda: idx.batch_query(q, 10))
+    allowed = np.arange(0, n, 301)
+    both(lambda: idx.batch_query(q, 100, allowed=allowed))   # fewer allowed than wanted
+
+
+def test_flat_sorted_rows():
+    """Rows stored nearest last: every chunk holds more near rows than the one before it."""
+    d, n = 32, 60_000
+    rng = np.random.default_rng(3)
+    x = (rng.normal(size=(n, d)) * np.linspace(4.0, 0.1, n)[:, None]).astype(np.float32)
+    idx = qb.FlatIndex(d)
+    idx.add(x)
+    q = (0.1 * rng.normal(size=(70, d))).astype(np.float32)
+    both(lambda: idx.batch_query(q, 50))
+
+
+def test_flat_non_finite():
+    """Infinite and NaN components rank as the exact path ranks them."""
+    d, n = 48, 9000
+    x = rows_of("normal", 1, n, d)
+    x[5, 3] = np.inf
+    x[77, 0] = -np.inf
+    x[100, 1] = np.nan
+    idx = qb.FlatIndex(d)
+    idx.add(x)
+    q = rows_of("normal", 2, 66, d)
+    for k in (1, 20):
+        both(lambda: idx.batch_query(q, k))
+    q[3, 2] = np.inf
+    q[9, 7] = 1e30
+    both(lambda: idx.batch_query(q, 20))
+
+
+@pytest.mark.parametrize("d,m", [(129, None), (256, 64), (768, 64)])
+@pytest.mark.parametrize("metric", [0, 2])
+def test_coarse_wide(d, m, metric):
+    """The coarse step of dimensions past 128 on the tensor cores."""
+    if m is None:
+        d, m = 130, 26
+    x = rows_of("mixture", d, 20_000, d)
+    ivf = qb.IVFIndex(d, 400, 8, metric=qb.Metric(metric))
+    ivf.enable_pq(m, fast_scan=True)
+    ivf.train(x, max_iters=2, seed=5, clustering=qb.Clustering.Lloyd)
+    ivf.add(x)
+    q = rows_of("mixture", d + 1, 300, d)
+    for nprobe in (1, 40):
+        ivf.nprobe = nprobe
+        qb.set_tensor_filter(0)
+        exact = ivf.batch_query(q, 10)
+        qb.set_tensor_filter(2)
+        before = qb.tensor_filter_counts()["coarse_queries"]
+        got = ivf.batch_query(q, 10)
+        assert qb.tensor_filter_counts()["coarse_queries"] - before == 300
+        np.testing.assert_array_equal(exact[0], got[0])
+        assert exact[1].tobytes() == got[1].tobytes()
