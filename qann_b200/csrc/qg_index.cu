@@ -253,6 +253,24 @@ void ensure_device(FlatObj& o, cudaStream_t) {
     ++o.dev_gen;
 }
 
+const TileBase* tile_base(FlatObj& o) {
+    const size_t n = o.model.idmap.slots();
+    const int dim = static_cast<int>(o.model.dim);
+    if (n == 0 || !tile_supported(dim)) return nullptr;
+    const cudaStream_t st = resident_stream();
+    std::lock_guard<std::mutex> g(o.dev_mu);
+    DeviceRows& D = o.dev;
+    if (!D.tile_made) {
+        size_t free_b = 0, total_b = 0;
+        QG_CUDA(cudaMemGetInfo(&free_b, &total_b));
+        if (n * static_cast<size_t>((dim + 7) & ~7) * 2 > free_b / 4) return nullptr;
+        tile_prepare_base(D.rows.get(), n, dim, D.tile, st);
+        QG_CUDA(cudaStreamSynchronize(st));
+        D.tile_made = true;
+    }
+    return &D.tile;
+}
+
 void RefineObj::release_mapping() {
     if (registered) {
         cudaHostUnregister(registered);

@@ -33,6 +33,8 @@ struct DeviceRows {
     const float* ext = nullptr;        // rows read in place from host memory (a mapped file), or null
     DevBuf<int64_t> labels;
     DevBuf<uint64_t> deleted;
+    TileBase tile;                     // the rows' f16 copy for the tensor cores (tile_base), made by the
+    bool tile_made = false;            // first search that wants it and kept until the rows change
     const float* ptr() const { return ext ? ext : rows.get(); }
 };
 
@@ -143,6 +145,11 @@ cudaStream_t resident_stream();
 void ensure_device(IVFObj& o, cudaStream_t st);
 void ensure_device(FlatObj& o, cudaStream_t st);
 void ensure_device(RefineObj& o, cudaStream_t st);
+
+// The f16 copy of a FlatIndex's rows, kept with them (half their size): made
+// on the first call, or null when it would take more than a quarter of the free
+// device memory. Callers hold the object's lock and have called ensure_device.
+const TileBase* tile_base(FlatObj& o);
 
 // Packs plain codes (n x m bytes, lists concatenated in order) into the
 // device superblock layout. sb_list: the list of each superblock; voff: the

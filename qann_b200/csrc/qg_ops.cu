@@ -126,13 +126,19 @@ void count_tensor_filter(int64_t queries, int64_t redone) {
 void set_tensor_filter(int mode) { g_tensor_filter.store(mode); }
 int tensor_filter() { return g_tensor_filter.load(); }
 
-// The exact top-k either way; the tensor-core filter when the work is large
-// enough to pay for its f16 copy (or always, in mode 2), the FP32 tiles
-// otherwise.
-bool use_tensor_filter(size_t nq, size_t n, int dim, size_t k) {
+// The exact top-k either way; the tensor-core filter (or always, in mode 2)
+// once the exact tiles' work, which comes in tiles of 16 queries, passes 4e7
+// multiply-adds for rows whose f16 copy is kept. batch_query, k = 10, exact
+// tiles / filter: 1 query over 20,000 rows of 32 / 128 dims (1e7 / 4.1e7) 119 /
+// 126 and 147 / 127 us; 64 queries over 5,000 x 128 (4.1e7) 124 / 131, over
+// 20,000 x 32 (4.1e7) 148 / 129; 512 queries over 5,000 x 32 (8.2e7) 224 / 147.
+// Without a kept copy the call makes one: from 1.5e8, and for few queries only
+// up to 256 MB of it.
+bool use_tensor_filter(size_t nq, size_t n, int dim, size_t k, bool kept) {
     const int mode = g_tensor_filter.load();
+    const double work = static_cast<double>(std::max<size_t>(nq, 16)) * double(n) * dim;
     return mode > 0 && tile_supported(dim) && k <= kTileMaxK &&
-           (mode == 2 || (nq >= 64 && static_cast<double>(nq) * double(n) * dim >= 5e8));
+           (mode == 2 || work >= (kept ? 4e7 : nq >= 64 || double(n) * dim <= 1.28e8 ? 1.5e8 : HUGE_VAL));
 }
 
 // Nearest-centroid assignment on the tensor cores from 1e8 multiply-adds: the
@@ -190,7 +196,7 @@ __global__ void k_put_back(const uint64_t* __restrict__ key, const uint32_t* __r
 void flat_candidates(const float* q_dev, size_t nq, const float* rows_dev, size_t n, int dim, bool ip, size_t k,
                      const uint64_t* allow_dev, const uint64_t* deny_dev, uint64_t* out_key, uint32_t* out_slot,
                      cudaStream_t st, bool allow_mm, const TileBase* pre) {
-    if (!allow_mm || !use_tensor_filter(nq, n, dim, k)) {
+    if (!allow_mm || !use_tensor_filter(nq, n, dim, k, pre != nullptr)) {
         flat_candidates_fp32(q_dev, nq, rows_dev, n, dim, ip, k, allow_dev, deny_dev, out_key, out_slot, st);
         return;
     }
@@ -390,6 +396,11 @@ static void require_unsharded(const IndexObj& idx) {
             "this index holds one shard of its lists: search it through the sharded search", kLogicError);
 }
 
+// A FlatIndex's kept f16 copy for a search that goes through the filter with it, else null.
+static const TileBase* kept_base(FlatObj& o, size_t nq, size_t k) {
+    return use_tensor_filter(nq, o.model.idmap.slots(), static_cast<int>(o.model.dim), k, true) ? tile_base(o) : nullptr;
+}
+
 void search(IndexObj& idx, const SearchRequest& r, cudaStream_t st) {
     if (r.nq == 0) return;
     require_unsharded(idx);
@@ -459,7 +470,8 @@ void search(IndexObj& idx, const SearchRequest& r, cudaStream_t st) {
         DevBuf<uint64_t> ck(r.nq * r.k, st);
         DevBuf<uint32_t> cs(r.nq * r.k, st);
         flat_candidates(p.q.get(), r.nq, o.dev.rows.get(), o.model.idmap.slots(), dim, ip, r.k, p.filter.get(),
-                        r.filter ? nullptr : o.dev.deleted.get(), ck.get(), cs.get(), st);
+                        r.filter ? nullptr : o.dev.deleted.get(), ck.get(), cs.get(), st, true,
+                        kept_base(o, r.nq, r.k));
         k_finalize_flat<<<static_cast<unsigned>(ceil_div(r.nq * r.k, 256)), 256, 0, st>>>(
             p.q.get(), dim, o.dev.rows.get(), ck.get(), cs.get(), static_cast<int>(r.k), ip, o.dev.labels.get(), cosine,
             out_ids, out_d, r.nq);
@@ -508,7 +520,8 @@ void search(IndexObj& idx, const SearchRequest& r, cudaStream_t st) {
     } else {
         auto& b = static_cast<FlatObj&>(*o.base);
         flat_candidates(p.q.get(), r.nq, b.dev.rows.get(), b.model.idmap.slots(), dim, ip, kp, p.filter.get(),
-                        r.filter ? nullptr : b.dev.deleted.get(), ck.get(), cs.get(), st);
+                        r.filter ? nullptr : b.dev.deleted.get(), ck.get(), cs.get(), st, true,
+                        kept_base(b, r.nq, kp));
     }
     refine_candidates(p.q.get(), static_cast<int>(r.nq), dim, o.dev.ptr(), ck.get(), cs.get(), static_cast<int>(kp),
                       static_cast<int>(r.k), ip, o.dev.labels.get(), cosine, out_ids, out_d, st);

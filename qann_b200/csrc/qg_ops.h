@@ -91,8 +91,9 @@ int tensor_filter();
 // Queries answered through the filter so far, and those of them redone exactly
 // because their candidate lists overflowed.
 void tensor_filter_counts(int64_t* queries, int64_t* redone);
-// Whether an exact top-k of nq queries over n rows goes through the filter.
-bool use_tensor_filter(size_t nq, size_t n, int dim, size_t k);
+// Whether an exact top-k of nq queries over n rows goes through the filter;
+// kept: the rows' f16 copy is kept between calls.
+bool use_tensor_filter(size_t nq, size_t n, int dim, size_t k, bool kept = false);
 
 // Flat exact search over device rows: the k smallest by (score, slot) per
 // query, as (key64 = key_eq0(score) << 32 | slot) sorted lists of length k.

@@ -84,19 +84,22 @@ struct TileArgs {
 };
 
 // Where the pipeline's parts lie in shared memory. Up to two K blocks (d <=
-// 128) the query tile is resident, double buffered, and the ring stages one K
-// block of base rows; deeper rows stream both operands through the ring.
+// 128) the query tile is resident, double buffered when there are several, and
+// the ring stages one K block of base rows; deeper rows stream both operands
+// through the ring. (A batch of one query tile is bound by the base rows'
+// stream from HBM and has the whole ring for them.)
 struct TilePipe {
     bool resident;
-    uint32_t a_bytes, stage_bytes;
+    uint32_t a_bytes, stage_bytes, ring_at;
     int stages;
-    __host__ __device__ explicit TilePipe(int kblocks)
+    __host__ __device__ TilePipe(int kblocks, int mtiles)
         : resident(kblocks <= 2),
           a_bytes(resident ? kblocks * kABlock : 0),
           stage_bytes(resident ? kBBlock : kABlock + kBBlock),
-          stages(static_cast<int>((kPipeBytes - 2 * a_bytes) / stage_bytes)) {}
+          ring_at(mtiles > 1 ? 2 * a_bytes : a_bytes),
+          stages(static_cast<int>((kPipeBytes - ring_at) / stage_bytes)) {}
 };
-constexpr int kMaxStages = 8;
+constexpr int kMaxStages = 10;
 constexpr int kTermBufs = 8;                          // tiles whose row terms are staged ahead
 constexpr uint32_t kTermBytes = BN * 4, kSlackBytes = BN / 32 * 4;
 constexpr uint32_t kTermStride = (kTermBytes + kSlackBytes + 127) / 128 * 128;
@@ -195,10 +198,10 @@ __global__ void __launch_bounds__(tile_threads<EPI>(), 1)
     using namespace sm100;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* base = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
-    const TilePipe pipe(a.kblocks);
+    const TilePipe pipe(a.kblocks, a.mtiles);
     const int S = pipe.stages;
     uint8_t* sA = base;                       // resident: two query tiles
-    uint8_t* ring = base + 2 * pipe.a_bytes;
+    uint8_t* ring = base + pipe.ring_at;
     uint2* slots = reinterpret_cast<uint2*>(base + kPipeBytes);                        // [kSlots][EPI * 32]
     uint8_t* terms = reinterpret_cast<uint8_t*>(slots + static_cast<size_t>(EPI) * 32 * kSlots);   // [kTermBufs]
     uint64_t* bars = reinterpret_cast<uint64_t*>(terms + kTermBufs * kTermStride);
@@ -764,54 +767,110 @@ __global__ void __launch_bounds__(256) k_tile_pick(const float* __restrict__ q, 
 // the threshold to the k-th smallest upper bound of all its candidates and
 // drops those above. Only what is left at the end is scored exactly.
 
-// The k-th smallest upper bound of n candidates as a float on the lower
-// bounds' scale (kOpen when fewer than k are bounded), by one block. key: the
-// upper bounds' keys in shared memory (0xFFFFFFFF: unbounded).
+// A threshold at or just above the k-th smallest of n upper bounds (kOpen when
+// fewer than k are finite), by one block; ub: the bounds in shared memory. They
+// are counted into 1,024 equal intervals of their range, and the interval that
+// holds the k-th is cut again while it holds many more than are wanted; the
+// threshold is the largest bound in the last one. (Intervals of the bounds'
+// ordered bits took in 6 times too many when the range crosses zero.)
 struct CutScratch {
     int hist[kKeyHist];
-    uint32_t lo[8], hi[8], t;
-    int fin[8], count;
+    float lo[8], hi[8];
+    int fin[8], pick[3], count;
 };
-__device__ __forceinline__ float cut_threshold(const uint32_t* key, int n, int k, CutScratch& s) {
+__device__ __forceinline__ float cut_threshold(const float* ub, int n, int k, CutScratch& s) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int t = threadIdx.x; t < kKeyHist; t += blockDim.x) s.hist[t] = 0;
+    constexpr float kInf = __builtin_huge_valf();
     if (threadIdx.x == 0) s.count = 0;
-    uint32_t lo = 0xFFFFFFFFu, hi = 0;
-    int fin = 0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const uint32_t u = key[i];
-        if (u != 0xFFFFFFFFu) {
-            lo = min(lo, u);
-            hi = max(hi, u);
-            ++fin;
+    // the range and number of the bounds that in() admits
+    auto range = [&](auto in, float& lo, float& hi, int& fin) {
+        lo = kInf;
+        hi = -kInf;
+        fin = 0;
+        for (int i = threadIdx.x; i < n; i += blockDim.x) {
+            const float u = ub[i];
+            if (in(u)) {
+                lo = fminf(lo, u);
+                hi = fmaxf(hi, u);
+                ++fin;
+            }
         }
+        for (int o = 16; o > 0; o >>= 1) {
+            lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+            hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+        }
+        fin = __reduce_add_sync(0xffffffffu, fin);
+        __syncthreads();   // (the scratch of an earlier call is read)
+        if (lane == 0) {
+            s.lo[warp] = lo;
+            s.hi[warp] = hi;
+            s.fin[warp] = fin;
+        }
+        for (int t = threadIdx.x; t < kKeyHist; t += blockDim.x) s.hist[t] = 0;
+        __syncthreads();
+        fin = 0;
+        for (int w = 0; w < nw; ++w) {
+            lo = fminf(lo, s.lo[w]);
+            hi = fmaxf(hi, s.hi[w]);
+            fin += s.fin[w];
+        }
+    };
+    float lo, hi;
+    int fin, need = k;
+    range([](float u) { return u <= kOpen; }, lo, hi, fin);
+    if (fin < k) return kOpen;   // (block-uniform, as everything below)
+    for (int level = 0; level < 3; ++level) {
+        const float scale = __fdiv_rn(static_cast<float>(kKeyBins), __fsub_rn(hi, lo));
+        if (fin - need <= k / 8 || !(scale > 0.0f && scale <= kOpen)) break;
+        const float from = lo, to = hi;
+        // (monotone in u: the subtraction, the product and the conversion are)
+        auto bin = [&](float u) { return min(kKeyBins - 1, __float2int_rd(__fmul_rn(__fsub_rn(u, from), scale))); };
+        for (int i = threadIdx.x; i < n; i += blockDim.x) {
+            const float u = ub[i];
+            if (u >= from && u <= to) {
+                const int b = bin(u);
+                atomicAdd(&s.hist[b + (b >> 5)], 1);
+            }
+        }
+        __syncthreads();
+        if (warp == 0) {   // lane l owns bins 32 l .. 32 l + 31
+            int own = 0;
+#pragma unroll 8
+            for (int b = 0; b < 32; ++b) own += s.hist[33 * lane + b];
+            int incl = own;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += t;
+            }
+            const int excl = incl - own;
+            if (excl < need && need <= incl) {
+                int acc = excl;
+                for (int b = 0; b < 32; ++b) {
+                    const int c = s.hist[33 * lane + b];
+                    if (acc + c >= need) {
+                        s.pick[0] = 32 * lane + b;
+                        s.pick[1] = acc;
+                        break;
+                    }
+                    acc += c;
+                }
+            }
+        }
+        __syncthreads();
+        const int pick = s.pick[0];
+        need -= s.pick[1];
+        range([&](float u) { return u >= from && u <= to && bin(u) == pick; }, lo, hi, fin);
     }
-    lo = __reduce_min_sync(0xffffffffu, lo);
-    hi = __reduce_max_sync(0xffffffffu, hi);
-    fin = __reduce_add_sync(0xffffffffu, fin);
-    if (lane == 0) {
-        s.lo[warp] = lo;
-        s.hi[warp] = hi;
-        s.fin[warp] = fin;
-    }
-    __syncthreads();
-    fin = 0;
-    for (int w = 0; w < nw; ++w) {
-        lo = min(lo, s.lo[w]);
-        hi = max(hi, s.hi[w]);
-        fin += s.fin[w];
-    }
-    const uint32_t T = block_threshold_u32(key, n, k, lo, hi, fin, s.hist, &s.t);
-    return T == 0xFFFFFFFFu ? kOpen : fminf(key_float(T), kOpen);
+    return hi;   // need of the bounds in [lo, hi] and k of all are at or below it
 }
 
-__device__ __forceinline__ uint32_t upper_key(float lb, float x2, float c2, float qslack) {
+__device__ __forceinline__ float upper_bound(float lb, float x2, float c2, float qslack) {
     // (an extreme row's lower bound says nothing about where it is)
-    return tile_extreme(x2) ? 0xFFFFFFFFu : float_key(__fadd_ru(lb, __fadd_ru(__fmul_ru(c2, x2), qslack)));
+    return tile_extreme(x2) ? __builtin_huge_valf() : __fadd_ru(lb, __fadd_ru(__fmul_ru(c2, x2), qslack));
 }
 
 // One block per query over the stored products of the first ncols rows: its
-// threshold and the rows at or below it. lbs, keys: ncols words of shared memory each.
+// threshold and the rows at or below it. lbs, ub: ncols floats of shared memory each.
 __global__ void __launch_bounds__(256) k_tile_seed(const float* __restrict__ acc, size_t ld, int ncols,
                                                    const float* __restrict__ xterm, const float* __restrict__ sq,
                                                    float c2, const float* __restrict__ qmul,
@@ -823,17 +882,17 @@ __global__ void __launch_bounds__(256) k_tile_seed(const float* __restrict__ acc
     const int qi = blockIdx.x;
     if (count[qi] > static_cast<uint32_t>(cap)) return;   // an extreme query
     float* lbs = reinterpret_cast<float*>(sm_raw);
-    uint32_t* keys = reinterpret_cast<uint32_t*>(lbs + ncols);
+    float* ub = lbs + ncols;
     const float* row = acc + static_cast<size_t>(qi) * ld;
     const float mul = -qmul[qi], qs = qslack[qi];
     for (int j = threadIdx.x; j < ncols; j += blockDim.x) {
         const float lb = __fmaf_rn(mul, row[j], xterm[j]);
         lbs[j] = lb;
         // (refused rows: +inf)
-        keys[j] = lb <= kOpen ? upper_key(lb, sq[j], c2, qs) : 0xFFFFFFFFu;
+        ub[j] = lb <= kOpen ? upper_bound(lb, sq[j], c2, qs) : __builtin_huge_valf();
     }
     __syncthreads();
-    const float T = cut_threshold(keys, ncols, k, s);
+    const float T = cut_threshold(ub, ncols, k, s);
     const int lane = threadIdx.x & 31;
     for (int j0 = 0; j0 < ncols; j0 += blockDim.x) {   // (trip count block-uniform)
         const int j = j0 + threadIdx.x;
@@ -855,13 +914,13 @@ __global__ void __launch_bounds__(256) k_tile_seed(const float* __restrict__ acc
 
 // The candidates of one query at or below their k-th smallest upper bound,
 // compacted to the front of list[] in shared memory (by one block; n of them
-// on entry); returns how many, and the threshold in T. key: n words of scratch.
-__device__ __forceinline__ int cut_list(uint2* list, uint32_t* key, int n, int k, const float* __restrict__ sq,
-                                        float c2, float qs, CutScratch& s, float& T) {
+// on entry); returns how many, and the threshold in T. ub: n floats of scratch.
+__device__ __forceinline__ int cut_list(uint2* list, float* ub, int n, int k, const float* __restrict__ sq, float c2,
+                                        float qs, CutScratch& s, float& T) {
     for (int i = threadIdx.x; i < n; i += blockDim.x)
-        key[i] = upper_key(__uint_as_float(list[i].x), sq[list[i].y], c2, qs);
+        ub[i] = upper_bound(__uint_as_float(list[i].x), sq[list[i].y], c2, qs);
     __syncthreads();
-    T = cut_threshold(key, n, k, s);
+    T = cut_threshold(ub, n, k, s);
     const int lane = threadIdx.x & 31;
     int kept = 0;
     for (int i0 = 0; i0 < n; i0 += blockDim.x) {   // (trip count block-uniform)
@@ -895,12 +954,12 @@ __global__ void __launch_bounds__(128) k_tile_cut(const float* __restrict__ sq, 
     }
     const int n = static_cast<int>(cnt);
     uint2* list = reinterpret_cast<uint2*>(sm_raw);
-    uint32_t* key = reinterpret_cast<uint32_t*>(list + cap);
+    float* ub = reinterpret_cast<float*>(list + cap);
     uint2* mine = cand + static_cast<size_t>(qi) * cap;
     for (int i = threadIdx.x; i < n; i += blockDim.x) list[i] = mine[i];
     __syncthreads();
     float T;
-    const int kept = cut_list(list, key, n, k, sq, c2, qslack[qi], s, T);
+    const int kept = cut_list(list, ub, n, k, sq, c2, qslack[qi], s, T);
     for (int i = threadIdx.x; i < kept; i += blockDim.x) mine[i] = list[i];
     if (threadIdx.x == 0) {
         count[qi] = static_cast<uint32_t>(kept);
@@ -930,12 +989,12 @@ __global__ void __launch_bounds__(256) k_tile_finish(const float* __restrict__ q
     }
     const int n = static_cast<int>(cnt);
     uint2* list = reinterpret_cast<uint2*>(sm_raw);
-    uint32_t* key = reinterpret_cast<uint32_t*>(list + cap);
+    float* ub = reinterpret_cast<float*>(list + cap);
     const uint2* mine = cand + static_cast<size_t>(qi) * cap;
     for (int i = threadIdx.x; i < n; i += blockDim.x) list[i] = mine[i];
     __syncthreads();
     float T;
-    const int m = cut_list(list, key, n, k, sq, c2, qslack[qi], s, T);
+    const int m = cut_list(list, ub, n, k, sq, c2, qslack[qi], s, T);
     // exact keys over the list, entry by entry (a group reads its row first)
     uint64_t* ekey = reinterpret_cast<uint64_t*>(list);
     const float* qv = q + static_cast<size_t>(qi) * d;
@@ -1305,7 +1364,8 @@ size_t tile_topk(const float* q, const TileQueries& qs, const float* base_rows, 
     // chunks grow so that about 320 rows pass in each, of a list of at least
     // 2,048 (10,000 queries against 2M x 96, k = 100: the chunks and cuts of
     // growth 3, 4 and 6 took 6.35, 6.32 and 6.52 ms)
-    const size_t growth = std::clamp<size_t>(1 + 320 / k, 2, 8);
+    // Few queries, whose chunks are short of work, grow faster.
+    const size_t growth = std::clamp<size_t>(1 + 320 / k, 2, nq <= 64 ? 32 : 8);
     for (size_t q0 = 0; q0 < nq; q0 += QB) {
         const int nb = static_cast<int>(std::min(QB, nq - q0));
         a.nq = nb;

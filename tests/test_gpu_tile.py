@@ -170,3 +170,46 @@ def test_coarse_wide(d, m, metric):
         assert qb.tensor_filter_counts()["coarse_queries"] - before == 300
         np.testing.assert_array_equal(exact[0], got[0])
         assert exact[1].tobytes() == got[1].tobytes()
+
+
+def test_flat_kept_copy_follows_the_rows():
+    """The f16 copy kept with a FlatIndex is made again after rows are added or removed."""
+    d = 64
+    x = rows_of("normal", 4, 50_000, d)
+    q = rows_of("normal", 5, 9, d)
+    idx = qb.FlatIndex(d)
+    idx.add(x[:30_000])
+    both(lambda: idx.batch_query(q, 10))
+    idx.add(x[30_000:] * np.float32(0.01))
+    both(lambda: idx.batch_query(q, 10))
+    idx.remove(np.arange(30_000, 50_000, 2))
+    both(lambda: idx.batch_query(q, 10))
+    refine = qb.RefineIndex(qb.FlatIndex(d), 4)
+    refine.add(x)
+    both(lambda: refine.batch_query(q, 10))
+
+
+def test_flat_concurrent_first_searches():
+    """Threads that search a fresh FlatIndex at the same time get the same answers (one of them makes the copy)."""
+    import threading
+    d = 48
+    x = rows_of("mixture", 6, 60_000, d)
+    q = rows_of("mixture", 7, 40, d)
+    qb.set_tensor_filter(0)
+    ref = qb.FlatIndex(d)
+    ref.add(x)
+    want = ref.batch_query(q, 10)
+    qb.set_tensor_filter(2)
+    idx = qb.FlatIndex(d)
+    idx.add(x)
+    got = [None] * 4
+    def work(i):
+        got[i] = idx.batch_query(q, 10)
+    ts = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    for g in got:
+        np.testing.assert_array_equal(g[0], want[0])
+        assert g[1].tobytes() == want[1].tobytes()
