@@ -15,7 +15,6 @@
 
 #include <algorithm>
 #include <cmath>
-#include <vector>
 
 namespace qg {
 
@@ -61,16 +60,44 @@ __device__ void ranked_out(uint64_t* key, int cnt, int P, const float* score_of,
     }
 }
 
-__global__ void __launch_bounds__(256, 6) k_coarse_recheck(const float* __restrict__ q, const float* __restrict__ q2,
-                                                        const int* __restrict__ qexp, const float* __restrict__ cent,
-                                                        const float* __restrict__ c2, const int* __restrict__ cexp,
-                                                        int nlist, int d, bool ip, float c_up, float c_lo,
-                                                        const float* __restrict__ accm, size_t ld, int P, int cap,
-                                                        uint32_t* __restrict__ probe, float* __restrict__ pdist,
-                                                        int* __restrict__ redo,
-                                                        unsigned long long* __restrict__ ncand) {
+// What the recheck of one query reads and writes.
+struct RecheckArgs {
+    const float *q, *q2;
+    const int* qexp;
+    const float *cent, *c2;
+    const int* cexp;
+    int nlist, d;
+    bool ip;
+    float c_up, c_lo;
+    const float* accm;
+    size_t ld;
+    int P;
+    uint32_t* probe;
+    float* pdist;
+    uint32_t *list, *nlist_redo;   // queries left to k_coarse_redo, and how many
+    int* nredone;                  // statistics: those queries,
+    unsigned long long* ncand;     // and the lists rescored exactly
+};
+
+// One query by one block, with room for cap candidates. can_defer: a query of
+// extreme norm, or with more candidates than that (too many near-ties), goes on
+// the list instead; otherwise cap holds every list.
+__device__ __forceinline__ void recheck_query(const RecheckArgs& ra, int qi, int cap, bool can_defer) {
     extern __shared__ __align__(16) uint8_t sm_raw[];
-    const int qi = blockIdx.x;
+    const float *q = ra.q, *q2 = ra.q2, *cent = ra.cent, *c2 = ra.c2, *accm = ra.accm;
+    const int *qexp = ra.qexp, *cexp = ra.cexp;
+    const int nlist = ra.nlist, d = ra.d, P = ra.P;
+    const bool ip = ra.ip;
+    const float c_up = ra.c_up, c_lo = ra.c_lo;
+    const size_t ld = ra.ld;
+    uint32_t* const probe = ra.probe;
+    float* const pdist = ra.pdist;
+    auto defer = [&] {
+        if (threadIdx.x == 0) {
+            ra.list[atomicAdd(ra.nlist_redo, 1u)] = static_cast<uint32_t>(qi);
+            atomicAdd(ra.nredone, 1);
+        }
+    };
     uint64_t* ckey = reinterpret_cast<uint64_t*>(sm_raw);             // cap
     float* qv = reinterpret_cast<float*>(ckey + cap);                   // d, 16-byte aligned
     uint32_t* ub = reinterpret_cast<uint32_t*>(qv + ((d + 3) & ~3));    // nlist
@@ -83,9 +110,9 @@ __global__ void __launch_bounds__(256, 6) k_coarse_recheck(const float* __restri
     // overflow): the relative bound does not hold, so such a query takes the
     // exact path and such a list is always rescored
     auto extreme = [](float x2) { return (x2 > 0.0f && x2 < 0x1p-60f) || !(x2 < 0x1p60f); };
-    const bool all = extreme(qq);   // rescored in full here when there is no exact path to send it to
-    if (all && redo) {
-        if (threadIdx.x == 0) redo[qi] = 1;
+    const bool all = extreme(qq);   // every list rescored
+    if (all && can_defer) {
+        defer();
         return;
     }
     for (int t = threadIdx.x; t < d; t += blockDim.x) qv[t] = q[static_cast<size_t>(qi) * d + t];
@@ -165,9 +192,9 @@ __global__ void __launch_bounds__(256, 6) k_coarse_recheck(const float* __restri
         if (lower_in(arow[j], c2[j], cexp[j])) push(j);
     __syncthreads();
     const int cnt = s_count;
-    if (threadIdx.x == 0 && ncand) atomicAdd(ncand, static_cast<unsigned long long>(cnt));
-    if (cnt > cap) {   // too many near-ties: this query takes the exact path (cap >= nlist when redo is null)
-        if (threadIdx.x == 0 && redo) redo[qi] = 1;
+    if (threadIdx.x == 0) atomicAdd(ra.ncand, static_cast<unsigned long long>(cnt));
+    if (cnt > cap) {   // (cap >= nlist when it cannot be deferred)
+        if (can_defer) defer();
         return;
     }
     // exact scores, one candidate per 8-lane group; each list's score is kept
@@ -228,6 +255,22 @@ __global__ void __launch_bounds__(256, 6) k_coarse_recheck(const float* __restri
     }
 }
 
+__global__ void __launch_bounds__(256, 6) k_coarse_recheck(RecheckArgs ra, int cap, bool can_defer) {
+    recheck_query(ra, blockIdx.x, cap, can_defer);
+}
+
+// The queries on the list, with room for every list: a few blocks that take
+// one after the other (none, nearly always, so the list is not read back to
+// the host to decide; the launch costs 3 us, the read-back cost the search a
+// wait of about 30).
+__global__ void __launch_bounds__(256) k_coarse_redo(RecheckArgs ra, int cap) {
+    const uint32_t n = *ra.nlist_redo;
+    for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {   // (block-uniform)
+        recheck_query(ra, static_cast<int>(ra.list[i]), cap, false);
+        __syncthreads();
+    }
+}
+
 static size_t coarse_recheck_smem(int nlist, int d, int cap) {
     return static_cast<size_t>(cap) * 8 + static_cast<size_t>((d + 3) & ~3) * 4 + static_cast<size_t>(nlist) * 4;
 }
@@ -236,18 +279,18 @@ static int coarse_cap(int nlist, int P) {
     return std::min(next_pow2(nlist), std::max(1024, next_pow2(4 * P)));
 }
 
-bool coarse_mm_supported(int nlist, int dim, int P, bool cent_prepared, bool no_readback) {
-    const int cap = no_readback ? next_pow2(nlist) : coarse_cap(nlist, P);
+bool coarse_mm_supported(int nlist, int dim, int P, bool cent_prepared) {
+    const int cap = next_pow2(nlist);
     return cent_prepared && tile_supported(dim) && P >= 1 && P <= nlist && nlist <= 16384 &&
            coarse_recheck_smem(nlist, dim, cap) <= 200 * 1024;
 }
 
-void coarse_probes_mm(const IvfView& v, const float* q, int nq, int P, uint32_t* probe, float* pdist,
-                      std::vector<int>& redo_q, cudaStream_t st, int* err_dev) {
-    const bool no_readback = err_dev != nullptr;
-    redo_q.clear();
+void coarse_probes_mm(const IvfView& v, const float* q, int nq, int P, uint32_t* probe, float* pdist, int* flags,
+                      bool hold_all, bool may_tune, cudaStream_t st) {
     if (nq == 0) return;
     const int d = v.dim, nlist = v.nlist;
+    allow_large_smem<k_coarse_recheck>();
+    allow_large_smem<k_coarse_redo>();
     const size_t QB = 65536;   // query blocks bound the score matrix
     for (size_t q0 = 0; q0 < static_cast<size_t>(nq); q0 += QB) {
         const int nb = static_cast<int>(std::min(QB, static_cast<size_t>(nq) - q0));
@@ -255,48 +298,50 @@ void coarse_probes_mm(const IvfView& v, const float* q, int nq, int P, uint32_t*
         tile_prepare_queries(q + q0 * d, nb, d, qs, st);
         const size_t ld = (static_cast<size_t>(nlist) + 3) & ~size_t{3};
         DevBuf<float> accm(static_cast<size_t>(nb) * ld, st);
-        DevBuf<int> redo, err;
-        DevBuf<unsigned long long> ncand;
-        if (!no_readback) {
-            redo.alloc(nb, st);
-            err.alloc(1, st);
-            ncand.alloc(1, st);
-            QG_CUDA(cudaMemsetAsync(ncand.get(), 0, sizeof(unsigned long long), st));
-            QG_CUDA(cudaMemsetAsync(redo.get(), 0, nb * sizeof(int), st));
-            QG_CUDA(cudaMemsetAsync(err.get(), 0, sizeof(int), st));
-        }
         {
             KernelTimer kt("coarse_mm", st);
-            tile_store(qs, v.cent_f16, nlist, v.cent_dpad, accm.get(), ld, no_readback ? err_dev : err.get(),
-                       /*may_tune=*/!no_readback, st);
+            tile_store(qs, v.cent_f16, nlist, v.cent_dpad, accm.get(), ld, flags + 2, may_tune, st);
         }
-        const int cap = no_readback ? next_pow2(nlist) : coarse_cap(nlist, P);   // no read-back: every list fits
-        const size_t rsm = coarse_recheck_smem(nlist, d, cap);
-        allow_large_smem<k_coarse_recheck>();
         const double C = tile_error_factor(d);
+        RecheckArgs ra{};
+        ra.q = q + q0 * d;
+        ra.q2 = qs.sq.get();
+        ra.qexp = qs.exps.get();
+        ra.cent = v.centroids;
+        ra.c2 = v.cent_sq;
+        ra.cexp = v.cent_exp;
+        ra.nlist = nlist;
+        ra.d = d;
+        ra.ip = v.ip_metric;
         // the bound's factors as floats rounded outwards
-        const float c_up = v.ip_metric ? std::nextafter(static_cast<float>(0.5 * C), 1.0f)
-                                       : std::nextafter(static_cast<float>(1.0 + C), 2.0f);
-        const float c_lo = std::nextafter(static_cast<float>(1.0 - C), 0.0f);
-        {
-            KernelTimer kt("coarse_recheck", st);
-            k_coarse_recheck<<<static_cast<unsigned>(nb), 256, rsm, st>>>(
-                q + q0 * d, qs.sq.get(), qs.exps.get(), v.centroids, v.cent_sq, v.cent_exp, nlist, d, v.ip_metric, c_up,
-                c_lo, accm.get(), ld, P, cap, probe + q0 * P, pdist + q0 * P, redo.get(), ncand.get());
+        ra.c_up = v.ip_metric ? std::nextafter(static_cast<float>(0.5 * C), 1.0f)
+                              : std::nextafter(static_cast<float>(1.0 + C), 2.0f);
+        ra.c_lo = std::nextafter(static_cast<float>(1.0 - C), 0.0f);
+        ra.accm = accm.get();
+        ra.ld = ld;
+        ra.P = P;
+        ra.probe = probe + q0 * P;
+        ra.pdist = pdist + q0 * P;
+        ra.nredone = flags + 3;
+        ra.ncand = reinterpret_cast<unsigned long long*>(flags + 4);
+        const int full = next_pow2(nlist);
+        const int cap = hold_all ? full : coarse_cap(nlist, P);
+        const bool defer = cap < full;
+        DevBuf<uint32_t> list;
+        if (defer) {
+            list.alloc(static_cast<size_t>(nb) + 1, st);
+            ra.list = list.get();
+            ra.nlist_redo = list.get() + nb;
+            QG_CUDA(cudaMemsetAsync(ra.nlist_redo, 0, sizeof(uint32_t), st));
+        }
+        KernelTimer kt("coarse_recheck", st);
+        k_coarse_recheck<<<static_cast<unsigned>(nb), 256, coarse_recheck_smem(nlist, d, cap), st>>>(ra, cap, defer);
+        QG_LAUNCH_CHECK();
+        if (defer) {
+            k_coarse_redo<<<static_cast<unsigned>(std::min(nb, 148)), 256, coarse_recheck_smem(nlist, d, full), st>>>(
+                ra, full);
             QG_LAUNCH_CHECK();
         }
-        if (no_readback) continue;   // the caller reads the flag with the results
-        int herr = 0;
-        unsigned long long hcand = 0;
-        std::vector<int> hredo(nb);
-        QG_CUDA(cudaMemcpyAsync(&hcand, ncand.get(), sizeof(hcand), cudaMemcpyDeviceToHost, st));
-        QG_CUDA(cudaMemcpyAsync(&herr, err.get(), sizeof(int), cudaMemcpyDeviceToHost, st));
-        QG_CUDA(cudaMemcpyAsync(hredo.data(), redo.get(), nb * sizeof(int), cudaMemcpyDeviceToHost, st));
-        QG_CUDA(cudaStreamSynchronize(st));
-        require(herr == 0, "tensor-core coarse step: a pipeline wait timed out", kRuntimeError);
-        count_tensor_coarse_candidates(static_cast<int64_t>(hcand));
-        for (int i = 0; i < nb; ++i)
-            if (hredo[i]) redo_q.push_back(static_cast<int>(q0) + i);
     }
 }
 

@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <cstring>
 #include <exception>
 #include <numeric>
 #include <thread>
@@ -256,8 +257,9 @@ namespace {
 struct Prepared {
     DevBuf<float> q;     // prepared queries (normalised for cosine)
     DevBuf<uint64_t> filter;
+    const float* qp = nullptr;   // them, or the caller's where nothing changes them
     DevBuf<int> err_own;
-    int* err = nullptr;  // [0] scan overflow, [1] zero cosine row, [2] tensor-core pipeline timeout
+    int* err = nullptr;  // kFlags ints (IvfSearchArgs::d_err)
 };
 } // namespace
 
@@ -267,23 +269,23 @@ static void prepare(IndexObj& idx, const SearchRequest& r, Prepared& p, cudaStre
     if (r.err_dev) {
         p.err = r.err_dev;
     } else {
-        p.err_own.alloc(3, st);
+        p.err_own.alloc(kFlags, st);
         p.err = p.err_own.get();
     }
-    QG_CUDA(cudaMemsetAsync(p.err, 0, 3 * sizeof(int), st));
-    DevBuf<float> raw;
+    QG_CUDA(cudaMemsetAsync(p.err, 0, kFlags * sizeof(int), st));
     const float* src = r.q;
     if (r.io == IoSpace::Host) {
-        raw.alloc(n, st);
-        QG_CUDA(cudaMemcpyAsync(raw.get(), r.q, n * sizeof(float), cudaMemcpyHostToDevice, st));
-        src = raw.get();
+        p.q.alloc(n, st);
+        QG_CUDA(cudaMemcpyAsync(p.q.get(), r.q, n * sizeof(float), cudaMemcpyHostToDevice, st));
+        src = p.q.get();
     }
-    p.q.alloc(n, st);
     if (idx.metric() == Metric::Cosine) {
-        normalize_rows(src, p.q.get(), static_cast<int>(r.nq), static_cast<int>(dim), p.err + 1, st);
-    } else {
-        QG_CUDA(cudaMemcpyAsync(p.q.get(), src, n * sizeof(float), cudaMemcpyDeviceToDevice, st));
+        DevBuf<float> unit(n, st);
+        normalize_rows(src, unit.get(), static_cast<int>(r.nq), static_cast<int>(dim), p.err + 1, st);
+        p.q = std::move(unit);
+        src = p.q.get();
     }
+    p.qp = src;
     if (r.filter && upload_filter) {
         p.filter.alloc(r.filter->words.size(), st);
         QG_CUDA(cudaMemcpyAsync(p.filter.get(), r.filter->words.data(), r.filter->words.size() * 8,
@@ -294,10 +296,10 @@ static void prepare(IndexObj& idx, const SearchRequest& r, Prepared& p, cudaStre
 // IVF stages see rotated queries when the index rotates (reference
 // src/ivf_index.cpp:196-204); a RefineIndex re-ranks with the unrotated ones.
 static const float* ivf_queries(const IVFObj& o, const Prepared& p, size_t nq, DevBuf<float>& rot, cudaStream_t st) {
-    if (!o.model.rotate) return p.q.get();
+    if (!o.model.rotate) return p.qp;
     const int dim = static_cast<int>(o.model.dim);
     rot.alloc(nq * dim, st);
-    rotate_rows(o.dev.rot.get(), p.q.get(), nq, dim, rot.get(), st);
+    rotate_rows(o.dev.rot.get(), p.qp, nq, dim, rot.get(), st);
     return rot.get();
 }
 
@@ -316,13 +318,22 @@ static void fill_empty(const SearchRequest& r, cudaStream_t st) {
     }
 }
 
-static void check_err(const int* err, cudaStream_t st) {
-    int h[3] = {0, 0, 0};
-    QG_CUDA(cudaMemcpyAsync(h, err, sizeof(h), cudaMemcpyDeviceToHost, st));
-    QG_CUDA(cudaStreamSynchronize(st));
+// The flags of a finished search: its statistics, and its errors.
+static void take_flags(const int (&h)[kFlags]) {
+    if (h[3]) count_tensor_coarse(0, h[3]);
+    unsigned long long cand;
+    std::memcpy(&cand, h + 4, sizeof(cand));
+    if (cand) count_tensor_coarse_candidates(static_cast<int64_t>(cand));
     if (h[1]) throw Error(kInvalidArgument, "cosine metric needs non-zero vectors");
     if (h[0]) throw Error(kRuntimeError, "fast-scan candidate buffer overflowed (internal error)");
     if (h[2]) throw Error(kRuntimeError, "tensor-core coarse step: a pipeline wait timed out");
+}
+
+static void check_err(const int* err, cudaStream_t st) {
+    int h[kFlags];
+    QG_CUDA(cudaMemcpyAsync(h, err, sizeof(h), cudaMemcpyDeviceToHost, st));
+    QG_CUDA(cudaStreamSynchronize(st));
+    take_flags(h);
 }
 
 // Filtered probing of an IVF index (reference src/ivf_index.cpp:501-521): at
@@ -381,7 +392,7 @@ static void refine_direct(RefineObj& o, const Prepared& p, const SearchRequest& 
     gather_rows(o.dev.ptr(), slots_dev, n, dim, rows.get(), st);
     DevBuf<uint64_t> ck(r.nq * r.k, st);
     DevBuf<uint32_t> cs(r.nq * r.k, st);
-    flat_candidates(p.q.get(), r.nq, rows.get(), n, dim, ip, r.k, nullptr, nullptr, ck.get(), cs.get(), st);
+    flat_candidates(p.qp, r.nq, rows.get(), n, dim, ip, r.k, nullptr, nullptr, ck.get(), cs.get(), st);
     k_cols_to_slots<<<static_cast<unsigned>(ceil_div(r.nq * r.k, 256)), 256, 0, st>>>(cs.get(), r.nq * r.k, slots_dev);
     QG_LAUNCH_CHECK();
     finalize_ivf(ck.get(), cs.get(), static_cast<int>(r.nq), static_cast<int>(r.k), static_cast<int>(r.k),
@@ -409,18 +420,33 @@ void search(IndexObj& idx, const SearchRequest& r, cudaStream_t st) {
     const int dim = static_cast<int>(idx.dim());
     const bool cosine = idx.metric() == Metric::Cosine;
     const bool ip = idx.metric() == Metric::InnerProduct;
-    // output staging
-    DevBuf<int64_t> o_ids;
-    DevBuf<float> o_d;
+    // output staging: ids, distances and the flags in one block, which small
+    // results come back in by one copy (each copy to pageable memory waits for
+    // the stream; three of them cost a small search about 25 us)
+    const size_t nout = r.nq * r.k, flags_at = (nout * 12 + 15) & ~size_t{15};
+    constexpr size_t kOneCopy = 128 * 1024;
+    DevBuf<uint8_t> o_all;
     int64_t* out_ids = r.out_ids;
     float* out_d = r.out_d;
+    SearchRequest rq = r;
     if (r.io == IoSpace::Host) {
-        o_ids.alloc(r.nq * r.k, st);
-        o_d.alloc(r.nq * r.k, st);
-        out_ids = o_ids.get();
-        out_d = o_d.get();
+        o_all.alloc(flags_at + kFlags * sizeof(int), st);
+        out_ids = reinterpret_cast<int64_t*>(o_all.get());
+        out_d = reinterpret_cast<float*>(o_all.get() + nout * 8);
+        if (!rq.err_dev) rq.err_dev = reinterpret_cast<int*>(o_all.get() + flags_at);
     }
     auto finish = [&](const Prepared& p) {
+        if (r.io == IoSpace::Host && !r.err_dev && o_all.count <= kOneCopy) {
+            std::vector<uint8_t> h(o_all.count);
+            QG_CUDA(cudaMemcpyAsync(h.data(), o_all.get(), o_all.count, cudaMemcpyDeviceToHost, st));
+            QG_CUDA(cudaStreamSynchronize(st));
+            std::memcpy(r.out_ids, h.data(), nout * 8);
+            std::memcpy(r.out_d, h.data() + nout * 8, nout * 4);
+            int flags[kFlags];
+            std::memcpy(flags, h.data() + flags_at, sizeof(flags));
+            take_flags(flags);
+            return;
+        }
         if (r.io == IoSpace::Host) {
             QG_CUDA(cudaMemcpyAsync(r.out_ids, out_ids, r.nq * r.k * 8, cudaMemcpyDeviceToHost, st));
             QG_CUDA(cudaMemcpyAsync(r.out_d, out_d, r.nq * r.k * 4, cudaMemcpyDeviceToHost, st));
@@ -436,7 +462,7 @@ void search(IndexObj& idx, const SearchRequest& r, cudaStream_t st) {
         }
         ensure_device(o, st);
         Prepared p;
-        prepare(idx, r, p, st);
+        prepare(idx, rq, p, st);
         const int kp = static_cast<int>(r.k);
         require(kp <= 3072, "k above 3072 is not supported by the GPU fast-scan", kUnsupported);
         DevBuf<uint64_t> ck(r.nq * kp, st);
@@ -466,14 +492,14 @@ void search(IndexObj& idx, const SearchRequest& r, cudaStream_t st) {
         }
         ensure_device(o, st);
         Prepared p;
-        prepare(idx, r, p, st);
+        prepare(idx, rq, p, st);
         DevBuf<uint64_t> ck(r.nq * r.k, st);
         DevBuf<uint32_t> cs(r.nq * r.k, st);
-        flat_candidates(p.q.get(), r.nq, o.dev.rows.get(), o.model.idmap.slots(), dim, ip, r.k, p.filter.get(),
+        flat_candidates(p.qp, r.nq, o.dev.rows.get(), o.model.idmap.slots(), dim, ip, r.k, p.filter.get(),
                         r.filter ? nullptr : o.dev.deleted.get(), ck.get(), cs.get(), st, true,
                         kept_base(o, r.nq, r.k));
         k_finalize_flat<<<static_cast<unsigned>(ceil_div(r.nq * r.k, 256)), 256, 0, st>>>(
-            p.q.get(), dim, o.dev.rows.get(), ck.get(), cs.get(), static_cast<int>(r.k), ip, o.dev.labels.get(), cosine,
+            p.qp, dim, o.dev.rows.get(), ck.get(), cs.get(), static_cast<int>(r.k), ip, o.dev.labels.get(), cosine,
             out_ids, out_d, r.nq);
         QG_LAUNCH_CHECK();
         finish(p);
@@ -493,7 +519,7 @@ void search(IndexObj& idx, const SearchRequest& r, cudaStream_t st) {
     const bool direct =
         r.filter && o.base->kind == Kind::IVF && r.filter->count <= 6 * static_cast<IVFObj&>(*o.base).model.nlist;
     Prepared p;
-    prepare(idx, r, p, st, !direct);   // (the direct scan lists the allowed slots on the host)
+    prepare(idx, rq, p, st, !direct);   // (the direct scan lists the allowed slots on the host)
     if (direct) {
         refine_direct(o, p, r, dim, ip, cosine, out_ids, out_d, st);
         finish(p);
@@ -519,11 +545,11 @@ void search(IndexObj& idx, const SearchRequest& r, cudaStream_t st) {
         ivf_candidates(b.dev.view, a, ck.get(), cs.get(), st);
     } else {
         auto& b = static_cast<FlatObj&>(*o.base);
-        flat_candidates(p.q.get(), r.nq, b.dev.rows.get(), b.model.idmap.slots(), dim, ip, kp, p.filter.get(),
+        flat_candidates(p.qp, r.nq, b.dev.rows.get(), b.model.idmap.slots(), dim, ip, kp, p.filter.get(),
                         r.filter ? nullptr : b.dev.deleted.get(), ck.get(), cs.get(), st, true,
                         kept_base(b, r.nq, kp));
     }
-    refine_candidates(p.q.get(), static_cast<int>(r.nq), dim, o.dev.ptr(), ck.get(), cs.get(), static_cast<int>(kp),
+    refine_candidates(p.qp, static_cast<int>(r.nq), dim, o.dev.ptr(), ck.get(), cs.get(), static_cast<int>(kp),
                       static_cast<int>(r.k), ip, o.dev.labels.get(), cosine, out_ids, out_d, st);
     finish(p);
 }
@@ -590,7 +616,7 @@ void finish_candidates(IndexObj& idx, const float* q_dev, size_t nq, size_t k, c
     prepare(idx, r, p, st);
     if (idx.kind == Kind::Refine) {
         auto& o = static_cast<RefineObj&>(idx);
-        refine_candidates(p.q.get(), static_cast<int>(nq), static_cast<int>(idx.dim()), o.dev.ptr(), key, slot,
+        refine_candidates(p.qp, static_cast<int>(nq), static_cast<int>(idx.dim()), o.dev.ptr(), key, slot,
                           static_cast<int>(kp), static_cast<int>(k), ip, o.dev.labels.get(), cosine, out_ids, out_d, st);
     } else {
         finalize_ivf(key, slot, static_cast<int>(nq), static_cast<int>(kp), static_cast<int>(k), b.dev.labels.get(),
@@ -645,12 +671,7 @@ bool search_graph(IndexObj& idx, const SearchRequest& r, cudaStream_t st) {
         QG_CUDA(cudaGraphLaunch(e->exec, st));
         profiler().launches.fetch_add(e->launches, std::memory_order_relaxed);
         g_graph_replays += 1;
-        int h[3] = {0, 0, 0};
-        QG_CUDA(cudaMemcpyAsync(h, e->err, sizeof(h), cudaMemcpyDeviceToHost, st));
-        QG_CUDA(cudaStreamSynchronize(st));
-        if (h[1]) throw Error(kInvalidArgument, "cosine metric needs non-zero vectors");
-        if (h[0]) throw Error(kRuntimeError, "fast-scan candidate buffer overflowed (internal error)");
-        if (h[2]) throw Error(kRuntimeError, "tensor-core coarse step: a pipeline wait timed out");
+        check_err(e->err, st);
         return true;
     }
     // first call with this key: the search itself (results, tuning, one-time setup), then its capture
@@ -665,7 +686,7 @@ bool search_graph(IndexObj& idx, const SearchRequest& r, cudaStream_t st) {
     ent->d = r.out_d;
     ent->st = st;
     ent->gen = gen;
-    QG_CUDA(cudaMalloc(reinterpret_cast<void**>(&ent->err), 3 * sizeof(int)));
+    QG_CUDA(cudaMalloc(reinterpret_cast<void**>(&ent->err), kFlags * sizeof(int)));
     SearchRequest rc = r;
     rc.capture = true;
     rc.err_dev = ent->err;
@@ -881,7 +902,7 @@ void search_mixed(IndexObj& idx, const float* q, size_t nq, const MixedQuery* qs
         DevBuf<float> od(nb * kmax_g, st);
         const bool cosine = idx.metric() == Metric::Cosine, ip = idx.metric() == Metric::InnerProduct;
         if (ref)
-            refine_candidates(p.q.get(), static_cast<int>(nb), static_cast<int>(dim), ref->dev.ptr(), ck.get(), cs.get(),
+            refine_candidates(p.qp, static_cast<int>(nb), static_cast<int>(dim), ref->dev.ptr(), ck.get(), cs.get(),
                               kpmax, static_cast<int>(kmax_g), ip, ref->dev.labels.get(), cosine, oid.get(), od.get(), st,
                               a.pq.kp, a.pq.k);
         else

@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(NW * 32, kMinB) k_scan(ScanArgs a) {
     }
     for (;;) {
         __syncthreads();   // the previous unit is done with every shared array
-        if (tid == 0) s_unit = atomicAdd(a.work, 1);
+        if (tid == 0) s_unit = atomicAdd(a.work, 1) + 1;   // (from -1 at launch)
         __syncthreads();
         const int unit = s_unit;
         if (unit >= a.nunits) break;
@@ -898,9 +898,12 @@ static void run_scan(const ScanShape& sh, ScanArgs a, const IvfView& v, int qtab
     const bool shared_lut = v.mode == kModeIP || v.mode == kModeCosIP;
     a.lc = sh.lc;
     const size_t smem = scan_layout(a.kp, v.m_pad, qtab_len, a.pch, shared_lut, sh.nw, sh.lc, sh.staged).bytes;
-    QG_CUDA(cudaMemsetAsync(a.work, 0, sizeof(int), st));
-    if (a.qthr)   // (every timed run of the autotuner starts from no bound too)
-        QG_CUDA(cudaMemsetAsync(a.qthr, 0xFF, static_cast<size_t>(a.nunits / a.nchunks) * sizeof(unsigned long long), st));
+    // the work counter and, after it, the queries' bounds, all ones by one
+    // memset (every timed run of the autotuner starts from no bound too)
+    QG_CUDA(cudaMemsetAsync(a.work, 0xFF,
+                            a.qthr ? (1 + static_cast<size_t>(a.nunits / a.nchunks)) * sizeof(unsigned long long)
+                                   : sizeof(int),
+                            st));
     if (sh.staged) {
         switch (sh.nw) {
             case 8: launch_scan<8, true>(a, smem, st); break;
@@ -980,14 +983,11 @@ static void scan_query_major(const IvfView& v, const IvfSearchArgs& s, int nq, i
     const size_t nout = static_cast<size_t>(nq) * nchunks * kp;
     DevBuf<uint64_t> ckey;
     DevBuf<uint32_t> cslot;
-    DevBuf<unsigned long long> qthr;
+    DevBuf<unsigned long long> work(1 + (direct ? 0 : static_cast<size_t>(nq)), st);   // the counter, then the bounds
     if (!direct) {
         ckey.alloc(nout, st);
         cslot.alloc(nout, st);
-        qthr.alloc(nq, st);
     }
-    DevBuf<int> work(1, st);
-    QG_CUDA(cudaMemsetAsync(work.get(), 0, sizeof(int), st));
     ScanArgs a{};
     a.v = v;
     a.q = q;
@@ -1005,8 +1005,8 @@ static void scan_query_major(const IvfView& v, const IvfSearchArgs& s, int nq, i
     a.nchunks = nchunks;
     a.kp = kp;
     a.nunits = nq * nchunks;
-    a.work = work.get();
-    a.qthr = direct ? nullptr : qthr.get();
+    a.work = reinterpret_cast<int*>(work.get());
+    a.qthr = direct ? nullptr : work.get() + 1;
     a.out_key = direct ? out_key : ckey.get();
     a.out_slot = direct ? out_slot : cslot.get();
     a.err = s.d_err;
@@ -1054,34 +1054,14 @@ void nearest_lists(const IvfView& v, const IvfSearchArgs& s, int nq, int P, uint
         pair_scores(qs, n, v.centroids, v.nlist, v.dim, v.ip_metric, scores.get(), v.nlist, st);
         select_rows(scores.get(), v.nlist, n, v.nlist, P, pr, pd, st, nullptr, nullptr, 0, true);
     };
-    // batches of at most one query per SM (and captured ones) read nothing
-    // back mid-search: their recheck holds every list, so none is redone
-    const bool no_readback = s.d_err && (s.capture || nq <= s.sm_count);
-    if (!use_tensor_coarse(nq, v.nlist, v.dim) ||
-        !coarse_mm_supported(v.nlist, v.dim, P, v.cent_f16 != nullptr, no_readback)) {
+    if (!use_tensor_coarse(nq, v.nlist, v.dim) || !coarse_mm_supported(v.nlist, v.dim, P, v.cent_f16 != nullptr)) {
         exact_coarse(s.q, nq, probe, pdist);
         return;
     }
-    std::vector<int> redo;
-    coarse_probes_mm(v, s.q, nq, P, probe, pdist, redo, st, no_readback ? s.d_err + 2 : nullptr);
-    if (!s.capture) count_tensor_coarse(nq, static_cast<int64_t>(redo.size()));
-    if (redo.empty()) return;
-    // queries with too many near-ties: the exact path, results copied into place
-    const size_t m = redo.size();
-    std::vector<uint32_t> hidx(redo.begin(), redo.end());
-    DevBuf<uint32_t> idx(m, st);
-    QG_CUDA(cudaMemcpyAsync(idx.get(), hidx.data(), m * 4, cudaMemcpyHostToDevice, st));
-    DevBuf<float> qs(m * v.dim, st);
-    gather_rows(s.q, idx.get(), m, v.dim, qs.get(), st);
-    DevBuf<uint32_t> pr(m * P, st);
-    DevBuf<float> pd(m * P, st);
-    exact_coarse(qs.get(), static_cast<int>(m), pr.get(), pd.get());
-    for (size_t j = 0; j < m; ++j) {
-        QG_CUDA(cudaMemcpyAsync(probe + static_cast<size_t>(redo[j]) * P, pr.get() + j * P, P * 4,
-                                cudaMemcpyDeviceToDevice, st));
-        QG_CUDA(cudaMemcpyAsync(pdist + static_cast<size_t>(redo[j]) * P, pd.get() + j * P, P * 4,
-                                cudaMemcpyDeviceToDevice, st));
-    }
+    require(s.d_err != nullptr, "the coarse step needs its flags");
+    // batches of at most one query per SM: the recheck holds every list
+    coarse_probes_mm(v, s.q, nq, P, probe, pdist, s.d_err, nq <= s.sm_count, !s.capture && nq > s.sm_count, st);
+    if (!s.capture) count_tensor_coarse(nq, 0);   // (those redone are counted from the flags)
 }
 
 void ivf_candidates(const IvfView& v, const IvfSearchArgs& s, uint64_t* out_key, uint32_t* out_slot, cudaStream_t st) {

@@ -55,6 +55,8 @@ struct PerQuery {
     const int* wanted = nullptr;       // then on until this many allowed vectors were seen
 };
 
+inline constexpr int kFlags = 8;
+
 struct ScanArgs {
     IvfView v;
     const float* q;          // nq * dim prepared queries
@@ -70,7 +72,7 @@ struct ScanArgs {
     int P, pch, nchunks, kp;
     int nunits;              // nq * nchunks work units (query, chunk of pch probes)
     int lc;                  // lists per LUT group
-    int* work;               // next unit to take (zero at launch)
+    int* work;               // the last unit taken (-1 at launch)
     // per query, shared by its chunks (nchunks > 1; else null): a bound on the
     // query's k'-th key, all ones at launch; every chunk lowers it and prunes by it
     unsigned long long* qthr;
@@ -92,7 +94,10 @@ struct IvfSearchArgs {
     PerQuery pq;                // mixed batches; nprobe above is then the largest nprobe
     bool any_filter = false;    // some query of a mixed batch has a filter
     int sm_count = 0;
-    int* d_err = nullptr;       // [0] scan overflow, [2] tensor-core pipeline timeout
+    // kFlags ints, read with the results: [0] scan overflow, [1] a zero cosine
+    // row, [2] tensor-core pipeline timeout, [3] coarse queries taken by the
+    // second pass, [4..5] coarse lists rescored exactly (a 64-bit count)
+    int* d_err = nullptr;
     bool capture = false;       // being captured into a CUDA graph: no host reads, waits or tuning
 };
 
@@ -132,10 +137,9 @@ void nearest_lists(const IvfView& v, const IvfSearchArgs& s, int nq, int P, uint
 void ivf_candidates(const IvfView& v, const IvfSearchArgs& s, uint64_t* out_key, uint32_t* out_slot, cudaStream_t st);
 // Coarse assignment through the tensor cores (qg_coarse.cu): the P nearest lists
 // of each query by exact score, ties by list, from F16 estimates with an
-// error bound and an exact recheck; queries with too many near-ties are
-// listed in redo_q for the exact path. use_tensor_coarse: whether the batch
+// error bound and an exact recheck. use_tensor_coarse: whether the batch
 // goes this way (the process-wide tensor-filter mode and the work's size).
-bool coarse_mm_supported(int nlist, int dim, int P, bool cent_prepared, bool no_readback = false);
+bool coarse_mm_supported(int nlist, int dim, int P, bool cent_prepared);
 bool use_tensor_coarse(size_t nq, int nlist, int dim);
 // Queries whose coarse step went through the tensor cores, and those of them redone exactly.
 void count_tensor_coarse(int64_t queries, int64_t redone);
@@ -143,12 +147,12 @@ void tensor_coarse_counts(int64_t* queries, int64_t* redone);
 // Lists rescored exactly by the tensor-core coarse step so far (its candidates).
 void count_tensor_coarse_candidates(int64_t n);
 int64_t tensor_coarse_candidates();
-// With err_dev (under graph capture, and for batches of at most one query per
-// SM) nothing is read back and redo_q stays empty: every list fits the
-// recheck, queries with extreme norms rescore every list, and a pipeline
-// timeout is flagged in *err_dev for the caller to read with the results.
-void coarse_probes_mm(const IvfView& v, const float* q, int nq, int P, uint32_t* probe, float* pdist,
-                      std::vector<int>& redo_q, cudaStream_t st, int* err_dev = nullptr);
+// Nothing is read back: flags (kFlags ints) take a pipeline timeout and the
+// statistics for the caller to read with the results. hold_all: the recheck
+// holds every list of every query; otherwise queries of extreme norm or with too
+// many near-ties are taken by a second pass that does.
+void coarse_probes_mm(const IvfView& v, const float* q, int nq, int P, uint32_t* probe, float* pdist, int* flags,
+                      bool hold_all, bool may_tune, cudaStream_t st);
 
 // The scan's shape autotuner: on (1, the default) it times the candidate
 // shapes on the first large search of each problem key; off (0) every search

@@ -213,3 +213,35 @@ def test_flat_concurrent_first_searches():
     for g in got:
         np.testing.assert_array_equal(g[0], want[0])
         assert g[1].tobytes() == want[1].tobytes()
+
+
+@pytest.mark.parametrize("metric", [0, 1, 2])
+@pytest.mark.parametrize("nq,k", [(1, 1), (149, 10), (400, 10), (1200, 9), (1200, 100)])
+def test_one_copy_results(metric, nq, k):
+    """Small results come back in one copy, larger ones apart; from device
+    buffers (whatever their alignment) the same bits, coarse step either way."""
+    import torch
+    d = 40
+    x = rows_of("mixture", 12, 20_000, d)
+    ivf = qb.IVFIndex(d, 300, 20, metric=qb.Metric(metric))
+    ivf.enable_pq(20, fast_scan=True)
+    ivf.train(x, max_iters=2, seed=5, clustering=qb.Clustering.Lloyd)
+    idx = qb.RefineIndex(ivf, 4)
+    idx.add(x)
+    q = rows_of("mixture", 13, nq, d)
+    q[0] *= np.float32(1e-12)   # a norm its coarse bounds do not hold for
+    qb.set_tensor_filter(0)
+    want = idx.batch_query(q, k)
+    for mode in (1, 2):
+        qb.set_tensor_filter(mode)
+        got = idx.batch_query(q, k)
+        np.testing.assert_array_equal(got[0], want[0])
+        assert got[1].tobytes() == want[1].tobytes()
+        pad = torch.zeros(nq * d + 1, device="cuda")
+        pad[1:] = torch.from_numpy(q).cuda().ravel()   # rows 4 bytes off
+        ids = torch.empty(nq, k, dtype=torch.int64, device="cuda")
+        dist = torch.empty(nq, k, device="cuda")
+        idx.search_device(pad.data_ptr() + 4, nq, k, ids.data_ptr(), dist.data_ptr(),
+                          torch.cuda.current_stream().cuda_stream)
+        np.testing.assert_array_equal(ids.cpu().numpy(), want[0])
+        assert dist.cpu().numpy().tobytes() == want[1].tobytes()
