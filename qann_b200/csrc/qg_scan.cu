@@ -24,7 +24,8 @@
 // they can enter, as the reference's push() does. The integer pre-test
 // `sum <= S*` is exact: S* is the largest sum whose distance is <= the
 // threshold distance (sum_limit). At the end of a unit the warps' survivors
-// are gathered, cut to k', sorted, and their slots looked up from the push
+// are gathered, put in order by the block (bins of their range, then ranks
+// within a bin), and the first k' slots looked up from the push
 // index.
 #include "qg_device.cuh"
 #include "qg_search.h"
@@ -253,7 +254,7 @@ __device__ __forceinline__ int upper_index(const uint32_t* pre, int n, uint32_t 
 }
 
 // Shared memory of one block. The LUT ring shares its space with the
-// end-of-unit gather of candidates and their final sort.
+// end-of-unit gather of candidates.
 struct ScanLayout {
     int nw, lc, wcap, lut_stride;   // lut_stride: uint4s per LUT (m_pad + 2: 32 bytes keep
                                     // consecutive LUTs of a warp's octets on distinct banks)
@@ -271,8 +272,7 @@ __host__ __device__ inline ScanLayout scan_layout(int kp, int m_pad, int qtab_le
     L.lut_stride = m_pad + 2;
     const size_t lut = shared_lut ? static_cast<size_t>(m_pad) * 16 : static_cast<size_t>(2) * lc * L.lut_stride * 16;
     const size_t gather = static_cast<size_t>(nw) * kp * 8;
-    const size_t sortb = static_cast<size_t>(next_pow2(kp < 2 ? 2 : kp)) * 8;
-    size_t b = align16(lut > gather ? (lut > sortb ? lut : sortb) : (gather > sortb ? gather : sortb));
+    size_t b = align16(lut > gather ? lut : gather);
     L.off_wbuf = b;
     b += static_cast<size_t>(nw) * L.wcap * 8;
     L.off_hist = b;
@@ -370,7 +370,9 @@ __global__ void __launch_bounds__(NW * 32, kMinB) k_scan(ScanArgs a) {
             const uint32_t l = a.probe[qp + p0 + p];
             p_list[p] = l;
             p_size[p] = v.list_size[l];
-            p_sboff[p] = v.sb_off[l];
+            const uint32_t off = v.sb_off[l];
+            p_sboff[p] = off;
+            p_sbpre[p] = v.sb_off[l + 1] - off;   // superblocks held on this device (none for another shard's list)
         }
         if (v.mode == kModeL2)
             for (int t = tid; t < v.m * 16; t += NT)
@@ -394,8 +396,7 @@ __global__ void __launch_bounds__(NW * 32, kMinB) k_scan(ScanArgs a) {
             for (int base = 0; base < np; base += 32) {
                 const int p = base + lane;
                 const uint32_t sz = p < np ? p_size[p] : 0;
-                // superblocks held on this device (none for another shard's list)
-                const uint32_t nsb = p < np ? v.sb_off[p_list[p] + 1] - p_sboff[p] : 0;
+                const uint32_t nsb = p < np ? p_sbpre[p] : 0;
                 uint32_t ip = sz, is = nsb;
                 for (int o = 1; o < 32; o <<= 1) {
                     const uint32_t t1 = __shfl_up_sync(kFull, ip, o), t2 = __shfl_up_sync(kFull, is, o);
@@ -466,26 +467,43 @@ __global__ void __launch_bounds__(NW * 32, kMinB) k_scan(ScanArgs a) {
             }
         };
 
-        // (all threads, after a block barrier; the per-warp histograms serve as one)
-        auto seed_threshold = [&]() {
-            int total = 0;
-            for (int w = 0; w < NW; ++w) total += s_wcount[w];
-            if (total <= kp) return;   // (block-uniform)
-            constexpr int kBins = NW * 256 < 1024 ? NW * 256 : 1024;
-            int* bh = reinterpret_cast<int*>(sm + lay.off_hist);
-            const uint64_t* wb0 = reinterpret_cast<const uint64_t*>(sm + lay.off_wbuf);
-            uint32_t lo = ~0u, hi = 0;
-            for (int w = 0; w < NW; ++w)
-                for (int i = tid; i < s_wcount[w]; i += NT) {
-                    const uint32_t k = static_cast<uint32_t>(wb0[static_cast<size_t>(w) * wcap + i] >> 32);
-                    lo = min(lo, k);
-                    hi = max(hi, k);
-                }
-            for (int t = tid; t < kBins; t += NT) bh[t] = 0;
-            for (int o = 16; o > 0; o >>= 1) {
-                lo = min(lo, __shfl_xor_sync(kFull, lo, o));
-                hi = max(hi, __shfl_xor_sync(kFull, hi, o));
+        // The per-warp histograms as one of kBins bins, and its exclusive prefix
+        // sums in place, kPer bins a thread (all threads; the bins are complete and
+        // behind a barrier on entry; one more inside). before: keys in the bins
+        // ahead of this thread's.
+        constexpr int kBins = NW * 256 < 1024 ? NW * 256 : 1024;
+        constexpr int kPer = kBins / NT;
+        int* bh = reinterpret_cast<int*>(sm + lay.off_hist);
+        auto bin_prefix = [&](int (&own)[kPer], int& before) {
+            int sum = 0;
+#pragma unroll
+            for (int b = 0; b < kPer; ++b) {
+                own[b] = bh[kPer * tid + b];
+                sum += own[b];
             }
+            int incl = sum;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(kFull, incl, o);
+                if (lane >= o) incl += t;
+            }
+            if (lane == 31) s_red[warp] = static_cast<uint32_t>(incl);
+            __syncthreads();
+            before = incl - sum;
+            for (int w = 0; w < warp; ++w) before += static_cast<int>(s_red[w]);
+        };
+        // the range of the high halves of n keys per warp at mine, over the block
+        // (all threads; zeroes the bins; one barrier)
+        auto key_range = [&](const uint64_t* mine, int n, uint32_t& lo, uint32_t& hi) {
+            lo = ~0u;
+            hi = 0;
+            for (int i = lane; i < n; i += 32) {
+                const uint32_t k = static_cast<uint32_t>(mine[i] >> 32);
+                lo = min(lo, k);
+                hi = max(hi, k);
+            }
+            lo = __reduce_min_sync(kFull, lo);
+            hi = __reduce_max_sync(kFull, hi);
+            for (int t = tid; t < kBins; t += NT) bh[t] = 0;
             if (lane == 0) {
                 s_red[warp] = lo;
                 s_red2[warp] = hi;
@@ -495,46 +513,37 @@ __global__ void __launch_bounds__(NW * 32, kMinB) k_scan(ScanArgs a) {
                 lo = min(lo, s_red[w]);
                 hi = max(hi, s_red2[w]);
             }
+        };
+
+        // (all threads, after a block barrier)
+        auto seed_threshold = [&](int mine) {
+            int total = 0;
+            for (int w = 0; w < NW; ++w) total += s_wcount[w];
+            if (total <= kp) return;   // (block-uniform)
+            uint32_t lo, hi;
+            key_range(wbuf, mine, lo, hi);
+            auto lower = [&](uint32_t T) {
+                atomicMin(&s_thr, (static_cast<unsigned long long>(T) << 32) | 0xFFFFFFFFull);
+                if (a.qthr) atomicMin(a.qthr + qi, (static_cast<unsigned long long>(T) << 32) | 0xFFFFFFFFull);
+            };
             if (lo == hi) {   // (block-uniform)
-                if (tid == 0) {
-                    atomicMin(&s_thr, (static_cast<unsigned long long>(lo) << 32) | 0xFFFFFFFFull);
-                    if (a.qthr) atomicMin(a.qthr + qi, (static_cast<unsigned long long>(lo) << 32) | 0xFFFFFFFFull);
-                }
+                if (tid == 0) lower(lo);
+                __syncthreads();   // (s_red is read before the next use)
                 return;
             }
             const KeyBins kb(lo, static_cast<uint64_t>(hi - lo) + 1, kBins);
-            for (int w = 0; w < NW; ++w)
-                for (int i = tid; i < s_wcount[w]; i += NT) {
-                    const uint32_t k = static_cast<uint32_t>(wb0[static_cast<size_t>(w) * wcap + i] >> 32);
-                    atomicAdd(&bh[kb.bin(k)], 1);
-                }
+            for (int i = lane; i < mine; i += 32) atomicAdd(&bh[kb.bin(static_cast<uint32_t>(wbuf[i] >> 32))], 1);
             __syncthreads();
-            if (warp == 0) {   // lane l owns bins kPer l .. kPer l + kPer - 1
-                constexpr int kPer = kBins / 32;
-                int own = 0;
-                for (int b = 0; b < kPer; ++b) own += bh[kPer * lane + b];
-                int incl = own;
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int t = __shfl_up_sync(kFull, incl, o);
-                    if (lane >= o) incl += t;
-                }
-                const int excl = incl - own;
-                if (excl < kp && kp <= incl) {
-                    int acc = excl, bin = kPer * lane + kPer - 1;
-                    for (int b = 0; b < kPer; ++b) {
-                        acc += bh[kPer * lane + b];
-                        if (acc >= kp) {
-                            bin = kPer * lane + b;
-                            break;
-                        }
-                    }
-                    // every key counted in bins <= bin is <= kb.last(bin)
-                    const uint32_t T = static_cast<uint32_t>(min(kb.last(bin), static_cast<uint64_t>(hi)));
-                    atomicMin(&s_thr, (static_cast<unsigned long long>(T) << 32) | 0xFFFFFFFFull);
-                    if (a.qthr) atomicMin(a.qthr + qi, (static_cast<unsigned long long>(T) << 32) | 0xFFFFFFFFull);
-                }
+            int own[kPer], acc;
+            bin_prefix(own, acc);
+#pragma unroll
+            for (int b = 0; b < kPer; ++b) {
+                // every key counted in bins <= the one holding the k'-th is <= its last
+                if (acc < kp && kp <= acc + own[b])
+                    lower(static_cast<uint32_t>(min(kb.last(kPer * tid + b), static_cast<uint64_t>(hi))));
+                acc += own[b];
             }
-            __syncthreads();   // warp 0 is done with the histograms before any trim reuses them
+            __syncthreads();   // the bins and s_red are read before any trim reuses them
         };
 
         const int ngroups = np <= first ? 1 : 1 + (np - first + LC - 1) / LC;
@@ -551,7 +560,7 @@ __global__ void __launch_bounds__(NW * 32, kMinB) k_scan(ScanArgs a) {
             // any single warp's k'-th, so about half as many later takes reach
             // the candidate path. (At later groups it cost more barriers than it
             // saved.)
-            if (NW >= 4 && (g == 1 || g == 2)) seed_threshold();
+            if (NW >= 4 && (g == 1 || g == 2)) seed_threshold(min(wcount, wcap));
             const int h = g & 1, gp0 = group_start(g), nc = group_start(g + 1) - gp0;
             // The group's superblocks without those of skipped lists, numbered
             // 0..total-1 list after list: list lane (and lane + 32 when LC = 64)
@@ -755,7 +764,7 @@ __global__ void __launch_bounds__(NW * 32, kMinB) k_scan(ScanArgs a) {
             if (g + 1 < ngroups) build_group(g + 1);
         }
 
-        // ---- the unit's k' best: each warp's own, gathered, cut to k', sorted ----
+        // ---- the unit's k' best: each warp's own, gathered, in order ----
         __syncwarp();
         // keys above the block threshold first (as at a trim), so that fewer
         // reach warp 0's cut below
@@ -764,44 +773,61 @@ __global__ void __launch_bounds__(NW * 32, kMinB) k_scan(ScanArgs a) {
             warp_select_keep(wbuf, min(wcount, wcap), kp, hist);
             wcount = kp;
         }
-        if (lane == 0) s_wcount[warp] = min(wcount, wcap);
+        wcount = min(wcount, wcap);
+        if (lane == 0) s_wcount[warp] = wcount;
         __syncthreads();   // every warp is done with the LUT ring: gather over it
+        // Gathered and put in order by the whole block: the keys are counted into
+        // bins of their range, moved bin by bin into the warps' buffers, and each
+        // one's place is its bin's start plus the smaller keys in its bin. Most bins
+        // hold a few keys. (Warp 0 alone cut and sorted them before: 20,700 cycles a
+        // unit of 102,400 at k' = 100 and 1,000 queries, 32,700 of 378,700 at k' =
+        // 200 and 10,000, the other warps waiting.)
         int off = 0, total = 0;
         for (int w = 0; w < NW; ++w) {
             if (w < warp) off += s_wcount[w];
             total += s_wcount[w];
         }
-        for (int i = lane; i < s_wcount[warp]; i += 32) gath[off + i] = wbuf[i];
-        __syncthreads();
+        for (int i = lane; i < wcount; i += 32) gath[off + i] = wbuf[i];
+        uint32_t lo, hi;
+        key_range(wbuf, wcount, lo, hi);   // (its barrier ends the gather too)
         const int kept = min(total, kp);
-        if (kept <= 256) {   // warp 0 alone cuts to k' and sorts in registers; one barrier
-            if (warp == 0) {
-                if (total > kp) warp_select_keep(gath, total, kp, hist);
-                warp_sort_keys(gath, kept);
+        uint64_t* bucket = reinterpret_cast<uint64_t*>(sm + lay.off_wbuf);
+        if (total > 0) {   // (block-uniform)
+            const KeyBins kb(lo, static_cast<uint64_t>(hi - lo) + 1, kBins);
+            for (int i = lane; i < wcount; i += 32) atomicAdd(&bh[kb.bin(static_cast<uint32_t>(wbuf[i] >> 32))], 1);
+            __syncthreads();
+            int own[kPer], acc;
+            bin_prefix(own, acc);
+#pragma unroll
+            for (int b = 0; b < kPer; ++b) {
+                bh[kPer * tid + b] = acc;
+                acc += own[b];
             }
             __syncthreads();
-        } else {
-            if (total > kp) {
-                if (warp == 0) warp_select_keep(gath, total, kp, hist);
-                __syncthreads();
-            }
-            const int ns = next_pow2(kept);
-            for (int i = kept + tid; i < ns; i += NT) gath[i] = ~0ull;
-            bitonic_sort_keys(gath, ns);
-        }
-        for (int i = tid; i < kp; i += NT) {
-            if (i < kept) {
+            for (int i = tid; i < total; i += NT) {
                 const uint64_t key = gath[i];
+                bucket[atomicAdd(&bh[kb.bin(static_cast<uint32_t>(key >> 32))], 1)] = key;
+            }
+            __syncthreads();   // bin b now ends at bh[b], where bin b + 1 starts
+            for (int i = tid; i < total; i += NT) {
+                const uint64_t key = bucket[i];
+                const int b = kb.bin(static_cast<uint32_t>(key >> 32));
+                const int start = b > 0 ? bh[b - 1] : 0, end = bh[b];
+                if (start >= kp) continue;
+                int place = start;
+                for (int e = start; e < end; ++e) place += bucket[e] < key;
+                if (place >= kp) continue;
                 const uint32_t push = static_cast<uint32_t>(key);
                 const int pp = upper_index(p_push, np, push);
                 const uint32_t pos = push - p_push[pp];
                 const size_t sbg = static_cast<size_t>(p_sboff[pp]) + pos / kSuperBlock;
-                a.out_key[ob + i] = key;
-                a.out_slot[ob + i] = v.ids[sbg * kSuperBlock + pos % kSuperBlock];
-            } else {
-                a.out_key[ob + i] = ~0ull;
-                a.out_slot[ob + i] = 0xFFFFFFFFu;
+                a.out_key[ob + place] = key;
+                a.out_slot[ob + place] = v.ids[sbg * kSuperBlock + pos % kSuperBlock];
             }
+        }
+        for (int i = kept + tid; i < kp; i += NT) {
+            a.out_key[ob + i] = ~0ull;
+            a.out_slot[ob + i] = 0xFFFFFFFFu;
         }
         if (tid == 0 && s_overflow) atomicExch(a.err, 1);
     }
