@@ -229,6 +229,86 @@ __device__ __noinline__ static int warp_keep_upto(uint64_t* buf, int n, uint64_t
     return out;
 }
 
+// nbins nearly equal intervals over the keys lo .. lo + span - 1, found by a
+// multiply-high instead of a 64-bit division per key. With span > nbins,
+// mul = floor(2^32 nbins / span) < 2^32 and bin(x) = floor((x - lo) mul / 2^32)
+// <= floor(nbins (span - 1) / span) < nbins; otherwise every key has its own
+// interval (mul = 0). last(b), the largest key whose interval is <= b, is
+// lo + ceil((b + 1) 2^32 / mul) - 1 (x mul < (b + 1) 2^32), so a threshold
+// taken there is at or above every key counted in intervals 0 .. b.
+struct KeyBins {
+    uint32_t lo, mul;
+    __device__ __forceinline__ KeyBins(uint32_t lo_, uint64_t span, int nbins)
+        : lo(lo_),
+          mul(span > static_cast<uint64_t>(nbins)
+                  ? static_cast<uint32_t>((static_cast<uint64_t>(nbins) << 32) / span)
+                  : 0u) {}
+    __device__ __forceinline__ int bin(uint32_t key) const {
+        const uint32_t x = key - lo;
+        return static_cast<int>(mul ? __umulhi(x, mul) : x);
+    }
+    __device__ __forceinline__ uint64_t last(int b) const {
+        return static_cast<uint64_t>(lo) +
+               (mul ? ((static_cast<uint64_t>(b + 1) << 32) + mul - 1) / mul - 1 : static_cast<uint64_t>(b));
+    }
+};
+
+// One warp cuts the n distinct keys buf[0, n), in place and in order, to about
+// the `keep` smallest: all of them and at most `room` keys; returns how many
+// and, in lim, a key at or above the largest of them below which the others do
+// not lie. One pass over 256 intervals of the high halves' range, and the
+// interval that holds the keep-th key stays whole; where that is more than
+// `room`, the radix select (up to 8 passes) cuts to `keep` exactly. hist: 256
+// ints of warp-private scratch, 16-byte aligned. n > keep >= 1, room >= keep.
+__device__ __noinline__ static int warp_trim(uint64_t* buf, int n, int keep, int room, int* hist, uint64_t& lim) {
+    const int lane = threadIdx.x & 31;
+    constexpr unsigned kFull = 0xffffffffu;
+    uint32_t lo = ~0u, hi = 0;
+    for (int i = lane; i < n; i += 32) {
+        const uint32_t k = static_cast<uint32_t>(buf[i] >> 32);
+        lo = min(lo, k);
+        hi = max(hi, k);
+    }
+    int4* h4 = reinterpret_cast<int4*>(hist);
+    h4[lane] = make_int4(0, 0, 0, 0);
+    h4[32 + lane] = make_int4(0, 0, 0, 0);
+    lo = __reduce_min_sync(kFull, lo);
+    hi = __reduce_max_sync(kFull, hi);
+    __syncwarp();
+    const KeyBins kb(lo, static_cast<uint64_t>(hi - lo) + 1, 256);
+    for (int i = lane; i < n; i += 32) atomicAdd(&hist[kb.bin(static_cast<uint32_t>(buf[i] >> 32))], 1);
+    __syncwarp();
+    const int4 c0 = h4[2 * lane], c1 = h4[2 * lane + 1];   // bins 8 lane .. 8 lane + 7
+    const int c[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+    int own = 0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) own += c[j];
+    int incl = own;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(kFull, incl, o);
+        if (lane >= o) incl += t;
+    }
+    int acc = incl - own, bin = -1, kept = 0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        if (acc < keep && keep <= acc + c[j]) {
+            bin = 8 * lane + j;
+            kept = acc + c[j];
+        }
+        acc += c[j];
+    }
+    const int owner = __ffs(__ballot_sync(kFull, bin >= 0)) - 1;
+    bin = __shfl_sync(kFull, bin, owner);
+    kept = __shfl_sync(kFull, kept, owner);
+    if (kept > room) {
+        lim = warp_select_keep(buf, n, keep, hist);
+        return keep;
+    }
+    const uint32_t T = static_cast<uint32_t>(min(kb.last(bin), static_cast<uint64_t>(hi)));
+    lim = (static_cast<uint64_t>(T) << 32) | 0xFFFFFFFFull;
+    return warp_keep_upto(buf, n, lim);
+}
+
 // ---------------------------------------------------------------------------
 // Block reductions
 // ---------------------------------------------------------------------------
@@ -515,30 +595,6 @@ __device__ __forceinline__ int sum_limit_fast(uint32_t thr_key, float scale, flo
     }
     return sum_limit(thr_key, scale, offset);
 }
-
-// nbins nearly equal intervals over the keys lo .. lo + span - 1, found by a
-// multiply-high instead of a 64-bit division per key. With span > nbins,
-// mul = floor(2^32 nbins / span) < 2^32 and bin(x) = floor((x - lo) mul / 2^32)
-// <= floor(nbins (span - 1) / span) < nbins; otherwise every key has its own
-// interval (mul = 0). last(b), the largest key whose interval is <= b, is
-// lo + ceil((b + 1) 2^32 / mul) - 1 (x mul < (b + 1) 2^32), so a threshold
-// taken there is at or above every key counted in intervals 0 .. b.
-struct KeyBins {
-    uint32_t lo, mul;
-    __device__ __forceinline__ KeyBins(uint32_t lo_, uint64_t span, int nbins)
-        : lo(lo_),
-          mul(span > static_cast<uint64_t>(nbins)
-                  ? static_cast<uint32_t>((static_cast<uint64_t>(nbins) << 32) / span)
-                  : 0u) {}
-    __device__ __forceinline__ int bin(uint32_t key) const {
-        const uint32_t x = key - lo;
-        return static_cast<int>(mul ? __umulhi(x, mul) : x);
-    }
-    __device__ __forceinline__ uint64_t last(int b) const {
-        return static_cast<uint64_t>(lo) +
-               (mul ? ((static_cast<uint64_t>(b + 1) << 32) + mul - 1) / mul - 1 : static_cast<uint64_t>(b));
-    }
-};
 
 // A threshold T at or above the k-th smallest (1-based) of the n uint32 keys
 // in shared memory, by one block. 0xFFFFFFFF marks an unbounded key, above

@@ -18,9 +18,9 @@
 // sequence of probed lists: exactly the set the reference's TopK keeps
 // (distance first, first pushed among ties). Each warp appends the candidates
 // that beat the block's threshold to its own buffer; when the buffer is
-// nearly full it keeps its k' best (radix select) and lowers the block
-// threshold to its k'-th key (an upper bound of the block's k'-th, so the
-// pruning is exact). Deleted (or filtered-out) vectors are skipped before
+// nearly full it keeps its k' best, with a few more (warp_trim), and lowers the
+// block threshold to the bound they lie under (an upper bound of the block's
+// k'-th key, so the pruning is exact). Deleted (or filtered-out) vectors are skipped before
 // they can enter, as the reference's push() does. The integer pre-test
 // `sum <= S*` is exact: S* is the largest sum whose distance is <= the
 // threshold distance (sum_limit). At the end of a unit the warps' survivors
@@ -47,7 +47,10 @@ constexpr int kSbPerWarp = 4;    // superblocks a warp takes at a time, one per 
 // Row stride (floats) of the query's table C in shared memory: 80 bytes puts
 // the 16-byte reads of 8 lanes (one row each) on distinct banks.
 constexpr int kQtabStride = 20;
-constexpr int kFirstGroup = 2;   // lists in the first LUT group (at most LC)
+constexpr int kFirstGroup = 3;   // lists in the first LUT group (at most LC)
+// Keys above k' that a trimmed buffer may hold: what one interval of the trim's
+// range takes in at most, as a rule.
+constexpr int kTrimSlack = 32;
 }
 
 // LUT of one list by one warp. Same arithmetic as quantize_lut. Lane l forms
@@ -268,7 +271,7 @@ __host__ __device__ inline ScanLayout scan_layout(int kp, int m_pad, int qtab_le
     ScanLayout L;
     L.nw = nw;
     L.lc = lc;
-    L.wcap = (kp + kSbPerWarp * kSuperBlock + 31) & ~31;
+    L.wcap = (kp + kTrimSlack + kSbPerWarp * kSuperBlock + 31) & ~31;
     L.lut_stride = m_pad + 2;
     const size_t lut = shared_lut ? static_cast<size_t>(m_pad) * 16 : static_cast<size_t>(2) * lc * L.lut_stride * 16;
     const size_t gather = static_cast<size_t>(nw) * kp * 8;
@@ -420,10 +423,11 @@ __global__ void __launch_bounds__(NW * 32, kMinB) k_scan(ScanArgs a) {
         // build more of them. A list none of whose vectors can beat the block
         // threshold (even a zero sum's distance is above it) gets scale -1 (real
         // scales are >= 0) and no LUT; the group's scan skips its superblocks.
-        // Groups of LC lists, the first one of 2 only: its keys meet no threshold
+        // Groups of LC lists, the first one of 3 only: its keys meet no threshold
         // yet, so the block's bound on the k'-th key after it (below) comes
-        // sooner. (2 to 4 lists measured best for 8 x 32, 8 x 16 and 4 x 8 shapes
-        // alike, 2 by a little.)
+        // sooner. (2, 3, 4, 6 and 8 lists: 6.21, 5.98, 5.97, 6.10 and 6.24 ms for
+        // 10,000 angular queries, 172, 165, 166, 179 and 184 us for 1,000 queries of
+        // 16 probes.)
         const int first = min(LC, kFirstGroup);
         auto group_start = [&](int g) { return g == 0 ? 0 : min(np, first + (g - 1) * LC); };
         auto build_group = [&](int g) {
@@ -725,12 +729,12 @@ __global__ void __launch_bounds__(NW * 32, kMinB) k_scan(ScanArgs a) {
                         const uint64_t lim = *reinterpret_cast<volatile unsigned long long*>(&s_thr);
                         wcount = warp_keep_upto(wbuf, min(wcount, wcap), lim);
                         if (wcount > kp) {
-                            const uint64_t kth = warp_select_keep(wbuf, wcount, kp, hist);
+                            uint64_t bound;
+                            wcount = warp_trim(wbuf, wcount, kp, wcap - kSbPerWarp * kSuperBlock, hist, bound);
                             if (lane == 0) {
-                                atomicMin(&s_thr, static_cast<unsigned long long>(kth));
-                                if (a.qthr) atomicMin(a.qthr + qi, static_cast<unsigned long long>(kth));
+                                atomicMin(&s_thr, static_cast<unsigned long long>(bound));
+                                if (a.qthr) atomicMin(a.qthr + qi, static_cast<unsigned long long>(bound));
                             }
-                            wcount = kp;
                         }
                     }
                 }
@@ -899,7 +903,15 @@ static std::vector<ScanShape> scan_shapes(int kp, int m_pad, int qtab_len, int p
         }
         return added > 0;
     };
-    if ((force == -1 || force == 0) && !fits(kUnstaged, false, 110 * 1024, 3)) fits(kUnstaged, false, 226 * 1024, 1);
+    if (force == -1 || force == 0) {
+        // a large k' leaves two blocks per SM fewer than 8 warps each: one block of
+        // 8 goes first then (256 filtered queries, k' = 1,000: 562 -> 511 us)
+        fits(kUnstaged, false, 110 * 1024, 3);
+        if (out.empty() || out.front().nw < 8) {
+            fits(kUnstaged, false, 226 * 1024, 1);
+            std::rotate(out.begin(), out.end() - 1, out.end());
+        }
+    }
     if (force == -1 || force == 2) {
         // dense: 8 warps x 3 blocks or 4 warps x 5 blocks per SM, the widest
         // LUT group whose shared memory allows that many blocks
