@@ -11,6 +11,8 @@
 #include <algorithm>
 #include <numeric>
 
+#include <sys/mman.h>
+
 namespace qg {
 
 // Warp per row: the column with the smallest key, first column on ties.
@@ -83,13 +85,14 @@ void assign_nearest(const float* x_dev, size_t n, const float* c_dev, size_t k, 
 
 // PQ codes of residuals x - center[assign], K = 16, thread per (row, subspace):
 // lo/hi halves start with a rounded product, then FMA over the remaining
-// sub-dimensions; the code is the first index of the minimum.
+// sub-dimensions; the code is the first index of the minimum. With order, the
+// j-th codes are row order[j]'s.
 __global__ void k_encode16(const float* __restrict__ x, size_t n, int dim, const float* __restrict__ centers,
                            const uint32_t* __restrict__ assign, const float* __restrict__ yt, int m, int sd,
-                           uint8_t* __restrict__ codes) {
+                           const uint32_t* __restrict__ order, uint8_t* __restrict__ codes) {
     const size_t t = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t >= n * m) return;
-    const size_t i = t / m;
+    const size_t i = order ? order[t / m] : t / m;
     const int s = static_cast<int>(t % m);
     const float* xr = x + i * dim + s * sd;
     const float* cr = centers + static_cast<size_t>(assign[i]) * dim + s * sd;
@@ -125,32 +128,84 @@ __global__ void k_encode16(const float* __restrict__ x, size_t n, int dim, const
 void encode16(const float* x, size_t n, int dim, const float* centers, const uint32_t* assign, const float* yt, int m,
               int sd, uint8_t* codes, cudaStream_t st) {
     if (n == 0) return;
-    k_encode16<<<static_cast<unsigned>(ceil_div(n * m, 256)), 256, 0, st>>>(x, n, dim, centers, assign, yt, m, sd, codes);
+    k_encode16<<<static_cast<unsigned>(ceil_div(n * m, 256)), 256, 0, st>>>(x, n, dim, centers, assign, yt, m, sd,
+                                                                           nullptr, codes);
     QG_LAUNCH_CHECK();
 }
 
-// Rows prepared for the metric: cosine rows scaled to unit length on the GPU
+// Rows on the GPU, prepared for the metric: cosine rows scaled to unit length
 // (reference src/index.cpp:193-218); a zero row refuses the whole call.
-static std::vector<float> prepare_rows(Metric metric, const float* x, size_t n, size_t dim, DevBuf<float>& dev,
-                                       cudaStream_t st) {
-    DevBuf<float> raw(n * dim, st);
-    QG_CUDA(cudaMemcpyAsync(raw.get(), x, n * dim * 4, cudaMemcpyHostToDevice, st));
-    std::vector<float> out(n * dim);
-    if (metric == Metric::Cosine) {
-        dev.alloc(n * dim, st);
-        DevBuf<int> zero(1, st);
-        QG_CUDA(cudaMemsetAsync(zero.get(), 0, 4, st));
-        normalize_rows(raw.get(), dev.get(), static_cast<int>(n), static_cast<int>(dim), zero.get(), st);
-        int z = 0;
-        QG_CUDA(cudaMemcpyAsync(&z, zero.get(), 4, cudaMemcpyDeviceToHost, st));
-        QG_CUDA(cudaMemcpyAsync(out.data(), dev.get(), n * dim * 4, cudaMemcpyDeviceToHost, st));
-        QG_CUDA(cudaStreamSynchronize(st));
-        if (z) throw Error(kInvalidArgument, "cosine metric needs non-zero vectors");
-    } else {
-        dev = std::move(raw);
-        std::copy(x, x + n * dim, out.begin());
+static void prepare_rows(Metric metric, const float* x, size_t n, size_t dim, DevBuf<float>& dev, cudaStream_t st) {
+    dev.alloc(n * dim, st);
+    QG_CUDA(cudaMemcpyAsync(dev.get(), x, n * dim * 4, cudaMemcpyHostToDevice, st));
+    if (metric != Metric::Cosine) return;
+    DevBuf<float> unit(n * dim, st);
+    DevBuf<int> zero(1, st);
+    QG_CUDA(cudaMemsetAsync(zero.get(), 0, 4, st));
+    normalize_rows(dev.get(), unit.get(), static_cast<int>(n), static_cast<int>(dim), zero.get(), st);
+    int z = 0;
+    QG_CUDA(cudaMemcpyAsync(&z, zero.get(), 4, cudaMemcpyDeviceToHost, st));
+    QG_CUDA(cudaStreamSynchronize(st));
+    if (z) throw Error(kInvalidArgument, "cosine metric needs non-zero vectors");
+    dev = std::move(unit);
+}
+
+// The prepared rows appended to the index's own: the caller's where the metric
+// leaves them as they are, else from the GPU through two pinned buffers, so
+// that each value is written to fresh memory once (a whole copy in between cost
+// as much again, most of it in page faults).
+static void append_rows(Metric metric, const float* x, size_t n, size_t dim, const DevBuf<float>& dev,
+                        std::vector<float>& data, cudaStream_t st) {
+    const size_t total = n * dim;
+    if (data.size() + total > data.capacity()) {
+        data.reserve(data.size() + std::max(data.size(), total));
+        // fresh memory in huge pages where the system has them
+        constexpr uintptr_t kHuge = uintptr_t{2} << 20;
+        const uintptr_t b = (reinterpret_cast<uintptr_t>(data.data() + data.size()) + kHuge - 1) & ~(kHuge - 1);
+        const uintptr_t e = reinterpret_cast<uintptr_t>(data.data() + data.capacity()) & ~(kHuge - 1);
+        if (e > b) (void)::madvise(reinterpret_cast<void*>(b), e - b, MADV_HUGEPAGE);
     }
-    return out;
+    if (metric != Metric::Cosine) {
+        data.insert(data.end(), x, x + total);
+        return;
+    }
+    const size_t had = data.size();
+    constexpr size_t kStep = size_t{1} << 20;   // floats per buffer
+    struct Pinned {
+        float* p = nullptr;
+        cudaEvent_t done = nullptr;
+        explicit Pinned(size_t floats) {
+            QG_CUDA(cudaMallocHost(reinterpret_cast<void**>(&p), floats * 4));
+            if (cudaEventCreateWithFlags(&done, cudaEventDisableTiming) != cudaSuccess) {
+                cudaFreeHost(p);
+                throw Error(kCudaError, "cudaEventCreateWithFlags failed");
+            }
+        }
+        ~Pinned() {
+            cudaEventDestroy(done);
+            cudaFreeHost(p);
+        }
+    };
+    const size_t step = std::min(kStep, total);
+    Pinned a(step), b(step);
+    Pinned* const buf[2] = {&a, &b};
+    auto start = [&](size_t at, Pinned& to) {
+        QG_CUDA(cudaMemcpyAsync(to.p, dev.get() + at, std::min(step, total - at) * 4, cudaMemcpyDeviceToHost, st));
+        QG_CUDA(cudaEventRecord(to.done, st));
+    };
+    try {
+        if (total) start(0, a);
+        int cur = 0;
+        for (size_t at = 0; at < total; at += step, cur ^= 1) {
+            if (at + step < total) start(at + step, *buf[cur ^ 1]);
+            QG_CUDA(cudaEventSynchronize(buf[cur]->done));
+            data.insert(data.end(), buf[cur]->p, buf[cur]->p + std::min(step, total - at));
+        }
+    } catch (...) {
+        cudaStreamSynchronize(st);   // no copy may land in a freed buffer
+        data.resize(had);
+        throw;
+    }
 }
 
 // IVFIndex::add_batch_impl on prepared rows (reference src/ivf_index.cpp:111-195).
@@ -161,7 +216,10 @@ static void ivf_add_impl(IVFObj& o, const float* x_dev, size_t n, const int64_t*
     M.idmap.check(n, ids);
     const uint32_t first = static_cast<uint32_t>(M.idmap.slots());
     const int dim = static_cast<int>(M.dim), m = static_cast<int>(M.pq.m), sd = static_cast<int>(M.pq.sub_dim);
-    std::vector<uint32_t> assign(n);
+    // the new vectors list by list, in input order within each (grouped and
+    // encoded in that order on the device, so each list takes one block of ids
+    // and one of codes)
+    std::vector<uint32_t> order(n), off(M.nlist + 1, 0);
     std::vector<uint8_t> codes(n * m);
     if (n) {
         DevBuf<float> cent(M.centroids.size(), st);
@@ -188,19 +246,23 @@ static void ivf_add_impl(IVFObj& o, const float* x_dev, size_t n, const int64_t*
         DevBuf<uint32_t> da(n, st);
         assign_nearest(x_dev, n, cent.get(), M.nlist, dim, da.get(), st);
         DevBuf<uint8_t> dc(n * m, st);
+        DevBuf<uint32_t> dorder(n, st), doff(M.nlist + 1, st);
+        group_by_label(da.get(), n, static_cast<int>(M.nlist), 1, dorder.get(), doff.get(), st);
         k_encode16<<<static_cast<unsigned>(ceil_div(n * m, 256)), 256, 0, st>>>(x_dev, n, dim, centers, da.get(), dyt.get(),
-                                                                                 m, sd, dc.get());
+                                                                                 m, sd, dorder.get(), dc.get());
         QG_LAUNCH_CHECK();
-        QG_CUDA(cudaMemcpyAsync(assign.data(), da.get(), n * 4, cudaMemcpyDeviceToHost, st));
+        QG_CUDA(cudaMemcpyAsync(order.data(), dorder.get(), n * 4, cudaMemcpyDeviceToHost, st));
+        QG_CUDA(cudaMemcpyAsync(off.data(), doff.get(), off.size() * 4, cudaMemcpyDeviceToHost, st));
         QG_CUDA(cudaMemcpyAsync(codes.data(), dc.get(), n * m, cudaMemcpyDeviceToHost, st));
         QG_CUDA(cudaStreamSynchronize(st));
     }
     M.idmap.add(n, ids);
-    // append in input order within each list
-    for (size_t i = 0; i < n; ++i) {
-        const uint32_t l = assign[i];
-        M.list_ids[l].push_back(first + static_cast<uint32_t>(i));
-        M.list_codes[l].insert(M.list_codes[l].end(), codes.begin() + i * m, codes.begin() + (i + 1) * m);
+    for (uint32_t& i : order) i += first;
+    for (size_t l = 0; l < M.nlist; ++l) {
+        if (off[l] == off[l + 1]) continue;
+        M.list_ids[l].insert(M.list_ids[l].end(), order.begin() + off[l], order.begin() + off[l + 1]);
+        M.list_codes[l].insert(M.list_codes[l].end(), codes.begin() + static_cast<size_t>(off[l]) * m,
+                               codes.begin() + static_cast<size_t>(off[l + 1]) * m);
     }
     o.dev_dirty = true;
 }
@@ -234,26 +296,26 @@ void add(IndexObj& idx, const float* x, size_t n, const int64_t* ids, int64_t* o
         auto& o = static_cast<FlatObj&>(idx);
         o.model.idmap.check(n, ids);
         DevBuf<float> dev;
-        std::vector<float> rows = prepare_rows(o.model.metric, x, n, dim, dev, st);
+        prepare_rows(o.model.metric, x, n, dim, dev, st);
+        append_rows(o.model.metric, x, n, dim, dev, o.model.data, st);
         o.model.idmap.add(n, ids);
-        o.model.data.insert(o.model.data.end(), rows.begin(), rows.end());
         o.dev_dirty = true;
     } else {
         auto& o = static_cast<RefineObj&>(idx);
         o.map.check(n, ids);
         o.materialize();   // rows of a mapped file move to memory before they change
         DevBuf<float> dev;
-        std::vector<float> rows = prepare_rows(o.metric(), x, n, dim, dev, st);
+        prepare_rows(o.metric(), x, n, dim, dev, st);
         if (o.base->kind == Kind::IVF) {
             ivf_add_impl(static_cast<IVFObj&>(*o.base), dev.get(), n, nullptr, st);
         } else {
             auto& b = static_cast<FlatObj&>(*o.base);
+            append_rows(o.metric(), x, n, dim, dev, b.model.data, st);
             b.model.idmap.add(n, nullptr);
-            b.model.data.insert(b.model.data.end(), rows.begin(), rows.end());
             b.dev_dirty = true;
         }
+        append_rows(o.metric(), x, n, dim, dev, o.data, st);
         o.map.add(n, ids);
-        o.data.insert(o.data.end(), rows.begin(), rows.end());
         o.dev_dirty = true;
     }
     if (out_ids)
