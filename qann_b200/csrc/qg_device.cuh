@@ -648,4 +648,113 @@ __device__ __noinline__ static uint32_t block_threshold_u32(const uint32_t* keys
     return *s_t;
 }
 
+// ---------------------------------------------------------------------------
+// The `want` smallest of n keys get(0 .. n-1) (distinct but for all-ones keys,
+// which are empty), by one block: put(rank, key, i) is called once for each of
+// them, in any order; returns how many there are, or -1 with nothing put when
+// the list would not hold them. The keys are counted into 1,024 equal
+// intervals of their high halves' range; those up to the interval that holds
+// the last one wanted are listed interval by interval, and a key's rank is its
+// interval's start plus the smaller keys in it (a few, as a rule). Six barriers,
+// where a bitonic sort of 1,024 pairs takes 55. lkey / lidx: room entries of
+// shared memory; blockDim.x a power of two from 32 to 1,024.
+// ---------------------------------------------------------------------------
+struct RankScratch {
+    int bins[1024];
+    uint32_t lo[32], hi[32];
+    int sum[32], bin, upto;
+};
+
+template <class Get, class Put>
+__device__ __forceinline__ int block_rank_smallest(int n, int want, Get get, uint64_t* lkey, uint32_t* lidx, int room,
+                                                   RankScratch& s, Put put) {
+    constexpr unsigned kFull = 0xffffffffu;
+    constexpr int U = 4;   // keys in flight per thread
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    const int step = U * static_cast<int>(blockDim.x);
+    auto each = [&](auto use) {
+        for (int b0 = 0; b0 < n; b0 += step) {
+            uint64_t k[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int i = b0 + u * static_cast<int>(blockDim.x) + static_cast<int>(threadIdx.x);
+                k[u] = i < n ? get(i) : ~0ull;
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (k[u] != ~0ull) use(k[u], b0 + u * static_cast<int>(blockDim.x) + static_cast<int>(threadIdx.x));
+        }
+    };
+    uint32_t lo = ~0u, hi = 0;
+    int valid = 0;
+    each([&](uint64_t k, int) {
+        const uint32_t h = static_cast<uint32_t>(k >> 32);
+        lo = min(lo, h);
+        hi = max(hi, h);
+        ++valid;
+    });
+    lo = __reduce_min_sync(kFull, lo);
+    hi = __reduce_max_sync(kFull, hi);
+    valid = __reduce_add_sync(kFull, valid);
+    for (int b = threadIdx.x; b < 1024; b += blockDim.x) s.bins[b] = 0;
+    if (lane == 0) {
+        s.lo[warp] = lo;
+        s.hi[warp] = hi;
+        s.sum[warp] = valid;
+    }
+    __syncthreads();
+    valid = 0;
+    for (int w = 0; w < nw; ++w) {
+        lo = min(lo, s.lo[w]);
+        hi = max(hi, s.hi[w]);
+        valid += s.sum[w];
+    }
+    want = min(want, valid);
+    if (want == 0) return 0;   // (block-uniform)
+    const KeyBins kb(lo, static_cast<uint64_t>(hi - lo) + 1, 1024);
+    each([&](uint64_t k, int) { atomicAdd(&s.bins[kb.bin(static_cast<uint32_t>(k >> 32))], 1); });
+    __syncthreads();
+    const int per = 1024 / static_cast<int>(blockDim.x);   // bins per thread
+    int own = 0;
+    for (int b = 0; b < per; ++b) own += s.bins[per * threadIdx.x + b];
+    int incl = own;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(kFull, incl, o);
+        if (lane >= o) incl += t;
+    }
+    if (lane == 31) s.sum[warp] = incl;   // (its last readers are behind the barrier above)
+    __syncthreads();
+    int acc = incl - own;
+    for (int w = 0; w < warp; ++w) acc += s.sum[w];
+    for (int b = 0; b < per; ++b) {
+        const int c = s.bins[per * threadIdx.x + b];
+        s.bins[per * threadIdx.x + b] = acc;
+        if (acc < want && want <= acc + c) {
+            s.bin = per * static_cast<int>(threadIdx.x) + b;
+            s.upto = acc + c;
+        }
+        acc += c;
+    }
+    __syncthreads();
+    const int last = s.bin, upto = s.upto;
+    if (upto > room) return -1;   // (block-uniform)
+    each([&](uint64_t k, int i) {
+        const int b = kb.bin(static_cast<uint32_t>(k >> 32));
+        if (b > last) return;
+        const int at = atomicAdd(&s.bins[b], 1);
+        lkey[at] = k;
+        lidx[at] = static_cast<uint32_t>(i);
+    });
+    __syncthreads();   // interval b now ends at bins[b], where interval b + 1 starts
+    for (int i = threadIdx.x; i < upto; i += blockDim.x) {
+        const uint64_t k = lkey[i];
+        const int b = kb.bin(static_cast<uint32_t>(k >> 32));
+        const int start = b > 0 ? s.bins[b - 1] : 0, end = s.bins[b];
+        int rank = start;
+        for (int e = start; e < end; ++e) rank += lkey[e] < k;
+        if (rank < want) put(rank, k, lidx[i]);
+    }
+    return want;
+}
+
 } // namespace qg
