@@ -555,7 +555,7 @@ def small_workload(args):
 def flat_workload(args):
     """Exact flat search as a GEMM: 10,000,000 x 96 float32 (N(0,1) per
     dimension, rows scaled by LogNormal(0, 0.25)), 10,000 queries of the same
-    law, k = 100, squared L2 and inner product. Exact results through the BF16
+    law, k = 100, squared L2 and inner product. Exact results through the F16
     tensor-core filter and FP32 recheck; per-distance error against FP64."""
     import torch
     import qann_b200 as qb
@@ -624,7 +624,7 @@ def flat_workload(args):
     print(json.dumps({
         "metric": "exact flat search QPS (10M x 96, k=100)", "value": l2["qps"], "unit": "queries/s", "n_gpus": 1,
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": l2["ms_per_step"], "higher_is_better": True,
-        "scaling": "weak", "vs_baseline": None, "dtype": "bf16 filter + f32 recheck", "data": "synthetic",
+        "scaling": "weak", "vs_baseline": None, "dtype": "f16 filter + f32 recheck", "data": "synthetic",
         "config": {"workload": f"flat_{n}x{d}_k{k}", "nq": nq, "l2": "inputs larger than L2 (3.84 GB rows)"},
         "per_metric": per_metric,
         "roofline": {"bound": "tensor", "achieved": l2["tensor_tflops"], "peak": peak, "unit": "TFLOP/s",
@@ -676,7 +676,7 @@ def train_workload(args):
     print(json.dumps({
         "metric": "IVF training time (2M x 128, nlist 16384, 20 Lloyd iterations, PQ 64x4)", "value": round(secs, 2),
         "unit": "s", "n_gpus": 1, "steps": 1, "warmup": 1, "ms_per_step": round(secs * 1e3, 1),
-        "higher_is_better": False, "scaling": "weak", "vs_baseline": None, "dtype": "bf16 filter + f32/f64",
+        "higher_is_better": False, "scaling": "weak", "vs_baseline": None, "dtype": "f16 filter + f32/f64",
         "data": "synthetic", "config": {"workload": f"train_{n}x{d}_nl{nlist}_lloyd{iters}_pq{m}"},
         "assign_pairs_per_s": round(pairs / secs, 1), "filter_schedule": qb.filter_options(), "cpu_baseline": cpu}))
     return 0

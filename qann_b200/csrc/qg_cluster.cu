@@ -236,22 +236,6 @@ void cluster_means(const float* sums, const uint32_t* off, int k, int d, int P, 
     QG_LAUNCH_CHECK();
 }
 
-// rows made unit length in place or into dst (zero rows become zero)
-__global__ void k_unit_rows(const float* __restrict__ src, size_t k, int d, float* __restrict__ dst) {
-    const size_t j = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (j >= k) return;
-    float* row = dst + j * d;
-    if (row != src + j * d)
-        for (int l = 0; l < d; ++l) row[l] = src[j * d + l];
-    unit_scale_row(row, d, true);
-}
-
-void unit_rows_dev(const float* src, size_t k, int d, float* dst, cudaStream_t st) {
-    if (k == 0) return;
-    k_unit_rows<<<static_cast<unsigned>(ceil_div(k, 128)), 128, 0, st>>>(src, k, d, dst);
-    QG_LAUNCH_CHECK();
-}
-
 // ---------------------------------------------------------------------------
 // e-means state on the device: centroid positions, masses, and the closing
 // pass's sums and counts. One step moves every cluster that received points
