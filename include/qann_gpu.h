@@ -217,8 +217,8 @@ int qg_fast_scan_noalloc_dev(const uint8_t* lut_dev, size_t nluts, size_t m, con
  *   "tensor_filter_redone" (those redone exactly after a candidate overflow). The same mode sends an IVF search's
  *   coarse step (the nprobe nearest lists, reference src/ivf_index.cpp:305-419) through F16 estimates with an
  *   error bound and an exact FP32 recheck of the lists that can still be among the nearest; qg_get_option reads
- *   "tensor_coarse_queries", "tensor_coarse_redone" (queries sent back to the exact path after too many
- *   near-ties) and "tensor_coarse_candidates" (lists rescored exactly). No counterpart in the reference, whose
+ *   "tensor_coarse_queries", "tensor_coarse_redone" (queries taken by a second pass with room for every list,
+ *   after too many near-ties) and "tensor_coarse_candidates" (lists rescored exactly). No counterpart in the reference, whose
  *   exact scores always come from its CPU distance kernels (reference src/flat_index.cpp:33-64).
  *   Filtered IVF searches rank only the nearest lists their probe walk is expected to need, through the same
  *   coarse step; "filtered_batches" counts filtered batches and "filtered_deep_walks" those of them whose walk
