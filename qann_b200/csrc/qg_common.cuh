@@ -141,60 +141,6 @@ __device__ __forceinline__ float exact_avx2(const float* __restrict__ a, const f
     return exact_tail<kL2>(a, b, n8, n, r);
 }
 
-// exact_avx2 with all 32 accumulators advanced together: each 32-float step
-// of a and b is eight 16-byte loads (both 16-byte aligned, n % 4 == 0). Every
-// accumulator's FMA chain runs in the same order as in exact_avx2, so the
-// result is the same to the bit; the loads of a step are all in flight at once.
-template <bool kL2>
-__device__ __forceinline__ float exact_avx2_vec(const float* __restrict__ a, const float* __restrict__ b, int n) {
-    const int n32 = n & ~31;
-    const int n8 = n & ~7;
-    float acc[32];   // acc[8 * j + L]: accumulator j, AVX2 lane L
-#pragma unroll
-    for (int e = 0; e < 32; ++e) acc[e] = 0.0f;
-    const float4* a4 = reinterpret_cast<const float4*>(a);
-    const float4* b4 = reinterpret_cast<const float4*>(b);
-    auto step4 = [&](const float4& av, const float4& bv, int base) {   // two chains per packed instruction
-        const float2 x01 = make_float2(av.x, av.y), x23 = make_float2(av.z, av.w);
-        const float2 y01 = make_float2(bv.x, bv.y), y23 = make_float2(bv.z, bv.w);
-        float2 c01 = make_float2(acc[base], acc[base + 1]), c23 = make_float2(acc[base + 2], acc[base + 3]);
-        if (kL2) {
-            const float2 d01 = sub2(x01, y01), d23 = sub2(x23, y23);
-            c01 = __ffma2_rn(d01, d01, c01);
-            c23 = __ffma2_rn(d23, d23, c23);
-        } else {
-            c01 = __ffma2_rn(x01, y01, c01);
-            c23 = __ffma2_rn(x23, y23, c23);
-        }
-        acc[base] = c01.x;
-        acc[base + 1] = c01.y;
-        acc[base + 2] = c23.x;
-        acc[base + 3] = c23.y;
-    };
-    for (int i = 0; i < n32; i += 32) {
-        float4 av[8], bv[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            av[k] = __ldg(a4 + (i >> 2) + k);
-            bv[k] = __ldg(b4 + (i >> 2) + k);
-        }
-#pragma unroll
-        for (int k = 0; k < 8; ++k) step4(av[k], bv[k], 4 * k);
-    }
-    for (int i = n32; i < n8; i += 8) {   // 8-float steps into accumulator 0
-        const float4 a0 = __ldg(a4 + (i >> 2)), a1 = __ldg(a4 + (i >> 2) + 1);
-        const float4 b0 = __ldg(b4 + (i >> 2)), b1 = __ldg(b4 + (i >> 2) + 1);
-        step4(a0, b0, 0);
-        step4(a1, b1, 4);
-    }
-    float s[8];
-#pragma unroll
-    for (int L = 0; L < 8; ++L) s[L] = __fadd_rn(__fadd_rn(acc[L], acc[8 + L]), __fadd_rn(acc[16 + L], acc[24 + L]));
-    const float r = __fadd_rn(__fadd_rn(__fadd_rn(s[0], s[4]), __fadd_rn(s[1], s[5])),
-                              __fadd_rn(__fadd_rn(s[2], s[6]), __fadd_rn(s[3], s[7])));
-    return exact_tail<kL2>(a, b, n8, n, r);
-}
-
 // exact_avx2 of one row by the 4 lanes of an aligned lane group: lane h runs
 // AVX2 lanes 2h and 2h + 1 (their four FMA chains, packed, over one 8-byte load
 // of a and of b per step), so each step of the group reads one 32-byte sector

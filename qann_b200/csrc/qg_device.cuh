@@ -107,17 +107,6 @@ __device__ __forceinline__ void warp_sort_keys_reg(uint64_t* key, int n) {
         if (i * 32 + lane < n) key[i * 32 + lane] = r[i];
 }
 
-// warp_sort_keys_reg for n <= 256 keys; false (nothing done) when n is larger.
-__device__ __forceinline__ bool warp_sort_keys(uint64_t* key, int n) {
-    if (n <= 32) warp_sort_keys_reg<1>(key, n);
-    else if (n <= 64) warp_sort_keys_reg<2>(key, n);
-    else if (n <= 128) warp_sort_keys_reg<4>(key, n);
-    else if (n <= 256) warp_sort_keys_reg<8>(key, n);
-    else return false;
-    __syncwarp();
-    return true;
-}
-
 __host__ __device__ __forceinline__ int next_pow2(int n) {
     int p = 1;
     while (p < n) p <<= 1;
