@@ -11,7 +11,6 @@
 #include <algorithm>
 #include <numeric>
 
-#include <sys/mman.h>
 
 namespace qg {
 
@@ -151,58 +150,25 @@ static void prepare_rows(Metric metric, const float* x, size_t n, size_t dim, De
 }
 
 // The prepared rows appended to the index's own: the caller's where the metric
-// leaves them as they are, else from the GPU through two pinned buffers, so
-// that each value is written to fresh memory once (a whole copy in between cost
-// as much again, most of it in page faults).
+// leaves them as they are, else copied from the GPU straight to their place (a
+// whole copy in between cost as much again, most of it in page faults). Plain
+// pages and a plain copy (an add of 165,423 x 37: 8.2 ms with the copy in between, 5.5
+// without): huge pages asked for by madvise and two pinned buffers
+// were faster on a quiet host, but an add of 165,423 x 37 then took 15 to 122 ms
+// where it takes 8, whenever the host had to compact its memory first.
 static void append_rows(Metric metric, const float* x, size_t n, size_t dim, const DevBuf<float>& dev,
                         std::vector<float>& data, cudaStream_t st) {
-    const size_t total = n * dim;
-    if (data.size() + total > data.capacity()) {
-        data.reserve(data.size() + std::max(data.size(), total));
-        // fresh memory in huge pages where the system has them
-        constexpr uintptr_t kHuge = uintptr_t{2} << 20;
-        const uintptr_t b = (reinterpret_cast<uintptr_t>(data.data() + data.size()) + kHuge - 1) & ~(kHuge - 1);
-        const uintptr_t e = reinterpret_cast<uintptr_t>(data.data() + data.capacity()) & ~(kHuge - 1);
-        if (e > b) (void)::madvise(reinterpret_cast<void*>(b), e - b, MADV_HUGEPAGE);
-    }
+    const size_t total = n * dim, had = data.size();
     if (metric != Metric::Cosine) {
         data.insert(data.end(), x, x + total);
         return;
     }
-    const size_t had = data.size();
-    constexpr size_t kStep = size_t{1} << 20;   // floats per buffer
-    struct Pinned {
-        float* p = nullptr;
-        cudaEvent_t done = nullptr;
-        explicit Pinned(size_t floats) {
-            QG_CUDA(cudaMallocHost(reinterpret_cast<void**>(&p), floats * 4));
-            if (cudaEventCreateWithFlags(&done, cudaEventDisableTiming) != cudaSuccess) {
-                cudaFreeHost(p);
-                throw Error(kCudaError, "cudaEventCreateWithFlags failed");
-            }
-        }
-        ~Pinned() {
-            cudaEventDestroy(done);
-            cudaFreeHost(p);
-        }
-    };
-    const size_t step = std::min(kStep, total);
-    Pinned a(step), b(step);
-    Pinned* const buf[2] = {&a, &b};
-    auto start = [&](size_t at, Pinned& to) {
-        QG_CUDA(cudaMemcpyAsync(to.p, dev.get() + at, std::min(step, total - at) * 4, cudaMemcpyDeviceToHost, st));
-        QG_CUDA(cudaEventRecord(to.done, st));
-    };
+    if (total == 0) return;
+    data.resize(had + total);
     try {
-        if (total) start(0, a);
-        int cur = 0;
-        for (size_t at = 0; at < total; at += step, cur ^= 1) {
-            if (at + step < total) start(at + step, *buf[cur ^ 1]);
-            QG_CUDA(cudaEventSynchronize(buf[cur]->done));
-            data.insert(data.end(), buf[cur]->p, buf[cur]->p + std::min(step, total - at));
-        }
+        QG_CUDA(cudaMemcpyAsync(data.data() + had, dev.get(), total * 4, cudaMemcpyDeviceToHost, st));
+        QG_CUDA(cudaStreamSynchronize(st));
     } catch (...) {
-        cudaStreamSynchronize(st);   // no copy may land in a freed buffer
         data.resize(had);
         throw;
     }
