@@ -154,8 +154,8 @@ static void prepare_rows(Metric metric, const float* x, size_t n, size_t dim, De
 // whole copy in between cost as much again, most of it in page faults). Plain
 // pages and a plain copy (an add of 165,423 x 37: 8.2 ms with the copy in between, 5.5
 // without): huge pages asked for by madvise and two pinned buffers
-// were faster on a quiet host, but an add of 165,423 x 37 then took 15 to 122 ms
-// where it takes 8, whenever the host had to compact its memory first.
+// were faster on a quiet host (a default build of 200,000 x 100 in 74 ms, now 78),
+// but the same add then took 15 to 122 ms whenever the host had to compact its memory first.
 static void append_rows(Metric metric, const float* x, size_t n, size_t dim, const DevBuf<float>& dev,
                         std::vector<float>& data, cudaStream_t st) {
     const size_t total = n * dim, had = data.size();
