@@ -907,10 +907,9 @@ static std::vector<ScanShape> scan_shapes(int kp, int m_pad, int qtab_len, int p
         // a large k' leaves two blocks per SM fewer than 8 warps each: one block of
         // 8 goes first then (256 filtered queries, k' = 1,000: 562 -> 511 us)
         fits(kUnstaged, false, 110 * 1024, 3);
-        if (out.empty() || out.front().nw < 8) {
-            fits(kUnstaged, false, 226 * 1024, 1);
+        // (where nothing fits, the list stays empty and the caller refuses the search)
+        if ((out.empty() || out.front().nw < 8) && fits(kUnstaged, false, 226 * 1024, 1))
             std::rotate(out.begin(), out.end() - 1, out.end());
-        }
     }
     if (force == -1 || force == 2) {
         // dense: 8 warps x 3 blocks or 4 warps x 5 blocks per SM, the widest
