@@ -49,7 +49,8 @@ constexpr int kSbPerWarp = 4;    // superblocks a warp takes at a time, one per 
 constexpr int kQtabStride = 20;
 constexpr int kFirstGroup = 3;   // lists in the first LUT group (at most LC)
 // Keys above k' that a trimmed buffer may hold: what one interval of the trim's
-// range takes in at most, as a rule.
+// range takes in at most, as a rule. Blocks of one warp, which are what is left
+// where the tables take nearly all of the shared memory, do without.
 constexpr int kTrimSlack = 32;
 }
 
@@ -271,7 +272,7 @@ __host__ __device__ inline ScanLayout scan_layout(int kp, int m_pad, int qtab_le
     ScanLayout L;
     L.nw = nw;
     L.lc = lc;
-    L.wcap = (kp + kTrimSlack + kSbPerWarp * kSuperBlock + 31) & ~31;
+    L.wcap = (kp + (nw > 1 ? kTrimSlack : 0) + kSbPerWarp * kSuperBlock + 31) & ~31;
     L.lut_stride = m_pad + 2;
     const size_t lut = shared_lut ? static_cast<size_t>(m_pad) * 16 : static_cast<size_t>(2) * lc * L.lut_stride * 16;
     const size_t gather = static_cast<size_t>(nw) * kp * 8;
