@@ -38,6 +38,7 @@ namespace qg {
 __global__ void __launch_bounds__(256) k_unit_rows(const float* x, float* y, size_t n, int d, int* zero_row) {
     __shared__ float t[32][33];
     __shared__ float s_scale[32];
+    __shared__ bool s_zero[32];   // (told apart from a scale that is NaN itself)
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     const size_t r0 = static_cast<size_t>(blockIdx.x) * 32;
     double s = 0.0;
@@ -68,15 +69,14 @@ __global__ void __launch_bounds__(256) k_unit_rows(const float* x, float* y, siz
             scale = s > 0.0 ? __double2float_rn(__ddiv_rn(1.0, __dsqrt_rn(s))) : 0.0f;
         }
         s_scale[tx] = scale;
-        // (told apart from a scale that is NaN itself)
-        t[0][tx] = zero_row && s == 0.0 ? 1.0f : 0.0f;
+        s_zero[tx] = zero_row && s == 0.0;
     }
     __syncthreads();
     for (int k = 0; k < 4; ++k) {
         const int r = ty + 8 * k;
         if (r0 + r >= n) continue;
         const float scale = s_scale[r];
-        const bool zero = t[0][r] != 0.0f;
+        const bool zero = s_zero[r];
         for (int c = tx; c < d; c += 32) {
             const size_t o = (r0 + r) * d + c;
             y[o] = zero ? 0.0f : __fmul_rn(x[o], scale);
