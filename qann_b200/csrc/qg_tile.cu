@@ -446,7 +446,9 @@ __global__ void __launch_bounds__(tile_threads<EPI>(), 1)
                 break;
             }
             tc_fence_after();
-            // one run of 32 columns: its products in v
+            __syncwarp();   // (the TMEM loads below want a converged warp)
+            // one run of 32 columns: its products in v. Lanes part ways in it (and where
+            // one of them hands back): each call is followed by a __syncwarp
             auto run = [&](int r, uint32_t (&v)[32]) {
                 if constexpr (MODE == kStore) {
                     const int c0 = w.nt * BN + col0 + 32 * r;
@@ -520,10 +522,12 @@ __global__ void __launch_bounds__(tile_threads<EPI>(), 1)
                     tmem_ld32_wait(va);
                     tmem_ld32_start(taddr + 32 * (r + 1), vb);
                     run(r, va);
+                    __syncwarp();
                     tmem_ld32_wait(vb);
                     if (r + 2 < kRuns) tmem_ld32_start(taddr + 32 * (r + 2), va);
                     else hand_back();
                     run(r + 1, vb);
+                    __syncwarp();
                 }
             } else {
 #pragma unroll 1
@@ -532,12 +536,13 @@ __global__ void __launch_bounds__(tile_threads<EPI>(), 1)
                     tmem_ld32(taddr + 32 * r, v);
                     if (r == kRuns - 1) hand_back();
                     run(r, v);
+                    __syncwarp();
                 }
             }
             acc ^= 1;
             if (acc == 0) apar ^= 1;
             if (MODE == kStore) continue;
-            __syncwarp();   // the warp's reads of the row terms are done
+            // (the warp's reads of the row terms are done)
             if (lane == 0) mbar_arrive(&empty_x[xb]);
             if (++xb == kTermBufs) {
                 xb = 0;
