@@ -11,7 +11,6 @@
 #include <algorithm>
 #include <numeric>
 
-
 namespace qg {
 
 // Warp per row: the column with the smallest key, first column on ties.
@@ -165,13 +164,35 @@ static void append_rows(Metric metric, const float* x, size_t n, size_t dim, con
     }
     if (total == 0) return;
     data.resize(had + total);
-    try {
-        QG_CUDA(cudaMemcpyAsync(data.data() + had, dev.get(), total * 4, cudaMemcpyDeviceToHost, st));
-        QG_CUDA(cudaStreamSynchronize(st));
-    } catch (...) {
-        data.resize(had);
-        throw;
+    QG_CUDA(cudaMemcpyAsync(data.data() + had, dev.get(), total * 4, cudaMemcpyDeviceToHost, st));
+    QG_CUDA(cudaStreamSynchronize(st));
+}
+
+// Runs `undo` when its scope is left before keep().
+template <class F>
+class Undo {
+public:
+    explicit Undo(F f) : f_(std::move(f)) {}
+    ~Undo() {
+        if (armed_) f_();
     }
+    void keep() { armed_ = false; }
+    Undo(const Undo&) = delete;
+    Undo& operator=(const Undo&) = delete;
+
+private:
+    F f_;
+    bool armed_ = true;
+};
+
+// A row store and its id map extended together, or neither: a failed copy or
+// allocation leaves both as they were.
+static void flat_add(Metric metric, const float* x, size_t n, size_t dim, const DevBuf<float>& dev, const int64_t* ids,
+                     std::vector<float>& data, IdMap& map, cudaStream_t st) {
+    Undo rows([&data, had = data.size()] { data.resize(had); });
+    append_rows(metric, x, n, dim, dev, data, st);
+    map.add(n, ids);
+    rows.keep();
 }
 
 // IVFIndex::add_batch_impl on prepared rows (reference src/ivf_index.cpp:111-195).
@@ -222,8 +243,13 @@ static void ivf_add_impl(IVFObj& o, const float* x_dev, size_t n, const int64_t*
         QG_CUDA(cudaMemcpyAsync(codes.data(), dc.get(), n * m, cudaMemcpyDeviceToHost, st));
         QG_CUDA(cudaStreamSynchronize(st));
     }
-    M.idmap.add(n, ids);
     for (uint32_t& i : order) i += first;
+    // all the room first: nothing has changed when one of these throws
+    for (size_t l = 0; l < M.nlist; ++l) {
+        make_room(M.list_ids[l], off[l + 1] - off[l]);
+        make_room(M.list_codes[l], static_cast<size_t>(off[l + 1] - off[l]) * m);
+    }
+    M.idmap.add(n, ids);
     for (size_t l = 0; l < M.nlist; ++l) {
         if (off[l] == off[l + 1]) continue;
         M.list_ids[l].insert(M.list_ids[l].end(), order.begin() + off[l], order.begin() + off[l + 1]);
@@ -263,8 +289,7 @@ void add(IndexObj& idx, const float* x, size_t n, const int64_t* ids, int64_t* o
         o.model.idmap.check(n, ids);
         DevBuf<float> dev;
         prepare_rows(o.model.metric, x, n, dim, dev, st);
-        append_rows(o.model.metric, x, n, dim, dev, o.model.data, st);
-        o.model.idmap.add(n, ids);
+        flat_add(o.model.metric, x, n, dim, dev, ids, o.model.data, o.model.idmap, st);
         o.dev_dirty = true;
     } else {
         auto& o = static_cast<RefineObj&>(idx);
@@ -272,16 +297,21 @@ void add(IndexObj& idx, const float* x, size_t n, const int64_t* ids, int64_t* o
         o.materialize();   // rows of a mapped file move to memory before they change
         DevBuf<float> dev;
         prepare_rows(o.metric(), x, n, dim, dev, st);
+        // the base last: a base slot without a row here would send a later search
+        // past the end of the rows
+        flat_add(o.metric(), x, n, dim, dev, ids, o.data, o.map, st);
+        Undo own([&o, n, total = n * dim] {
+            o.data.resize(o.data.size() - total);
+            o.map.take_back(n);
+        });
         if (o.base->kind == Kind::IVF) {
             ivf_add_impl(static_cast<IVFObj&>(*o.base), dev.get(), n, nullptr, st);
         } else {
             auto& b = static_cast<FlatObj&>(*o.base);
-            append_rows(o.metric(), x, n, dim, dev, b.model.data, st);
-            b.model.idmap.add(n, nullptr);
+            flat_add(o.metric(), x, n, dim, dev, nullptr, b.model.data, b.model.idmap, st);
             b.dev_dirty = true;
         }
-        append_rows(o.metric(), x, n, dim, dev, o.data, st);
-        o.map.add(n, ids);
+        own.keep();
         o.dev_dirty = true;
     }
     if (out_ids)

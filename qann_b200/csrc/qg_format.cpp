@@ -55,23 +55,35 @@ void IdMap::check(size_t n, const int64_t* ids) const {
 
 void IdMap::add(size_t n, const int64_t* ids) {
     check(n, ids);
-    if (!custom_) {
-        if (labels_.empty() && static_cast<size_t>(next_id_) == slots_) {
-            slots_ += n;
-            next_id_ += static_cast<int64_t>(n);
-        } else {
-            for (size_t i = 0; i < n; ++i) labels_.push_back(next_id_++);
-            slots_ += n;
+    const bool same = !custom_ && labels_.empty() && static_cast<size_t>(next_id_) == slots_;   // ids are slots
+    make_room(deleted_, n);
+    if (!same) make_room(labels_, n);
+    if (custom_) {
+        size_t i = 0;
+        try {
+            for (; i < n; ++i) slot_of_.emplace(ids[i], static_cast<uint32_t>(slots_ + i));
+        } catch (...) {
+            while (i > 0) slot_of_.erase(ids[--i]);
+            throw;
         }
-        deleted_.resize(slots_, 0);
-        return;
+        labels_.insert(labels_.end(), ids, ids + n);
+    } else if (same) {
+        next_id_ += static_cast<int64_t>(n);
+    } else {
+        for (size_t i = 0; i < n; ++i) labels_.push_back(next_id_++);
     }
-    for (size_t i = 0; i < n; ++i) {
-        labels_.push_back(ids[i]);
-        slot_of_[ids[i]] = static_cast<uint32_t>(slots_);
-        ++slots_;
-    }
+    slots_ += n;
     deleted_.resize(slots_, 0);
+}
+
+void IdMap::take_back(size_t n) noexcept {
+    slots_ -= n;
+    if (custom_)
+        for (size_t s = slots_; s < slots_ + n; ++s) slot_of_.erase(labels_[s]);
+    else
+        next_id_ -= static_cast<int64_t>(n);
+    if (!labels_.empty()) labels_.resize(slots_);
+    deleted_.resize(slots_);
 }
 
 // slot of an id, or -1 when unknown (deleted slots are reported; callers check)

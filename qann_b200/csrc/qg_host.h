@@ -85,6 +85,14 @@ struct Reader {
     [[noreturn]] static void throw_corrupt(const std::string& what);
 };
 
+// Room for `more` elements past v's size, which then grows by them without
+// throwing: at least twice what it had, as growing would take.
+template <class T>
+void make_room(std::vector<T>& v, size_t more) {
+    const size_t need = v.size() + more;
+    if (v.capacity() < need) v.reserve(need > 2 * v.capacity() ? need : 2 * v.capacity());
+}
+
 // ---- slot <-> id map (reference include/vecengine/id_map.hpp:42-131) --------
 
 struct SlotBits {
@@ -97,7 +105,8 @@ class IdMap {
 public:
     explicit IdMap(bool custom = false) : custom_(custom) {}
     void check(size_t n, const int64_t* ids) const;
-    void add(size_t n, const int64_t* ids);
+    void add(size_t n, const int64_t* ids);   // (nothing has changed when it throws)
+    void take_back(size_t n) noexcept;         // the last n added, none of them removed since
     size_t remove(std::span<const int64_t> ids, std::vector<uint32_t>* removed = nullptr);
     SlotBits filter(std::span<const int64_t> ids) const;
     SlotBits live(std::vector<uint64_t> words) const;
