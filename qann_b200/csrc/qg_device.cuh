@@ -242,12 +242,126 @@ struct KeyBins {
     }
 };
 
+// nbins equal intervals of the floats that the keys lo .. hi stand for, to rank
+// keys in. (Equal intervals of the keys themselves, KeyBins, are an eighth of an octave
+// when the range holds a zero or crosses it: scores of both signs, or a query that is
+// itself a row, then crowd into few.) Monotone in the key: the subtraction, the
+// product and the conversion are. KeyBins where the floats' range is not a positive
+// finite number.
+struct RankBins {
+    KeyBins keys;
+    float from, scale;
+    int top;
+    __device__ __forceinline__ RankBins(uint32_t lo, uint32_t hi, int nbins)
+        : keys(lo, static_cast<uint64_t>(hi - lo) + 1, nbins) {
+        from = key_float(lo);
+        scale = __fdiv_rn(static_cast<float>(nbins), __fsub_rn(key_float(hi), from));
+        top = scale > 0.0f && scale <= 3.402823466e+38f ? nbins - 1 : -1;
+    }
+    __device__ __forceinline__ int bin(uint32_t key) const {
+        return top < 0 ? keys.bin(key) : min(top, __float2int_rd(__fmul_rn(__fsub_rn(key_float(key), from), scale)));
+    }
+};
+
+// The work of ranking the c keys of one bin against each other, capped so that
+// the sum over a block's bins stays within 32 bits.
+__device__ __forceinline__ uint32_t bin_work(int c) { return static_cast<uint32_t>(c) * static_cast<uint32_t>(min(c, 4096)); }
+
+// The bin of a warp's 256 that holds the need-th of the keys counted in them
+// (need >= 1, at least so many), the keys in the bins before it, and the keys up to
+// its end. Each lane owns 8 bins; hist 16-byte aligned.
+__device__ __forceinline__ int warp_pick(const int* hist, int need, int& bin, int& before) {
+    const int lane = threadIdx.x & 31;
+    constexpr unsigned kFull = 0xffffffffu;
+    const int4* h4 = reinterpret_cast<const int4*>(hist);
+    const int4 c0 = h4[2 * lane], c1 = h4[2 * lane + 1];
+    const int c[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+    int own = 0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) own += c[j];
+    int incl = own;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(kFull, incl, o);
+        if (lane >= o) incl += t;
+    }
+    int acc = incl - own, upto = 0;
+    bin = -1;
+    before = 0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        if (acc < need && need <= acc + c[j]) {
+            bin = 8 * lane + j;
+            before = acc;
+            upto = acc + c[j];
+        }
+        acc += c[j];
+    }
+    const int owner = __ffs(__ballot_sync(kFull, bin >= 0)) - 1;
+    bin = __shfl_sync(kFull, bin, owner);
+    before = __shfl_sync(kFull, before, owner);
+    return __shfl_sync(kFull, upto, owner);
+}
+
+__device__ __forceinline__ void warp_zero_bins(int* hist) {
+    int4* h4 = reinterpret_cast<int4*>(hist);
+    h4[threadIdx.x & 31] = make_int4(0, 0, 0, 0);
+    h4[32 + (threadIdx.x & 31)] = make_int4(0, 0, 0, 0);
+}
+
+// warp_trim where one interval holds too many keys, as equal distances do: the
+// whole keys in [from, to] (`below` keys lie under it), cut again and again into
+// 256 intervals of what is left of their range. Distinct keys are apart once an
+// interval is one key wide, in at most 10 cuts; equal distances are after one.
+// (The radix select, up to 8 passes over keys that agree in their first 4
+// bytes, did this before: 1,000 queries over 40 distinct rows 1.4 -> 1.2 ms at k' = 1,000.)
+__device__ __noinline__ static int warp_trim_within(uint64_t* buf, int n, int keep, int room, int* hist, uint64_t from,
+                                                    uint64_t to, int below, uint64_t& lim) {
+    const int lane = threadIdx.x & 31;
+    constexpr unsigned kFull = 0xffffffffu;
+    for (int cut = 0; cut < 10; ++cut) {
+        unsigned long long lo = ~0ull, hi = 0;
+        for (int i = lane; i < n; i += 32) {
+            const unsigned long long k = buf[i];
+            if (k >= from && k <= to) {
+                lo = min(lo, k);
+                hi = max(hi, k);
+            }
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            lo = min(lo, __shfl_xor_sync(kFull, lo, o));
+            hi = max(hi, __shfl_xor_sync(kFull, hi, o));
+        }
+        const int sh = max(0, 56 - __clzll(static_cast<long long>(hi - lo)));   // (hi - lo) >> sh < 256
+        warp_zero_bins(hist);
+        __syncwarp();
+        for (int i = lane; i < n; i += 32) {
+            const unsigned long long k = buf[i];
+            if (k >= lo && k <= hi) atomicAdd(&hist[static_cast<int>((k - lo) >> sh)], 1);
+        }
+        __syncwarp();
+        int bin, before;
+        const int upto = warp_pick(hist, keep - below, bin, before);
+        __syncwarp();
+        const unsigned long long first = static_cast<unsigned long long>(bin) << sh, last = first | ((1ull << sh) - 1);
+        to = last >= hi - lo ? hi : lo + last;
+        // (`room` keys would leave no room for the next: near `keep`, the buffer lasts longer)
+        if (below + upto <= min(room, keep + 8)) {
+            lim = to;
+            return warp_keep_upto(buf, n, to);
+        }
+        from = lo + first;
+        below += before;
+    }
+    lim = warp_select_keep(buf, n, keep, hist);
+    return keep;
+}
+
 // One warp cuts the n distinct keys buf[0, n), in place and in order, to about
 // the `keep` smallest: all of them and at most `room` keys; returns how many
 // and, in lim, a key at or above the largest of them below which the others do
 // not lie. One pass over 256 intervals of the high halves' range, and the
 // interval that holds the keep-th key stays whole; where that is more than
-// `room`, the radix select (up to 8 passes) cuts to `keep` exactly. hist: 256
+// `room`, it is cut again (warp_trim_within). hist: 256
 // ints of warp-private scratch, 16-byte aligned. n > keep >= 1, room >= keep.
 __device__ __noinline__ static int warp_trim(uint64_t* buf, int n, int keep, int room, int* hist, uint64_t& lim) {
     const int lane = threadIdx.x & 31;
@@ -258,44 +372,21 @@ __device__ __noinline__ static int warp_trim(uint64_t* buf, int n, int keep, int
         lo = min(lo, k);
         hi = max(hi, k);
     }
-    int4* h4 = reinterpret_cast<int4*>(hist);
-    h4[lane] = make_int4(0, 0, 0, 0);
-    h4[32 + lane] = make_int4(0, 0, 0, 0);
+    warp_zero_bins(hist);
     lo = __reduce_min_sync(kFull, lo);
     hi = __reduce_max_sync(kFull, hi);
     __syncwarp();
     const KeyBins kb(lo, static_cast<uint64_t>(hi - lo) + 1, 256);
     for (int i = lane; i < n; i += 32) atomicAdd(&hist[kb.bin(static_cast<uint32_t>(buf[i] >> 32))], 1);
     __syncwarp();
-    const int4 c0 = h4[2 * lane], c1 = h4[2 * lane + 1];   // bins 8 lane .. 8 lane + 7
-    const int c[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-    int own = 0;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) own += c[j];
-    int incl = own;
-    for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(kFull, incl, o);
-        if (lane >= o) incl += t;
-    }
-    int acc = incl - own, bin = -1, kept = 0;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        if (acc < keep && keep <= acc + c[j]) {
-            bin = 8 * lane + j;
-            kept = acc + c[j];
-        }
-        acc += c[j];
-    }
-    const int owner = __ffs(__ballot_sync(kFull, bin >= 0)) - 1;
-    bin = __shfl_sync(kFull, bin, owner);
-    kept = __shfl_sync(kFull, kept, owner);
-    if (kept > room) {
-        lim = warp_select_keep(buf, n, keep, hist);
-        return keep;
-    }
-    const uint32_t T = static_cast<uint32_t>(min(kb.last(bin), static_cast<uint64_t>(hi)));
-    lim = (static_cast<uint64_t>(T) << 32) | 0xFFFFFFFFull;
-    return warp_keep_upto(buf, n, lim);
+    int bin, before;
+    const int kept = warp_pick(hist, keep, bin, before);
+    const uint64_t T = min(kb.last(bin), static_cast<uint64_t>(hi));
+    lim = (T << 32) | 0xFFFFFFFFull;
+    if (kept <= room) return warp_keep_upto(buf, n, lim);
+    __syncwarp();
+    const uint64_t from = bin > 0 ? (kb.last(bin - 1) + 1) << 32 : 0ull;
+    return warp_trim_within(buf, n, keep, room, hist, from, lim, before, lim);
 }
 
 // ---------------------------------------------------------------------------
@@ -641,18 +732,22 @@ __device__ __noinline__ static uint32_t block_threshold_u32(const uint32_t* keys
 // The `want` smallest of n keys get(0 .. n-1) (distinct but for all-ones keys,
 // which are empty), by one block: put(rank, key, i) is called once for each of
 // them, in any order; returns how many there are, or -1 with nothing put when
-// the list would not hold them. The keys are counted into 1,024 equal
-// intervals of their high halves' range; those up to the interval that holds
-// the last one wanted are listed interval by interval, and a key's rank is its
-// interval's start plus the smaller keys in it (a few, as a rule). Six barriers,
-// where a bitonic sort of 1,024 pairs takes 55. lkey / lidx: room entries of
+// the list would not hold them or they crowd into few intervals. The keys are
+// counted into 1,024 equal intervals of their high halves' range (RankBins); those up
+// to the interval that holds the last one wanted are listed interval by interval, and
+// a key's rank is its interval's start plus the smaller keys in it (a few, as a
+// rule). Six barriers, where a bitonic sort of 1,024 pairs takes 55. Ranking costs
+// the keys times the keys that share an interval, so past kCrowded of those on
+// average a sort is cheaper. lkey / lidx: room entries of
 // shared memory; blockDim.x a power of two from 32 to 1,024.
 // ---------------------------------------------------------------------------
 struct RankScratch {
     int bins[1024];
     uint32_t lo[32], hi[32];
     int sum[32], bin, upto;
+    uint32_t work;
 };
+inline constexpr uint32_t kCrowded = 64;
 
 template <class Get, class Put>
 __device__ __forceinline__ int block_rank_smallest(int n, int want, Get get, uint64_t* lkey, uint32_t* lidx, int room,
@@ -691,6 +786,7 @@ __device__ __forceinline__ int block_rank_smallest(int n, int want, Get get, uin
         s.hi[warp] = hi;
         s.sum[warp] = valid;
     }
+    if (threadIdx.x == 0) s.work = 0;
     __syncthreads();
     valid = 0;
     for (int w = 0; w < nw; ++w) {
@@ -700,7 +796,7 @@ __device__ __forceinline__ int block_rank_smallest(int n, int want, Get get, uin
     }
     want = min(want, valid);
     if (want == 0) return 0;   // (block-uniform)
-    const KeyBins kb(lo, static_cast<uint64_t>(hi - lo) + 1, 1024);
+    const RankBins kb(lo, hi, 1024);
     each([&](uint64_t k, int) { atomicAdd(&s.bins[kb.bin(static_cast<uint32_t>(k >> 32))], 1); });
     __syncthreads();
     const int per = 1024 / static_cast<int>(blockDim.x);   // bins per thread
@@ -715,18 +811,22 @@ __device__ __forceinline__ int block_rank_smallest(int n, int want, Get get, uin
     __syncthreads();
     int acc = incl - own;
     for (int w = 0; w < warp; ++w) acc += s.sum[w];
+    uint32_t work = 0;
     for (int b = 0; b < per; ++b) {
         const int c = s.bins[per * threadIdx.x + b];
         s.bins[per * threadIdx.x + b] = acc;
+        if (acc < want) work += bin_work(c);
         if (acc < want && want <= acc + c) {
             s.bin = per * static_cast<int>(threadIdx.x) + b;
             s.upto = acc + c;
         }
         acc += c;
     }
+    work = __reduce_add_sync(kFull, work);
+    if (lane == 0) atomicAdd(&s.work, work);
     __syncthreads();
     const int last = s.bin, upto = s.upto;
-    if (upto > room) return -1;   // (block-uniform)
+    if (upto > room || s.work > kCrowded * static_cast<uint32_t>(upto)) return -1;   // (block-uniform)
     each([&](uint64_t k, int i) {
         const int b = kb.bin(static_cast<uint32_t>(k >> 32));
         if (b > last) return;

@@ -52,6 +52,10 @@ constexpr int kFirstGroup = 3;   // lists in the first LUT group (at most LC)
 // range takes in at most, as a rule. Blocks of one warp, which are what is left
 // where the tables take nearly all of the shared memory, do without.
 constexpr int kTrimSlack = 32;
+// Ranking the keys of a unit against those of their bin costs about 1/16 cycle a pair,
+// sampled bins some 6,000 cycles and 2 a key: 1,000 queries over 40 distinct rows, k' =
+// 1,000, take 8.1 ms without them and 1.3 with (1.4 with one warp's radix select).
+constexpr uint32_t kCrowdedUnit = 32;
 }
 
 // LUT of one list by one warp. Same arithmetic as quantize_lut. Lane l forms
@@ -336,7 +340,7 @@ __global__ void __launch_bounds__(NW * 32, kMinB) k_scan(ScanArgs a) {
     __shared__ int s_next[2], s_build[2];
     __shared__ unsigned long long s_thr;
     __shared__ int s_wcount[NW];
-    __shared__ uint32_t s_red[NW], s_red2[NW];
+    __shared__ uint32_t s_red[NW], s_red2[NW], s_work;
 
     if (tid == 0) s_abort = 0;
     if (kStaged && lane == 0) {
@@ -509,6 +513,7 @@ __global__ void __launch_bounds__(NW * 32, kMinB) k_scan(ScanArgs a) {
             lo = __reduce_min_sync(kFull, lo);
             hi = __reduce_max_sync(kFull, hi);
             for (int t = tid; t < kBins; t += NT) bh[t] = 0;
+            if (tid == 0) s_work = 0;
             if (lane == 0) {
                 s_red[warp] = lo;
                 s_red2[warp] = hi;
@@ -771,8 +776,7 @@ __global__ void __launch_bounds__(NW * 32, kMinB) k_scan(ScanArgs a) {
 
         // ---- the unit's k' best: each warp's own, gathered, in order ----
         __syncwarp();
-        // keys above the block threshold first (as at a trim), so that fewer
-        // reach warp 0's cut below
+        // keys above the block threshold first (as at a trim)
         wcount = warp_keep_upto(wbuf, min(wcount, wcap), *reinterpret_cast<volatile unsigned long long*>(&s_thr));
         if (wcount > kp) {
             warp_select_keep(wbuf, min(wcount, wcap), kp, hist);
@@ -786,7 +790,9 @@ __global__ void __launch_bounds__(NW * 32, kMinB) k_scan(ScanArgs a) {
         // one's place is its bin's start plus the smaller keys in its bin. Most bins
         // hold a few keys. (Warp 0 alone cut and sorted them before: 20,700 cycles a
         // unit of 102,400 at k' = 100 and 1,000 queries, 32,700 of 378,700 at k' =
-        // 200 and 10,000, the other warps waiting.)
+        // 200 and 10,000, the other warps waiting.) Where a key shares its bin with
+        // many others, as equal distances do, the bins are laid between a sample of the
+        // keys instead.
         int off = 0, total = 0;
         for (int w = 0; w < NW; ++w) {
             if (w < warp) off += s_wcount[w];
@@ -798,36 +804,83 @@ __global__ void __launch_bounds__(NW * 32, kMinB) k_scan(ScanArgs a) {
         const int kept = min(total, kp);
         uint64_t* bucket = reinterpret_cast<uint64_t*>(sm + lay.off_wbuf);
         if (total > 0) {   // (block-uniform)
-            const KeyBins kb(lo, static_cast<uint64_t>(hi - lo) + 1, kBins);
+            const RankBins kb(lo, hi, kBins);
             for (int i = lane; i < wcount; i += 32) atomicAdd(&bh[kb.bin(static_cast<uint32_t>(wbuf[i] >> 32))], 1);
             __syncthreads();
             int own[kPer], acc;
             bin_prefix(own, acc);
+            uint32_t work = 0;
 #pragma unroll
             for (int b = 0; b < kPer; ++b) {
                 bh[kPer * tid + b] = acc;
+                if (acc < kp) work += bin_work(own[b]);
                 acc += own[b];
             }
+            work = __reduce_add_sync(kFull, work);
+            if (lane == 0) atomicAdd(&s_work, work);
             __syncthreads();
-            for (int i = tid; i < total; i += NT) {
-                const uint64_t key = gath[i];
-                bucket[atomicAdd(&bh[kb.bin(static_cast<uint32_t>(key >> 32))], 1)] = key;
-            }
-            __syncthreads();   // bin b now ends at bh[b], where bin b + 1 starts
-            for (int i = tid; i < total; i += NT) {
-                const uint64_t key = bucket[i];
-                const int b = kb.bin(static_cast<uint32_t>(key >> 32));
-                const int start = b > 0 ? bh[b - 1] : 0, end = bh[b];
-                if (start >= kp) continue;
-                int place = start;
-                for (int e = start; e < end; ++e) place += bucket[e] < key;
-                if (place >= kp) continue;
+            auto put = [&](int place, uint64_t key) {
                 const uint32_t push = static_cast<uint32_t>(key);
                 const int pp = upper_index(p_push, np, push);
                 const uint32_t pos = push - p_push[pp];
                 const size_t sbg = static_cast<size_t>(p_sboff[pp]) + pos / kSuperBlock;
                 a.out_key[ob + place] = key;
                 a.out_slot[ob + place] = v.ids[sbg * kSuperBlock + pos % kSuperBlock];
+            };
+            // start: where each bin starts in bucket[], on return where it ends
+            auto rank_out = [&](auto bin, int* start) {
+                for (int i = tid; i < total; i += NT) {
+                    const uint64_t key = gath[i];
+                    bucket[atomicAdd(&start[bin(key)], 1)] = key;
+                }
+                __syncthreads();   // bin b now ends at start[b], where bin b + 1 starts
+                for (int i = tid; i < total; i += NT) {
+                    const uint64_t key = bucket[i];
+                    const int b = bin(key);
+                    const int from = b > 0 ? start[b - 1] : 0, end = start[b];
+                    if (from >= kp) continue;
+                    int place = from;
+                    for (int e = from; e < end; ++e) place += bucket[e] < key;
+                    if (place < kp) put(place, key);
+                }
+            };
+            if (s_work <= kCrowdedUnit * (static_cast<uint32_t>(total) + 3072)) {   // (block-uniform)
+                rank_out([&](uint64_t key) { return kb.bin(static_cast<uint32_t>(key >> 32)); }, bh);
+            } else {
+                // bins between NT of the keys themselves (all distinct, as more than 313
+                // keys are here), in the histograms' space
+                uint64_t* const split = reinterpret_cast<uint64_t*>(bh);
+                uint64_t* const raw = split + NT;
+                int* const cnt = reinterpret_cast<int*>(raw + NT);
+                const uint64_t mine = gath[static_cast<uint32_t>(tid) * static_cast<uint32_t>(total) / NT];
+                raw[tid] = mine;
+                cnt[tid] = 0;
+                __syncthreads();
+                int at = 0;
+                for (int e = 0; e < NT; ++e) at += raw[e] < mine;
+                split[at] = mine;
+                __syncthreads();
+                auto bin = [&](uint64_t key) {
+                    int j = 0;   // the last splitter at or below the key, or the first
+#pragma unroll
+                    for (int step = NT / 2; step > 0; step >>= 1)
+                        if (split[j + step] <= key) j += step;
+                    return j;
+                };
+                for (int i = tid; i < total; i += NT) atomicAdd(&cnt[bin(gath[i])], 1);
+                __syncthreads();
+                const int n_bin = cnt[tid];
+                int incl = n_bin;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int t = __shfl_up_sync(kFull, incl, o);
+                    if (lane >= o) incl += t;
+                }
+                if (lane == 31) s_red[warp] = static_cast<uint32_t>(incl);
+                __syncthreads();
+                for (int w = 0; w < warp; ++w) incl += static_cast<int>(s_red[w]);
+                cnt[tid] = incl - n_bin;
+                __syncthreads();
+                rank_out(bin, cnt);
             }
         }
         for (int i = kept + tid; i < kp; i += NT) {

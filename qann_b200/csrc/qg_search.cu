@@ -475,7 +475,7 @@ __global__ void k_query_tables(IvfView v, const float* __restrict__ q, float* __
 // ---------------------------------------------------------------------------
 // Merge: the k' smallest key64 of a query's chunk outputs (each a list of k',
 // ~0 for empty entries), sorted, by one block per query: block_rank_smallest
-// over all of them. Where its last interval holds too many, a block-wide radix
+// over all of them. Where its intervals hold too many, a block-wide radix
 // select of the k'-th smallest valid key, 8 bits a pass from the top and stopping
 // once every key of the chosen bin is kept, then the survivors compacted and
 // sorted (what every merge did before: 12.8 us for one query of 800 keys, 6.3 now).
@@ -512,7 +512,7 @@ __global__ void __launch_bounds__(1024) k_merge(const uint64_t* __restrict__ in_
             }
             return;
         }
-        __syncthreads();   // (many keys in the last interval: the radix select below)
+        __syncthreads();   // (many keys in an interval: the radix select below)
     }
     if (threadIdx.x == 0) {
         s_valid = 0;
@@ -712,7 +712,7 @@ __global__ void __launch_bounds__(1024) k_refine_select(const float* __restrict_
                                                         const int64_t* __restrict__ labels, bool cosine,
                                                         int64_t* __restrict__ out_ids, float* __restrict__ out_d,
                                                         const int* __restrict__ k_q) {
-    extern __shared__ uint64_t rkey[];   // kp keys and kp indices: every candidate may be listed
+    extern __shared__ uint64_t rkey[];   // kp keys and kp indices: every candidate may be listed; or kp's power of two of keys
     __shared__ RankScratch rs;
     const int qi = blockIdx.x;
     const int kq = k_q ? min(k_q[qi], k) : k;
@@ -727,11 +727,23 @@ __global__ void __launch_bounds__(1024) k_refine_select(const float* __restrict_
         out_ids[o] = labels ? labels[slot] : static_cast<int64_t>(slot);
         out_d[o] = cosine ? __fmul_rn(d, 0.5f) : d;
     };
-    const int got = block_rank_smallest(kp, kq, [&](int i) { return src[i]; }, rkey,
-                                        reinterpret_cast<uint32_t*>(rkey + kp), kp, rs, put);
-    for (int i = got + threadIdx.x; i < k; i += blockDim.x) {
+    auto empty = [&](int i) {
         out_ids[static_cast<size_t>(qi) * k + i] = -1;
         out_d[static_cast<size_t>(qi) * k + i] = __int_as_float(0x7f800000);
+    };
+    const int got = block_rank_smallest(kp, kq, [&](int i) { return src[i]; }, rkey,
+                                        reinterpret_cast<uint32_t*>(rkey + kp), kp, rs, put);
+    if (got >= 0) {   // (block-uniform)
+        for (int i = got + threadIdx.x; i < k; i += blockDim.x) empty(i);
+        return;
+    }
+    // keys crowd, as equal distances do: sorted
+    const int kpow = next_pow2(max(2, kp));
+    for (int i = threadIdx.x; i < kpow; i += blockDim.x) rkey[i] = i < kp ? src[i] : ~0ull;
+    bitonic_sort_keys(rkey, kpow);
+    for (int i = threadIdx.x; i < k; i += blockDim.x) {
+        if (i < min(kq, kp) && rkey[i] != ~0ull) put(i, rkey[i], 0u);
+        else empty(i);
     }
 }
 
@@ -844,8 +856,9 @@ void refine_candidates(const float* q, int nq, int dim, const float* rows, const
                        int kp, int k, bool ip, const int64_t* labels, bool cosine, int64_t* out_ids, float* out_d,
                        cudaStream_t st, const int* kp_q, const int* k_q) {
     if (nq == 0 || k == 0) return;
-    const size_t ssm = static_cast<size_t>(kp) * 12;
-    require(static_cast<size_t>(std::max(2, next_pow2(kp))) * 8 <= 200 * 1024, "re-rank shared memory exceeds the B200 limit for this k * k_factor", kUnsupported);
+    const size_t sorted = static_cast<size_t>(std::max(2, next_pow2(kp))) * 8;
+    const size_t ssm = std::max(static_cast<size_t>(kp) * 12, sorted);
+    require(sorted <= 200 * 1024, "re-rank shared memory exceeds the B200 limit for this k * k_factor", kUnsupported);
     const size_t total = static_cast<size_t>(nq) * kp;
     DevBuf<uint64_t> scored(total, st);
     KernelTimer kt("refine", st);

@@ -1,0 +1,100 @@
+"""Ranks among keys that crowd: many equal distances, a query that is a row of the
+index, scores of both signs, rows a thousand times the others' length. The scan's
+candidates against the oracle's scan of the saved lists, and the time against
+that of rows with nothing in common."""
+import time
+
+import numpy as np
+import pytest
+
+import qann_b200 as qb
+from oracle import qann_file
+
+pytestmark = pytest.mark.gpu
+
+KINDS = ["spread", "own", "duplicates", "equal", "outliers"]
+
+
+def data(kind, n, d):
+    rng = np.random.default_rng(8)
+    x = rng.normal(size=(n, d)).astype(np.float32)
+    q = rng.normal(size=(64, d)).astype(np.float32)
+    if kind == "own":
+        q = x[:: n // 64][:64].copy()
+    elif kind == "duplicates":
+        x = x[rng.integers(0, 40, n)]
+    elif kind == "equal":
+        x[200:] = x[0]
+    elif kind == "outliers":
+        x[::50] *= 1e3
+    return x, q
+
+
+def ivf_of(x, metric, nlist=100, nprobe=16):
+    ivf = qb.IVFIndex(x.shape[1], nlist, nprobe, metric=qb.Metric(metric))
+    ivf.enable_pq(x.shape[1] // 2, fast_scan=True)
+    ivf.train(x, max_iters=2, seed=1, clustering=qb.Clustering.Lloyd)
+    return ivf
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("metric", [0, 2])
+@pytest.mark.parametrize("k", [1, 33, 257, 1000])
+def test_scan_against_oracle(kind, metric, k, tmp_path):
+    x, q = data(kind, 20_000, 32)
+    ivf = ivf_of(x, metric)
+    ivf.add(x)
+    ivf.save(tmp_path / "a.qann")
+    info = qann_file.read(tmp_path / "a.qann")["ivf"]
+    arr = qann_file.arrays(info)
+    alone = ivf.batch_query(q[:3], k)
+    # together: enough queries for a unit each
+    ids, dist = ivf.batch_query(np.concatenate([q] * 10), k)
+    for i in range(3):
+        probes, pterm = qann_file.coarse(info, q[i], info["nprobe"])
+        want_d, want_s = arr.query(q[i], probes, pterm, k)
+        order = np.lexsort((want_s, want_d))
+        want_ids = np.full(k, -1, np.int64)
+        want_ids[: len(order)] = want_s[order]
+        np.testing.assert_array_equal(ids[i], want_ids)
+        np.testing.assert_array_equal(alone[0][i], want_ids)
+        assert dist[i, : len(order)].tobytes() == want_d[order].tobytes()
+        assert alone[1][i, : len(order)].tobytes() == want_d[order].tobytes()
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("metric", [0, 2])
+@pytest.mark.parametrize("k,k_factor", [(10, 7), (100, 10), (250, 12)])
+def test_refine_is_the_exact_order(kind, metric, k, k_factor):
+    """Every list probed and every row a candidate: the exact search's answer."""
+    x, q = data(kind, k * k_factor if k > 10 else 2500, 24)
+    n = len(x)
+    idx = qb.RefineIndex(ivf_of(x, metric, nprobe=100), -(-n // k))
+    idx.add(x)
+    flat = qb.FlatIndex(24, metric=qb.Metric(metric))
+    flat.add(x)
+    got, want = idx.batch_query(q, k), flat.batch_query(q, k)
+    np.testing.assert_array_equal(got[0], want[0])
+    assert got[1].tobytes() == want[1].tobytes()
+
+
+@pytest.mark.parametrize("refined", [False, True])
+def test_crowding_costs_no_more(refined):
+    """1,000 candidates each of 200 queries: at most 3 times what spread rows take.
+    (Ranking each key against all that share its bin took 5 times and more.)"""
+    took = {}
+    for kind in KINDS:
+        x, q = data(kind, 100_000, 32)
+        idx = ivf_of(x, 0)
+        if refined:
+            idx = qb.RefineIndex(idx, 10)
+        idx.add(x)
+        qs, k = np.concatenate([q] * 4)[:200], 100 if refined else 1000
+        times = []
+        for _ in range(9):
+            t = time.perf_counter()
+            idx.batch_query(qs, k)
+            times.append(time.perf_counter() - t)
+        took[kind] = sorted(times)[4]
+    for kind in KINDS:
+        assert took[kind] < 3 * took["spread"], took
