@@ -194,6 +194,28 @@ __global__ void k_put_back(const uint64_t* __restrict__ key, const uint32_t* __r
     out_slot[o] = slot[t];
 }
 
+static void put_back(const uint64_t* key, const uint32_t* slot, const uint32_t* at, size_t m, size_t k,
+                     uint64_t* out_key, uint32_t* out_slot, cudaStream_t st) {
+    k_put_back<<<static_cast<unsigned>(ceil_div(m * k, 256)), 256, 0, st>>>(key, slot, at, m, static_cast<int>(k), out_key,
+                                                                            out_slot);
+    QG_LAUNCH_CHECK();
+}
+
+// at[i] = src[at[i]]
+__global__ void k_pick_u32(const uint32_t* __restrict__ src, size_t n, uint32_t* __restrict__ at) {
+    const size_t t = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (t < n) at[t] = src[at[t]];
+}
+
+// Whether m queries whose candidate lists overflowed are swept (tile_topk) before
+// the exact tiles, or always in mode 2: from 2e8 multiply-adds of those, which come in tiles
+// of 16 queries. Rows of 96 dims, each nearer than the ones before it, k = 10, batch_query
+// exact / swept: one query over 65,000 (1e8) 295 / 313 and 130,000 rows (2e8) 503 / 340 us;
+// 64 queries over 30,000 (1.8e8) 279 / 375 and 65,000 (4e8) 454 / 366 us.
+static bool sweeps_pay(size_t m, size_t n, int dim) {
+    return g_tensor_filter.load() == 2 || static_cast<double>(std::max<size_t>(m, 16)) * double(n) * dim >= 2e8;
+}
+
 void flat_candidates(const float* q_dev, size_t nq, const float* rows_dev, size_t n, int dim, bool ip, size_t k,
                      const uint64_t* allow_dev, const uint64_t* deny_dev, uint64_t* out_key, uint32_t* out_slot,
                      cudaStream_t st, bool allow_mm, const TileBase* pre) {
@@ -210,18 +232,45 @@ void flat_candidates(const float* q_dev, size_t nq, const float* rows_dev, size_
     TileQueries qs;
     tile_prepare_queries(q_dev, nq, dim, qs, st);
     DevBuf<uint32_t> redo;
-    const size_t m = tile_topk(q_dev, qs, rows_dev, *base, ip, k, allow_dev, deny_dev, out_key, out_slot, redo, st);
+    const TileRedo r = tile_topk(q_dev, qs, rows_dev, *base, ip, k, allow_dev, deny_dev, out_key, out_slot, redo, false, st);
+    // the queries it could not settle: some by sweeps with falling thresholds, where
+    // that pays, the others and what is left of those by the exact FP32 tiles over every row
+    DevBuf<uint32_t> exact(r.sweep + r.exact, st);
+    size_t m = 0;
+    auto list = [&](const uint32_t* at, size_t n_at) {
+        if (n_at)
+            QG_CUDA(cudaMemcpyAsync(exact.get() + m, at, n_at * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st));
+        m += n_at;
+    };
+    list(redo.get() + nq - r.exact, r.exact);
+    if (r.sweep > 0 && !sweeps_pay(r.sweep, n, dim)) {
+        list(redo.get(), r.sweep);
+    } else if (r.sweep > 0) {
+        DevBuf<float> qr(r.sweep * dim, st);
+        gather_rows(q_dev, redo.get(), r.sweep, dim, qr.get(), st);
+        TileQueries qrs;
+        tile_prepare_queries(qr.get(), r.sweep, dim, qrs, st);
+        DevBuf<uint64_t> sk(r.sweep * k, st);
+        DevBuf<uint32_t> ss(r.sweep * k, st), again;
+        const TileRedo r2 = tile_topk(qr.get(), qrs, rows_dev, *base, ip, k, allow_dev, deny_dev, sk.get(), ss.get(),
+                                      again, true, st);
+        // (those left are put there again)
+        put_back(sk.get(), ss.get(), redo.get(), r.sweep, k, out_key, out_slot, st);
+        if (r2.exact) {
+            uint32_t* const at = again.get() + r.sweep - r2.exact;
+            k_pick_u32<<<static_cast<unsigned>(ceil_div(r2.exact, 256)), 256, 0, st>>>(redo.get(), r2.exact, at);
+            QG_LAUNCH_CHECK();
+            list(at, r2.exact);
+        }
+    }
     count_tensor_filter(static_cast<int64_t>(nq), static_cast<int64_t>(m));
     if (m == 0) return;
-    // queries it could not settle: the exact FP32 tiles over every row
     DevBuf<float> qr(m * dim, st);
-    gather_rows(q_dev, redo.get(), m, dim, qr.get(), st);
+    gather_rows(q_dev, exact.get(), m, dim, qr.get(), st);
     DevBuf<uint64_t> sk(m * k, st);
     DevBuf<uint32_t> ss(m * k, st);
     flat_candidates_fp32(qr.get(), m, rows_dev, n, dim, ip, k, allow_dev, deny_dev, sk.get(), ss.get(), st);
-    k_put_back<<<static_cast<unsigned>(ceil_div(m * k, 256)), 256, 0, st>>>(sk.get(), ss.get(), redo.get(), m,
-                                                                            static_cast<int>(k), out_key, out_slot);
-    QG_LAUNCH_CHECK();
+    put_back(sk.get(), ss.get(), exact.get(), m, k, out_key, out_slot, st);
 }
 
 // Flat results in (score, slot) order with ids and the exact score, which its

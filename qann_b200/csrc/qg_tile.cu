@@ -53,6 +53,10 @@ constexpr int kSlots = 7;       // candidates a lane holds before it appends the
 constexpr uint32_t kTmemCols = 512;   // two accumulators of two halves
 constexpr float kOpen = 3.402823466e+38f;   // threshold of a query that has none yet
 constexpr int kNearestCap = 256;            // candidates of a query in nearest mode
+constexpr size_t kMaxChunkRows = size_t{1} << 22;   // base rows a launch
+constexpr int kSweeps = 6;      // each leaves about cap / k times fewer rows that pass
+constexpr int kMaxCap = 8192;   // candidates of a query in filter mode at most; lists are counted up to it
+constexpr uint32_t kGivenUp = 0x80000000u;   // the count of a list that a sweep would not settle either
 
 // What the epilogue does with an accumulator.
 enum TileMode {
@@ -416,6 +420,8 @@ __global__ void __launch_bounds__(tile_threads<EPI>(), 1)
             for (int i = 0; i < cnt; ++i)
                 if (pos + i < static_cast<uint32_t>(a.cap)) to[i] = slot[i * EPI * 32];
             sp = smem_u32(slot);
+            // (no list holds more: the lane stops)
+            if (MODE == kFilter && pos + cnt > static_cast<uint32_t>(kMaxCap)) thr = none;
         };
         auto leave = [&] {   // done with the query tile
             if (MODE == kStore) return;
@@ -874,18 +880,29 @@ __device__ __forceinline__ float upper_bound(float lb, float x2, float c2, float
     return tile_extreme(x2) ? __builtin_huge_valf() : __fadd_ru(lb, __fadd_ru(__fmul_ru(c2, x2), qslack));
 }
 
+// The key of a threshold that no row passes, extreme ones included.
+constexpr uint32_t kClosedKey = 0xFFFFFFFFu;   // (a NaN)
+
 // One block per query over the stored products of the first ncols rows: its
-// threshold and the rows at or below it. lbs, ub: ncols floats of shared memory each.
+// threshold and the rows at or below it, or for a sweep the threshold alone. lbs, ub:
+// ncols floats of shared memory each.
 __global__ void __launch_bounds__(256) k_tile_seed(const float* __restrict__ acc, size_t ld, int ncols,
                                                    const float* __restrict__ xterm, const float* __restrict__ sq,
                                                    float c2, const float* __restrict__ qmul,
-                                                   const float* __restrict__ qslack, int k, int cap,
+                                                   const float* __restrict__ qslack, int k, int cap, bool sweep,
                                                    uint32_t* __restrict__ thr_key, uint32_t* __restrict__ count,
                                                    uint2* __restrict__ cand) {
     extern __shared__ __align__(16) uint8_t sm_raw[];
     __shared__ CutScratch s;
     const int qi = blockIdx.x;
-    if (count[qi] > static_cast<uint32_t>(cap)) return;   // an extreme query
+    if (count[qi] > static_cast<uint32_t>(cap)) {   // an extreme query
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            count[qi] = kGivenUp;
+            thr_key[qi] = kClosedKey;
+        }
+        return;
+    }
     float* lbs = reinterpret_cast<float*>(sm_raw);
     float* ub = lbs + ncols;
     const float* row = acc + static_cast<size_t>(qi) * ld;
@@ -898,6 +915,10 @@ __global__ void __launch_bounds__(256) k_tile_seed(const float* __restrict__ acc
     }
     __syncthreads();
     const float T = cut_threshold(ub, ncols, k, s);
+    if (sweep) {
+        if (threadIdx.x == 0) thr_key[qi] = float_key(T);
+        return;
+    }
     const int lane = threadIdx.x & 31;
     for (int j0 = 0; j0 < ncols; j0 += blockDim.x) {   // (trip count block-uniform)
         const int j = j0 + threadIdx.x;
@@ -913,7 +934,7 @@ __global__ void __launch_bounds__(256) k_tile_seed(const float* __restrict__ acc
     __syncthreads();
     if (threadIdx.x == 0) {
         count[qi] = static_cast<uint32_t>(s.count);
-        thr_key[qi] = float_key(s.count > cap ? -kOpen : T);   // (an overflowed list takes no more)
+        thr_key[qi] = s.count > cap ? kClosedKey : float_key(T);   // (an overflowed list takes no more)
     }
 }
 
@@ -944,23 +965,51 @@ __device__ __forceinline__ int cut_list(uint2* list, float* ub, int n, int k, co
     return kept;
 }
 
+// Whether a sweep would settle a list that overflowed in the chunk from row `from`
+// on, under the threshold of key `was` and with cnt rows counted: its list holds what
+// passes (`ahead` times cnt by the last row), or the entries taken from the chunk give a
+// lower threshold (not so where distances tie), or too few were taken to tell. By one
+// block; list, ub: cap entries of shared memory each. (Not inlined: it is rare, and
+// its registers cost the kernels that call it 3 to 8 % of their callers' time.)
+__device__ __noinline__ bool worth_a_sweep(const uint2* mine, uint32_t cnt, float ahead, uint32_t from, uint32_t was,
+                                           uint2* list, float* ub, int cap, int k, const float* __restrict__ sq, float c2,
+                                           float qs, CutScratch& s) {
+    if (static_cast<float>(cnt) * ahead <= static_cast<float>(kMaxCap)) return true;   // (block-uniform)
+    int fresh = 0;
+    for (int i0 = 0; i0 < cap; i0 += blockDim.x) {   // (whole rounds: cap is a power of two)
+        const uint2 e = mine[i0 + threadIdx.x];
+        list[i0 + threadIdx.x] = e;
+        fresh += __syncthreads_count(e.y >= from);
+    }
+    if (fresh < k) return true;
+    float T;
+    cut_list(list, ub, cap, k, sq, c2, qs, s, T);
+    return float_key(T) < was;
+}
+
 // After a chunk, one block per query: the list cut, its threshold lowered.
-__global__ void __launch_bounds__(128) k_tile_cut(const float* __restrict__ sq, float c2,
-                                                  const float* __restrict__ qslack, int k, int cap,
+__global__ void __launch_bounds__(128, 16) k_tile_cut(const float* __restrict__ sq, float c2,
+                                                  const float* __restrict__ qslack, int k, int cap, float ahead, uint32_t from,
                                                   uint32_t* __restrict__ thr_key, uint32_t* __restrict__ count,
                                                   uint2* __restrict__ cand) {
     extern __shared__ __align__(16) uint8_t sm_raw[];
     __shared__ CutScratch s;
     const int qi = blockIdx.x;
-    const uint32_t cnt = count[qi];
-    if (cnt > static_cast<uint32_t>(cap)) {   // overflowed: it takes no more
-        if (threadIdx.x == 0) thr_key[qi] = float_key(-kOpen);
-        return;
-    }
+    const uint32_t cnt = count[qi], was = thr_key[qi];
+    if (was == kClosedKey) return;   // overflowed before
     const int n = static_cast<int>(cnt);
     uint2* list = reinterpret_cast<uint2*>(sm_raw);
     float* ub = reinterpret_cast<float*>(list + cap);
     uint2* mine = cand + static_cast<size_t>(qi) * cap;
+    if (cnt > static_cast<uint32_t>(cap)) {   // overflowed: it takes no more
+        const bool sweep = worth_a_sweep(mine, cnt, ahead, from, was, list, ub, cap, k, sq, c2, qslack[qi], s);
+        __syncthreads();   // (count and threshold are read)
+        if (threadIdx.x == 0) {
+            thr_key[qi] = kClosedKey;
+            if (!sweep) count[qi] = kGivenUp;
+        }
+        return;
+    }
     for (int i = threadIdx.x; i < n; i += blockDim.x) list[i] = mine[i];
     __syncthreads();
     float T;
@@ -972,30 +1021,71 @@ __global__ void __launch_bounds__(128) k_tile_cut(const float* __restrict__ sq, 
     }
 }
 
+// After a sweep over every row, one block per query. A list that held what
+// passed is cut and closed. In one that overflowed, the entries it did take are
+// rows like any others, so the k-th smallest of their upper bounds is a threshold: with
+// that one, where it is lower, the list is opened again (*open counts those);
+// otherwise, or after the last sweep, it is given up.
+__global__ void __launch_bounds__(128) k_tile_sweep_cut(const float* __restrict__ sq, float c2,
+                                                        const float* __restrict__ qslack, int k, int cap, bool last,
+                                                        uint32_t* __restrict__ thr_key, uint32_t* __restrict__ count,
+                                                        uint2* __restrict__ cand, uint32_t* __restrict__ open) {
+    extern __shared__ __align__(16) uint8_t sm_raw[];
+    __shared__ CutScratch s;
+    const int qi = blockIdx.x;
+    const uint32_t was = thr_key[qi], cnt = count[qi];
+    if (was == kClosedKey) return;
+    const bool held = cnt <= static_cast<uint32_t>(cap);
+    const int n = held ? static_cast<int>(cnt) : cap;
+    uint2* list = reinterpret_cast<uint2*>(sm_raw);
+    float* ub = reinterpret_cast<float*>(list + cap);
+    uint2* mine = cand + static_cast<size_t>(qi) * cap;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) list[i] = mine[i];
+    __syncthreads();
+    float T;
+    const int kept = cut_list(list, ub, n, k, sq, c2, qslack[qi], s, T);
+    const bool again = !held && !last && float_key(T) < was;
+    if (held)
+        for (int i = threadIdx.x; i < kept; i += blockDim.x) mine[i] = list[i];
+    if (threadIdx.x == 0) {
+        thr_key[qi] = again ? float_key(T) : kClosedKey;
+        count[qi] = held ? static_cast<uint32_t>(kept) : again ? 0u : kGivenUp;
+        if (again) atomicAdd(open, 1u);
+    }
+}
+
 // At the end, one block per query: the list cut, the rows left scored exactly
 // (a lane group of kG per row: 4 for an even dim at 8-byte alignment, else 8), and
 // the k smallest by (score, row) written in order. Up to 512 keys are ranked
 // over per-warp register-sorted runs (one barrier), more sorted by the block.
 template <int kG>
-__global__ void __launch_bounds__(256) k_tile_finish(const float* __restrict__ q, int d, const float* __restrict__ rows,
+__global__ void __launch_bounds__(256, 6) k_tile_finish(const float* __restrict__ q, int d, const float* __restrict__ rows,
                                                      bool ip, const float* __restrict__ sq, float c2,
                                                      const float* __restrict__ qslack, int k, int cap,
                                                      const uint32_t* __restrict__ count,
+                                                     const uint32_t* __restrict__ thr_key, uint32_t from,
                                                      const uint2* __restrict__ cand, uint32_t first,
                                                      uint64_t* __restrict__ out_key, uint32_t* __restrict__ out_slot,
-                                                     uint32_t* __restrict__ redo, uint32_t* __restrict__ nredo) {
+                                                     uint32_t* __restrict__ redo, uint32_t redo_end,
+                                                     uint32_t* __restrict__ nredo) {
     extern __shared__ __align__(16) uint8_t sm_raw[];
     __shared__ CutScratch s;
     const int qi = blockIdx.x;
     const uint32_t cnt = count[qi];
-    if (cnt > static_cast<uint32_t>(cap)) {
-        if (threadIdx.x == 0) redo[atomicAdd(nredo, 1u)] = first + qi;
-        return;
-    }
     const int n = static_cast<int>(cnt);
     uint2* list = reinterpret_cast<uint2*>(sm_raw);
     float* ub = reinterpret_cast<float*>(list + cap);
     const uint2* mine = cand + static_cast<size_t>(qi) * cap;
+    if (cnt > static_cast<uint32_t>(cap)) {   // to the front of redo[] to be swept, to its end where that would not help
+        const uint32_t was = thr_key[qi];
+        const bool sweep = cnt != kGivenUp && (was == kClosedKey || worth_a_sweep(mine, cnt, 1.0f, from, was, list, ub, cap,
+                                                                                  k, sq, c2, qslack[qi], s));
+        if (threadIdx.x == 0) {
+            if (sweep) redo[atomicAdd(nredo, 1u)] = first + qi;
+            else redo[redo_end - 1 - atomicAdd(nredo + 1, 1u)] = first + qi;
+        }
+        return;
+    }
     for (int i = threadIdx.x; i < n; i += blockDim.x) list[i] = mine[i];
     __syncthreads();
     float T;
@@ -1314,13 +1404,17 @@ size_t tile_nearest(const float* q, const TileQueries& qs, const float* base_row
     return h[0];
 }
 
-// The exact k nearest rows of each query (see "the k nearest" above).
-size_t tile_topk(const float* q, const TileQueries& qs, const float* base_rows, const TileBase& base, bool ip, size_t k,
+// The exact k nearest rows of each query (see "the k nearest" above). sweep: every
+// row under one threshold, again with a lower one while a list overflows, for
+// queries whose lists overflowed when chunks of growing size were taken: rows stored in
+// an order (by cluster, by time) bring what is near all at once, and the threshold
+// of the rows before them lets all of it pass.
+TileRedo tile_topk(const float* q, const TileQueries& qs, const float* base_rows, const TileBase& base, bool ip, size_t k,
                  const uint64_t* allow, const uint64_t* deny, uint64_t* out_key, uint32_t* out_slot,
-                 DevBuf<uint32_t>& redo, cudaStream_t st) {
+                 DevBuf<uint32_t>& redo, bool sweep, cudaStream_t st) {
     const size_t nq = qs.n, n = base.n;
     const int d = base.dim;
-    if (nq == 0 || k == 0) return 0;
+    if (nq == 0 || k == 0) return {};
     require(n >= 1 && n < (size_t{1} << 31) && nq < (size_t{1} << 31), "too many rows for the tensor-core path",
             kUnsupported);
     require(k <= kTileMaxK, "k too large for the tensor-core path", kUnsupported);
@@ -1332,7 +1426,7 @@ size_t tile_topk(const float* q, const TileQueries& qs, const float* base_rows, 
     QG_LAUNCH_CHECK();
     // the candidate list: about 8 times what is wanted, so that a chunk of rows
     // far from their average order does not overflow it
-    const int cap = std::clamp(next_pow2(static_cast<int>(8 * k)), 2048, 8192);
+    const int cap = sweep ? kMaxCap : std::clamp(next_pow2(static_cast<int>(8 * k)), 2048, kMaxCap);
     // the seed: enough rows that the first chunk's threshold lets few pass
     const size_t seed = std::min<size_t>(n, std::clamp<size_t>(ceil_div(16 * k, BN) * BN, 2048, 8192));
     const size_t ld = ceil_div(seed, 4) * 4;
@@ -1341,9 +1435,10 @@ size_t tile_topk(const float* q, const TileQueries& qs, const float* base_rows, 
     DevBuf<float> acc(QB * ld, st), qmul(QB, st), qslack(QB, st);
     DevBuf<uint32_t> thr(QB, st), count(QB, st);
     DevBuf<uint2> cand(QB * cap, st);
-    redo.alloc(nq + 2, st);   // the list, its length, and the error flag
+    // the lists from both ends, their lengths, the error flag, and a sweep's count of lists opened again
+    redo.alloc(nq + 4, st);
     uint32_t* const nredo = redo.get() + nq;
-    QG_CUDA(cudaMemsetAsync(nredo, 0, 2 * sizeof(uint32_t), st));
+    QG_CUDA(cudaMemsetAsync(nredo, 0, 3 * sizeof(uint32_t), st));
     TileArgs a{};
     a.kblocks = (base.dpad + KA - 1) / KA;
     a.ksteps = (d + 15) / 16;
@@ -1355,13 +1450,14 @@ size_t tile_topk(const float* q, const TileQueries& qs, const float* base_rows, 
     a.cand_count = count.get();
     a.cand = cand.get();
     a.cap = cap;
-    a.err = reinterpret_cast<int*>(nredo + 1);
+    a.err = reinterpret_cast<int*>(nredo + 2);
     a.store = acc.get();
     a.ld = ld;
     const CUtensorMap tmB = make_map(base.f16.get(), n, base.dpad, BN);
     const size_t seed_smem = seed * 8, cut_smem = static_cast<size_t>(cap) * 12;
     allow_large_smem<k_tile_seed>();
     allow_large_smem<k_tile_cut>();
+    allow_large_smem<k_tile_sweep_cut>();
     allow_large_smem<k_tile_finish<4>>();
     allow_large_smem<k_tile_finish<8>>();
     const bool g4 = (d & 1) == 0 && (reinterpret_cast<uintptr_t>(q) & 7) == 0 &&
@@ -1388,11 +1484,28 @@ size_t tile_topk(const float* q, const TileQueries& qs, const float* base_rows, 
             launch_tile<kStore>(tmA, tmB, a, st, /*may_tune=*/false, [] {}, [] {});
         }
         k_tile_seed<<<nb, 256, seed_smem, st>>>(acc.get(), ld, static_cast<int>(seed), xterm.get(), base.sq.get(),
-                                                bound.c2, qmul.get(), qslack.get(), static_cast<int>(k), cap, thr.get(),
-                                                count.get(), cand.get());
+                                                bound.c2, qmul.get(), qslack.get(), static_cast<int>(k), cap, sweep,
+                                                thr.get(), count.get(), cand.get());
         QG_LAUNCH_CHECK();
-        for (size_t n0 = seed; n0 < n;) {
-            const size_t n1 = std::min(n, std::min(n0 * growth, n0 + (size_t{1} << 22)));
+        for (int left = kSweeps; sweep && left > 0; --left) {
+            for (size_t n0 = 0; n0 < n; n0 += kMaxChunkRows) {
+                a.n0 = static_cast<int>(n0);
+                a.ntiles = static_cast<int>(ceil_div(std::min(n - n0, kMaxChunkRows), BN));
+                a.group_n = 16;
+                KernelTimer kt("mm_filter", st);
+                launch_tile<kFilter>(tmA, tmB, a, st, /*may_tune=*/false, [] {}, [] {});
+            }
+            uint32_t open = 0;
+            QG_CUDA(cudaMemsetAsync(nredo + 3, 0, sizeof(uint32_t), st));
+            k_tile_sweep_cut<<<nb, 128, cut_smem, st>>>(base.sq.get(), bound.c2, qslack.get(), static_cast<int>(k), cap,
+                                                        left == 1, thr.get(), count.get(), cand.get(), nredo + 3);
+            QG_LAUNCH_CHECK();
+            QG_CUDA(cudaMemcpyAsync(&open, nredo + 3, sizeof(open), cudaMemcpyDeviceToHost, st));
+            QG_CUDA(cudaStreamSynchronize(st));
+            if (open == 0) break;
+        }
+        for (size_t n0 = sweep ? n : seed; n0 < n;) {
+            const size_t n1 = std::min(n, std::min(n0 * growth, n0 + kMaxChunkRows));
             a.n0 = static_cast<int>(n0);
             a.ntiles = static_cast<int>(ceil_div(n1 - n0, BN));
             a.group_n = 16;
@@ -1411,24 +1524,25 @@ size_t tile_topk(const float* q, const TileQueries& qs, const float* base_rows, 
             n0 = n1;
             if (n0 == n) break;
             k_tile_cut<<<nb, 128, cut_smem, st>>>(base.sq.get(), bound.c2, qslack.get(), static_cast<int>(k), cap,
+                                                  static_cast<float>(n) / static_cast<float>(n0), static_cast<uint32_t>(a.n0),
                                                   thr.get(), count.get(), cand.get());
             QG_LAUNCH_CHECK();
         }
         auto finish = [&](auto kernel) {
             kernel<<<nb, 256, cut_smem, st>>>(q + q0 * d, d, base_rows, ip, base.sq.get(), bound.c2, qslack.get(),
-                                              static_cast<int>(k), cap, count.get(), cand.get(),
-                                              static_cast<uint32_t>(q0), out_key + q0 * k, out_slot + q0 * k, redo.get(),
-                                              nredo);
+                                              static_cast<int>(k), cap, count.get(), thr.get(), static_cast<uint32_t>(a.n0),
+                                              cand.get(), static_cast<uint32_t>(q0), out_key + q0 * k, out_slot + q0 * k, redo.get(),
+                                              static_cast<uint32_t>(nq), nredo);
             QG_LAUNCH_CHECK();
         };
         if (g4) finish(k_tile_finish<4>);
         else finish(k_tile_finish<8>);
     }
-    uint32_t h[2] = {0, 0};
+    uint32_t h[3] = {0, 0, 0};
     QG_CUDA(cudaMemcpyAsync(h, nredo, sizeof(h), cudaMemcpyDeviceToHost, st));
     QG_CUDA(cudaStreamSynchronize(st));
-    require(h[1] == 0, "tensor-core filter: a pipeline wait timed out", kRuntimeError);
-    return h[0];
+    require(h[2] == 0, "tensor-core filter: a pipeline wait timed out", kRuntimeError);
+    return {h[0], h[1]};
 }
 
 } // namespace qg

@@ -47,11 +47,16 @@ size_t tile_nearest(const float* q, const TileQueries& qs, const float* base_row
 // The exact k nearest base rows of each query by (score, row), -0 == +0:
 // out_key[nq][k] (key_eq0(score) << 32 | row, ~0 when there are fewer) and
 // out_slot[nq][k], sorted. ip: the score is -(q . x), else squared L2. allow /
-// deny: bitmaps over the rows, or null. redo as above. k at most kTileMaxK.
+// deny: bitmaps over the rows, or null. k at most kTileMaxK. Queries not settled are
+// listed in redo[0 .. nq): from its start those that the sweep form settles as a rule
+// (rows stored in an order), at its end those that want the exact path.
 inline constexpr size_t kTileMaxK = 1024;
-size_t tile_topk(const float* q, const TileQueries& qs, const float* base_rows, const TileBase& base, bool ip, size_t k,
-                 const uint64_t* allow, const uint64_t* deny, uint64_t* out_key, uint32_t* out_slot,
-                 DevBuf<uint32_t>& redo, cudaStream_t st);
+struct TileRedo {
+    size_t sweep = 0, exact = 0;   // redo[0 .. sweep) and redo[nq - exact .. nq)
+};
+TileRedo tile_topk(const float* q, const TileQueries& qs, const float* base_rows, const TileBase& base, bool ip, size_t k,
+                   const uint64_t* allow, const uint64_t* deny, uint64_t* out_key, uint32_t* out_slot,
+                   DevBuf<uint32_t>& redo, bool sweep, cudaStream_t st);
 
 // The raw products of the queries with n base rows (f16 rows of dpad
 // elements), row after row of `store` (ld apart). *err is set if a pipeline
