@@ -34,6 +34,10 @@ struct TileBase {
 
 // Dimensions the engine takes.
 bool tile_supported(int dim);
+// The device memory of n prepared query rows.
+inline size_t tile_query_bytes(size_t n, int dim) {
+    return n * ((static_cast<size_t>(dim) + 7) / 8 * 8 * sizeof(uint16_t) + sizeof(float) + sizeof(int));
+}
 void tile_prepare_queries(const float* rows, size_t n, int dim, TileQueries& out, cudaStream_t st);
 void tile_prepare_base(const float* rows, size_t n, int dim, TileBase& out, cudaStream_t st);
 

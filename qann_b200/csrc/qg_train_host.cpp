@@ -125,6 +125,18 @@ void refill_empty_clusters(const float* x_dev, size_t n, int d, int k, int P, fl
 // ---------------------------------------------------------------------------
 // Lloyd
 // ---------------------------------------------------------------------------
+// Whether the points are prepared for the tensor cores once, not a block of rows
+// at a time in every iteration: up to 4 GB of them and a quarter of the free memory,
+// which is not asked for where the assignment's own lists (268 MB) are larger.
+static bool room_for_points(size_t n, int d) {
+    const size_t bytes = tile_query_bytes(n, d);
+    if (bytes > size_t{4} << 30) return false;
+    if (bytes <= size_t{256} << 20) return true;
+    size_t free_b = 0, total_b = 0;
+    QG_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    return bytes <= free_b / 4;
+}
+
 KMeansOut kmeans_lloyd(const float* x_dev, size_t n, int d, int k, size_t iters,
                        const std::vector<std::optional<uint32_t>>& seeds, bool spherical, int P, cudaStream_t st) {
     if (n < static_cast<size_t>(k)) throw Error(kInvalidArgument, "kmeans: need at least k points");
@@ -149,9 +161,8 @@ KMeansOut kmeans_lloyd(const float* x_dev, size_t n, int d, int k, size_t iters,
     out.assign.alloc(pn, st);
     DevBuf<uint32_t> order(pn, st), off(static_cast<size_t>(P) * (k + 1), st);
     DevBuf<int> empty(1, st);
-    // the points prepared once for the tensor cores (up to 4 GB), not per iteration
     TileQueries xq;
-    const bool keep = P == 1 && k > 64 && use_tensor_nearest(n, k, d) && n * static_cast<size_t>(d) * 2 <= size_t{4} << 30;
+    const bool keep = P == 1 && k > 64 && use_tensor_nearest(n, k, d) && room_for_points(n, d);
     if (keep) tile_prepare_queries(x_dev, n, d, xq, st);
     auto assign_all = [&]() {
         if (k <= 64) {
