@@ -267,7 +267,7 @@ const TileBase* tile_base(FlatObj& o) {
     std::lock_guard<std::mutex> g(o.dev_mu);
     DeviceRows& D = o.dev;
     if (!D.tile_made) {
-        const size_t bytes = n * static_cast<size_t>((dim + 7) & ~7) * 2;
+        const size_t bytes = tile_base_bytes(n, dim);
         if (bytes > kSmallCopy) {
             size_t free_b = 0, total_b = 0;
             QG_CUDA(cudaMemGetInfo(&free_b, &total_b));

@@ -216,10 +216,20 @@ static bool sweeps_pay(size_t m, size_t n, int dim) {
     return g_tensor_filter.load() == 2 || static_cast<double>(std::max<size_t>(m, 16)) * double(n) * dim >= 2e8;
 }
 
+// Whether a call that makes the rows' f16 copy for itself has the memory for it: up to
+// 256 MB, which the exact tiles take too, without asking, then half of what is free.
+static bool room_for_copy(size_t n, int dim) {
+    const size_t bytes = tile_base_bytes(n, dim);
+    if (bytes <= size_t{256} << 20) return true;
+    size_t free_b = 0, total_b = 0;
+    QG_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    return bytes <= free_b / 2;
+}
+
 void flat_candidates(const float* q_dev, size_t nq, const float* rows_dev, size_t n, int dim, bool ip, size_t k,
                      const uint64_t* allow_dev, const uint64_t* deny_dev, uint64_t* out_key, uint32_t* out_slot,
                      cudaStream_t st, bool allow_mm, const TileBase* pre) {
-    if (!allow_mm || !use_tensor_filter(nq, n, dim, k, pre != nullptr)) {
+    if (!allow_mm || !use_tensor_filter(nq, n, dim, k, pre != nullptr) || (!pre && !room_for_copy(n, dim))) {
         flat_candidates_fp32(q_dev, nq, rows_dev, n, dim, ip, k, allow_dev, deny_dev, out_key, out_slot, st);
         return;
     }

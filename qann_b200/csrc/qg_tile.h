@@ -39,6 +39,10 @@ inline size_t tile_query_bytes(size_t n, int dim) {
     return n * ((static_cast<size_t>(dim) + 7) / 8 * 8 * sizeof(uint16_t) + sizeof(float) + sizeof(int));
 }
 void tile_prepare_queries(const float* rows, size_t n, int dim, TileQueries& out, cudaStream_t st);
+// The device memory of n prepared base rows.
+inline size_t tile_base_bytes(size_t n, int dim) {
+    return n * ((static_cast<size_t>(dim) + 7) / 8 * 8 * sizeof(uint16_t) + sizeof(float));
+}
 void tile_prepare_base(const float* rows, size_t n, int dim, TileBase& out, cudaStream_t st);
 
 // Each query's nearest base row by squared L2 (the smallest score, the first
