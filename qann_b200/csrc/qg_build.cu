@@ -58,8 +58,9 @@ void assign_nearest(const float* x_dev, size_t n, const float* c_dev, size_t k, 
         TileBase cent;
         tile_prepare_base(c_dev, k, dim, cent, st);
         DevBuf<uint32_t> redo;
-        // rows prepared a block at a time unless the caller has them
-        const size_t step = xq ? n : size_t{1} << 20;
+        // rows prepared a block at a time unless the caller has them: 256 MB of them, at most 2^20
+        const size_t step =
+            xq ? n : std::min(size_t{1} << 20, std::max<size_t>(256, (size_t{256} << 20) / tile_query_bytes(1, dim)));
         for (size_t r0 = 0; r0 < n; r0 += step) {
             const size_t nr = std::min(step, n - r0);
             TileQueries own;
