@@ -192,11 +192,11 @@ __device__ __forceinline__ void recheck_query(const RecheckArgs& ra, int qi, int
         if (lower_in(arow[j], c2[j], cexp[j])) push(j);
     __syncthreads();
     const int cnt = s_count;
-    if (threadIdx.x == 0) atomicAdd(ra.ncand, static_cast<unsigned long long>(cnt));
     if (cnt > cap) {   // (cap >= nlist when it cannot be deferred)
         if (can_defer) defer();
         return;
     }
+    if (threadIdx.x == 0) atomicAdd(ra.ncand, static_cast<unsigned long long>(cnt));
     // exact scores, one candidate per 8-lane group; each list's score is kept
     // by list (over its upper bound, no longer needed) for the output
     float* score_of = reinterpret_cast<float*>(ub);
