@@ -186,7 +186,7 @@ def set_filter_options(autotune: bool | None = None, epilogue_warps: int | None 
     """The tensor-core filter's schedule (flat search, direct scans,
     nearest-centroid assignment, the coarse step). autotune: time its 8- and
     16-warp epilogues on the first large launch of each problem and keep the
-    faster (default on); off, the 8-warp one. epilogue_warps: 8 or 16 forces
+    faster (default on); off, the 16-warp one. epilogue_warps: 8 or 16 forces
     that epilogue on every launch, 0 leaves the pick to the autotuner. Results
     are identical under every setting."""
     if autotune is not None:

@@ -133,8 +133,10 @@ int tensor_filter() { return g_tensor_filter.load(); }
 // tiles / filter: 1 query over 20,000 rows of 32 / 128 dims (1e7 / 4.1e7) 119 /
 // 126 and 147 / 127 us; 64 queries over 5,000 x 128 (4.1e7) 124 / 131, over
 // 20,000 x 32 (4.1e7) 148 / 129; 512 queries over 5,000 x 32 (8.2e7) 224 / 147.
-// Without a kept copy the call makes one: from 1.5e8, and for few queries only
-// up to 256 MB of it.
+// Without a kept copy the call makes one, from 1.5e8 on: 1, 16 and 63 queries over
+// 100,000 x 96 (1.5e8 at 16 and less) 319 / 169, 396 / 181 and 569 / 196 us. For few queries
+// only up to 256 MB of it, the scratch of the exact tiles: not for time (over 2M x 128,
+// a copy of 488 MB, one query would take 7.9 / 0.95 ms), but for memory held per call.
 bool use_tensor_filter(size_t nq, size_t n, int dim, size_t k, bool kept) {
     const int mode = g_tensor_filter.load();
     const double work = static_cast<double>(std::max<size_t>(nq, 16)) * double(n) * dim;

@@ -24,7 +24,7 @@ struct SearchRequest {
     IoSpace io = IoSpace::Host;
     int nprobe = 0;                  // > 0: probes instead of the IVF index's nprobe
     bool capture = false;            // being captured into a CUDA graph: no host reads or waits
-    int* err_dev = nullptr;          // caller-owned error flags (3 ints), read by the caller, or null
+    int* err_dev = nullptr;          // caller-owned flags (kFlags ints, cleared by the search), read by the caller, or null
     // the filter's allowed slots in ascending order on the device (filter->count
     // of them), or null: RefineIndex direct scans then list them from the bitmap
     const uint32_t* filter_slots_dev = nullptr;

@@ -959,7 +959,9 @@ static std::vector<ScanShape> scan_shapes(int kp, int m_pad, int qtab_len, int p
     };
     if (force == -1 || force == 0) {
         // a large k' leaves two blocks per SM fewer than 8 warps each: one block of
-        // 8 goes first then (256 filtered queries, k' = 1,000: 562 -> 511 us)
+        // 8 goes first then (256 filtered queries, k' = 1,000: 562 -> 511 us), or of 4 where
+        // 8 do not fit either (256 queries over 500,000 x 128, k' = 1,500: 1,600 -> 1,040 us
+        // with 8 warps, k' = 2,000: 2,120 -> 1,930 with 4; 1,000 queries, k' = 2,000: 5.8 -> 4.7 ms)
         fits(kUnstaged, false, 110 * 1024, 3);
         // (where nothing fits, the list stays empty and the caller refuses the search)
         if ((out.empty() || out.front().nw < 8) && fits(kUnstaged, false, 226 * 1024, 1))

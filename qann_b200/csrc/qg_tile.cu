@@ -1465,7 +1465,10 @@ TileRedo tile_topk(const float* q, const TileQueries& qs, const float* base_rows
     // chunks grow so that about 320 rows pass in each, of a list of at least
     // 2,048 (10,000 queries against 2M x 96, k = 100: the chunks and cuts of
     // growth 3, 4 and 6 took 6.35, 6.32 and 6.52 ms)
-    // Few queries, whose chunks are short of work, grow faster.
+    // Up to 8 times at small k (1M x 96, k = 10, growth 4 / 8 / 16 / 32: 65 queries 242 / 207 / 218 /
+    // 229 us, 1,000 queries 480 / 456 / 469 / 466, 10,000 queries 3,052 / 2,997 / 3,122 / 3,204), and 32
+    // for few queries, whose chunks are short of work (one query 232 / 204 / 200 / 190 us, 16
+    // queries 239 / 214 / 219 / 206; at 64 the two are even: 224 and 227).
     const size_t growth = std::clamp<size_t>(1 + 320 / k, 2, nq <= 64 ? 32 : 8);
     for (size_t q0 = 0; q0 < nq; q0 += QB) {
         const int nb = static_cast<int>(std::min(QB, nq - q0));
