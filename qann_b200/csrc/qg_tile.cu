@@ -71,6 +71,7 @@ struct TileArgs {
     int kblocks;         // 64-element K blocks of the padded rows
     int ksteps;          // 16-element MMA steps covering d
     int mtiles, ntiles, group_n;
+    int ctas;            // at most so many CTAs, or 0
     int scout;           // nearest: tiles of each group first read for their bounds alone
     const float* xterm;      // per base row: its part of the lower bound (+inf: not to be returned), padded
                              // with +inf to whole tiles
@@ -1199,8 +1200,8 @@ template <int EPI, int MODE>
 void launch_epi(const CUtensorMap& tmA, const CUtensorMap& tmB, const TileArgs& a, cudaStream_t st) {
     allow_large_smem<k_tile<EPI, MODE>>();
     const int tiles = a.mtiles * (a.ntiles + a.scout);
-    k_tile<EPI, MODE><<<static_cast<unsigned>(std::min(tiles, sm_count())), tile_threads<EPI>(),
-                        tile_smem_bytes<EPI>(), st>>>(tmA, tmB, a);
+    const int ctas = std::min(tiles, a.ctas > 0 ? std::min(a.ctas, sm_count()) : sm_count());
+    k_tile<EPI, MODE><<<static_cast<unsigned>(ctas), tile_threads<EPI>(), tile_smem_bytes<EPI>(), st>>>(tmA, tmB, a);
     QG_LAUNCH_CHECK();
 }
 
@@ -1324,6 +1325,17 @@ void tile_store(const TileQueries& qs, const uint16_t* base_f16, size_t n, int d
     launch_tile<kStore>(tmA, tmB, a, st, may_tune, [] {}, [] {});
 }
 
+// The CTAs that may share a query tile of a nearest launch over ntiles base tiles.
+// Each of them appends records of its own: two warps' running minima over 2 ntiles / ctas
+// runs of 32 rows each set about ln(2 ntiles / ctas) + 0.6 records, and 256 fit a query's list. (64 to 512
+// queries against 16,384 rows spread over 74 to 128 CTAs a tile all overflowed:
+// adding 512 x 128 took 1.13 ms, on the exact tiles alone 1.01, and takes 0.62.)
+int nearest_ctas(int ntiles) {
+    int c = std::min(ntiles, 128);
+    while (c > 1 && 2 * c * (std::log(2.0 * ntiles / c) + 0.6) > 0.75 * kNearestCap) --c;
+    return c;
+}
+
 // One launch over every base row per block of queries: a lane of the epilogue
 // owns one query, keeps its smallest upper bound so far and appends the rows
 // whose lower bound is at most that. Rows in random order give about ln(n)
@@ -1377,6 +1389,7 @@ size_t tile_nearest(const float* q, const TileQueries& qs, const float* base_row
         const int nb = static_cast<int>(std::min(QB, nq - q0));
         a.nq = nb;
         a.mtiles = static_cast<int>(ceil_div(static_cast<size_t>(nb), BM));
+        a.ctas = std::min(a.mtiles, sm_count()) * nearest_ctas(a.ntiles);
         auto open = [&] {
             k_tile_open<<<blocks_of(nb), 256, 0, st>>>(qs.sq.get() + q0, qs.exps.get() + q0, nb, bound, base.amax.get(),
                                                        kNearestCap, qmul.get(), qslack.get(), thr.get(), count.get());
