@@ -286,7 +286,7 @@ void flat_candidates(const float* q_dev, size_t nq, const float* rows_dev, size_
 }
 
 // Flat results in (score, slot) order with ids and the exact score, which its
-// key gives back but for the sign of a zero (formed again).
+// key gives back but for the sign of a zero or a NaN (formed again).
 __global__ void k_finalize_flat(const float* __restrict__ q, int dim, const float* __restrict__ rows,
                                 const uint64_t* __restrict__ key, const uint32_t* __restrict__ slot, int k, bool ip,
                                 const int64_t* __restrict__ labels, bool cosine, int64_t* __restrict__ out_ids,
@@ -300,7 +300,7 @@ __global__ void k_finalize_flat(const float* __restrict__ q, int dim, const floa
         return;
     }
     float d = key_float(static_cast<uint32_t>(key[t] >> 32));
-    if (d == 0.0f) d = exact_score(rows + static_cast<size_t>(s) * dim, q + (t / k) * dim, dim, ip);
+    if (!(fabsf(d) > 0.0f)) d = exact_score(rows + static_cast<size_t>(s) * dim, q + (t / k) * dim, dim, ip);
     out_ids[t] = labels ? labels[s] : static_cast<int64_t>(s);
     out_d[t] = cosine ? __fmul_rn(d, 0.5f) : d;
 }

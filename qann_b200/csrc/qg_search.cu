@@ -703,7 +703,7 @@ __global__ void __launch_bounds__(256) k_refine_scores(const float* __restrict__
 }
 
 // The kq best of a query's kp scored candidates, one block per query. The
-// score is its key's, but for the sign of a zero (formed again). (A bitonic sort
+// score is its key's, but for the sign of a zero or a NaN (formed again). (A bitonic sort
 // of 1,024 keys by 1,024 threads took 35 us for 256 queries, ranks over
 // register-sorted runs of 200 keys 99 us for 10,000 queries; 12 and 52 now.)
 __global__ void __launch_bounds__(1024) k_refine_select(const float* __restrict__ q, int dim,
@@ -722,8 +722,9 @@ __global__ void __launch_bounds__(1024) k_refine_select(const float* __restrict_
         const size_t o = static_cast<size_t>(qi) * k + rank;
         const uint32_t slot = static_cast<uint32_t>(key);
         float d = key_float(static_cast<uint32_t>(key >> 32));
-        // float_key_eq0 folded -0 into +0, and the reference returns the value itself
-        if (d == 0.0f) d = exact_score(qv, rows + static_cast<size_t>(slot) * dim, dim, ip);
+        // float_key_eq0 folded -0 into +0, and the reference returns the value itself; a
+        // NaN of an inner product is formed again too (its key holds the other sign)
+        if (!(fabsf(d) > 0.0f)) d = exact_score(qv, rows + static_cast<size_t>(slot) * dim, dim, ip);
         out_ids[o] = labels ? labels[slot] : static_cast<int64_t>(slot);
         out_d[o] = cosine ? __fmul_rn(d, 0.5f) : d;
     };
