@@ -211,8 +211,8 @@ __global__ void k_pick_u32(const uint32_t* __restrict__ src, size_t n, uint32_t*
 
 // Whether m queries whose candidate lists overflowed are swept (tile_topk) before
 // the exact tiles, or always in mode 2: from 2e8 multiply-adds of those, which come in tiles
-// of 16 queries. Rows of 96 dims, each nearer than the ones before it, k = 10, batch_query
-// exact / swept: one query over 65,000 (1e8) 295 / 313 and 130,000 rows (2e8) 503 / 340 us;
+// of 16 queries. Rows of 96 dims, each nearer than the ones before it, k = 10, thresholds
+// from the first of them (so that lists overflow), batch_query exact / swept: one query over 65,000 (1e8) 295 / 313 and 130,000 rows (2e8) 503 / 340 us;
 // 64 queries over 30,000 (1.8e8) 279 / 375 and 65,000 (4e8) 454 / 366 us.
 static bool sweeps_pay(size_t m, size_t n, int dim) {
     return g_tensor_filter.load() == 2 || static_cast<double>(std::max<size_t>(m, 16)) * double(n) * dim >= 2e8;

@@ -674,11 +674,15 @@ struct TileBound {
 
 // Each base row's part of the lower bound (+inf for rows that are refused,
 // -inf for extreme ones, which always pass), and per 32 rows the slack that
-// takes the smallest lower bound among them to an upper bound.
+// takes the smallest lower bound among them to an upper bound. The terms and norms of
+// the sample (rows step apart) once more, side by side: read in place by every query's
+// block they cost 10,000 queries 250 us. With `apart` the sample's rows are not to be
+// returned again.
 __global__ void __launch_bounds__(256) k_tile_terms(const float* __restrict__ sq, size_t n, size_t npad, TileBound b,
                                                     const uint64_t* __restrict__ allow,
                                                     const uint64_t* __restrict__ deny, float* __restrict__ xterm,
-                                                    float* __restrict__ run_slack) {
+                                                    float* __restrict__ run_slack, uint32_t step, uint32_t sampled, bool apart,
+                                                    float* __restrict__ sample_term, float* __restrict__ sample_sq) {
     const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     constexpr float kInf = __builtin_huge_valf();
     float s = 0.0f;
@@ -687,7 +691,14 @@ __global__ void __launch_bounds__(256) k_tile_terms(const float* __restrict__ sq
         const bool ex = tile_extreme(x2);
         const bool refused = (allow && !((allow[i >> 6] >> (i & 63)) & 1ull)) ||
                              (deny && ((deny[i >> 6] >> (i & 63)) & 1ull));
-        xterm[i] = refused ? kInf : ex ? -kInf : __fmul_rn(b.xc, x2);
+        const float term = refused ? kInf : ex ? -kInf : __fmul_rn(b.xc, x2);
+        const uint32_t j = static_cast<uint32_t>(i) / step;
+        const bool in = j < sampled && j * step == i;
+        xterm[i] = in && apart ? kInf : term;
+        if (in) {
+            sample_term[j] = term;
+            sample_sq[j] = x2;
+        }
         s = ex ? kInf : __fmul_ru(b.c2, x2);
     } else if (i < npad) {
         xterm[i] = kInf;
@@ -772,9 +783,12 @@ __global__ void __launch_bounds__(256) k_tile_pick(const float* __restrict__ q, 
 
 // ---- the k nearest ----------------------------------------------------------------
 //
-// The first rows' products are stored, and each query's threshold is the k-th
-// smallest upper bound among them; the rows below it open its candidate list.
-// The rows after them are taken in chunks of growing size: the engine appends
+// The products of a sample of the rows, at equal steps, are stored, and each
+// query's threshold is the k-th smallest upper bound among them. (The first rows
+// would do as well where rows are stored in random order. Where they are not, by
+// cluster or by time, what is near would meet a threshold from rows that are far.)
+// The sample's rows below it open the query's candidate list; the other
+// rows are taken in chunks of growing size: the engine appends
 // the rows whose lower bound is below the threshold, and a cut per query takes
 // the threshold to the k-th smallest upper bound of all its candidates and
 // drops those above. Only what is left at the end is scored exactly.
@@ -884,13 +898,13 @@ __device__ __forceinline__ float upper_bound(float lb, float x2, float c2, float
 // The key of a threshold that no row passes, extreme ones included.
 constexpr uint32_t kClosedKey = 0xFFFFFFFFu;   // (a NaN)
 
-// One block per query over the stored products of the first ncols rows: its
-// threshold and the rows at or below it, or for a sweep the threshold alone. lbs, ub:
-// ncols floats of shared memory each.
+// One block per query over the stored products of a sample of ncols rows: its
+// threshold, and with `step` (0: the threshold alone) the rows at or below it, which
+// are `step` apart. lbs, ub: ncols floats of shared memory each.
 __global__ void __launch_bounds__(256) k_tile_seed(const float* __restrict__ acc, size_t ld, int ncols,
                                                    const float* __restrict__ xterm, const float* __restrict__ sq,
                                                    float c2, const float* __restrict__ qmul,
-                                                   const float* __restrict__ qslack, int k, int cap, bool sweep,
+                                                   const float* __restrict__ qslack, int k, int cap, uint32_t step,
                                                    uint32_t* __restrict__ thr_key, uint32_t* __restrict__ count,
                                                    uint2* __restrict__ cand) {
     extern __shared__ __align__(16) uint8_t sm_raw[];
@@ -916,7 +930,7 @@ __global__ void __launch_bounds__(256) k_tile_seed(const float* __restrict__ acc
     }
     __syncthreads();
     const float T = cut_threshold(ub, ncols, k, s);
-    if (sweep) {
+    if (step == 0) {
         if (threadIdx.x == 0) thr_key[qi] = float_key(T);
         return;
     }
@@ -930,12 +944,12 @@ __global__ void __launch_bounds__(256) k_tile_seed(const float* __restrict__ acc
         if (lane == 0) at = atomicAdd(&s.count, __popc(in));
         at = __shfl_sync(0xffffffffu, at, 0) + __popc(in & ((1u << lane) - 1));
         if (lb <= T && at < cap)
-            cand[static_cast<size_t>(qi) * cap + at] = make_uint2(__float_as_uint(lb), static_cast<uint32_t>(j));
+            cand[static_cast<size_t>(qi) * cap + at] = make_uint2(__float_as_uint(lb), static_cast<uint32_t>(j) * step);
     }
     __syncthreads();
     if (threadIdx.x == 0) {
         count[qi] = static_cast<uint32_t>(s.count);
-        thr_key[qi] = s.count > cap ? kClosedKey : float_key(T);   // (an overflowed list takes no more)
+        thr_key[qi] = float_key(T);
     }
 }
 
@@ -966,51 +980,53 @@ __device__ __forceinline__ int cut_list(uint2* list, float* ub, int n, int k, co
     return kept;
 }
 
-// Whether a sweep would settle a list that overflowed in the chunk from row `from`
-// on, under the threshold of key `was` and with cnt rows counted: its list holds what
-// passes (`ahead` times cnt by the last row), or the entries taken from the chunk give a
-// lower threshold (not so where distances tie), or too few were taken to tell. By one
-// block; list, ub: cap entries of shared memory each. (Not inlined: it is rare, and
-// its registers cost the kernels that call it 3 to 8 % of their callers' time.)
-__device__ __noinline__ bool worth_a_sweep(const uint2* mine, uint32_t cnt, float ahead, uint32_t from, uint32_t was,
-                                           uint2* list, float* ub, int cap, int k, const float* __restrict__ sq, float c2,
-                                           float qs, CutScratch& s) {
-    if (static_cast<float>(cnt) * ahead <= static_cast<float>(kMaxCap)) return true;   // (block-uniform)
-    int fresh = 0;
-    for (int i0 = 0; i0 < cap; i0 += blockDim.x) {   // (whole rounds: cap is a power of two)
-        const uint2 e = mine[i0 + threadIdx.x];
-        list[i0 + threadIdx.x] = e;
-        fresh += __syncthreads_count(e.y >= from);
+// The stored products of the sample, and what bounds take from its rows.
+struct Sample {
+    const float* acc;   // per query, ld apart
+    size_t ld;
+    int ncols;
+    const float *xterm, *sq;
+};
+
+// Whether a sweep would settle a list that overflowed under the threshold of key
+// `was`, with cnt rows counted: its list holds them all, or a lower threshold is to be
+// had, from the entries the list did take or from the nearest row of the sample (not
+// so where more rows tie than any list holds). By one block; list, ub: cap entries of
+// shared memory each. (Not inlined: it is rare, and its registers cost the kernels
+// around it 3 to 8 % of the search.)
+__device__ __noinline__ bool worth_a_sweep(const uint2* mine, uint32_t cnt, uint32_t was, const float* acc, Sample sm,
+                                           float qmul, float qs, uint2* list, float* ub, int cap, int k,
+                                           const float* __restrict__ sq, float c2, CutScratch& s) {
+    if (cnt <= static_cast<uint32_t>(kMaxCap)) return true;   // (block-uniform)
+    const float T = key_float(was);
+    bool lower = false;
+    for (int j = threadIdx.x; j < sm.ncols; j += blockDim.x) {
+        const float lb = __fmaf_rn(-qmul, acc[j], sm.xterm[j]);
+        lower |= lb <= kOpen && upper_bound(lb, sm.sq[j], c2, qs) < T;
     }
-    if (fresh < k) return true;
-    float T;
-    cut_list(list, ub, cap, k, sq, c2, qs, s, T);
-    return float_key(T) < was;
+    if (__syncthreads_or(lower)) return true;
+    for (int i = threadIdx.x; i < cap; i += blockDim.x) list[i] = mine[i];
+    __syncthreads();
+    float best;
+    cut_list(list, ub, cap, k, sq, c2, qs, s, best);
+    return best < T;
 }
 
-// After a chunk, one block per query: the list cut, its threshold lowered.
-__global__ void __launch_bounds__(128, 16) k_tile_cut(const float* __restrict__ sq, float c2,
-                                                  const float* __restrict__ qslack, int k, int cap, float ahead, uint32_t from,
+// After a chunk, one block per query: the list cut, its threshold lowered (not while the
+// list holds fewer than k rows).
+__global__ void __launch_bounds__(128) k_tile_cut(const float* __restrict__ sq, float c2,
+                                                  const float* __restrict__ qslack, int k, int cap,
                                                   uint32_t* __restrict__ thr_key, uint32_t* __restrict__ count,
                                                   uint2* __restrict__ cand) {
     extern __shared__ __align__(16) uint8_t sm_raw[];
     __shared__ CutScratch s;
     const int qi = blockIdx.x;
     const uint32_t cnt = count[qi], was = thr_key[qi];
-    if (was == kClosedKey) return;   // overflowed before
+    if (cnt > static_cast<uint32_t>(cap)) return;   // overflowed: only counted on
     const int n = static_cast<int>(cnt);
     uint2* list = reinterpret_cast<uint2*>(sm_raw);
     float* ub = reinterpret_cast<float*>(list + cap);
     uint2* mine = cand + static_cast<size_t>(qi) * cap;
-    if (cnt > static_cast<uint32_t>(cap)) {   // overflowed: it takes no more
-        const bool sweep = worth_a_sweep(mine, cnt, ahead, from, was, list, ub, cap, k, sq, c2, qslack[qi], s);
-        __syncthreads();   // (count and threshold are read)
-        if (threadIdx.x == 0) {
-            thr_key[qi] = kClosedKey;
-            if (!sweep) count[qi] = kGivenUp;
-        }
-        return;
-    }
     for (int i = threadIdx.x; i < n; i += blockDim.x) list[i] = mine[i];
     __syncthreads();
     float T;
@@ -1018,7 +1034,7 @@ __global__ void __launch_bounds__(128, 16) k_tile_cut(const float* __restrict__ 
     for (int i = threadIdx.x; i < kept; i += blockDim.x) mine[i] = list[i];
     if (threadIdx.x == 0) {
         count[qi] = static_cast<uint32_t>(kept);
-        thr_key[qi] = float_key(T);
+        thr_key[qi] = min(was, float_key(T));
     }
 }
 
@@ -1064,8 +1080,9 @@ __global__ void __launch_bounds__(256, 6) k_tile_finish(const float* __restrict_
                                                      bool ip, const float* __restrict__ sq, float c2,
                                                      const float* __restrict__ qslack, int k, int cap,
                                                      const uint32_t* __restrict__ count,
-                                                     const uint32_t* __restrict__ thr_key, uint32_t from,
-                                                     const uint2* __restrict__ cand, uint32_t first,
+                                                     const uint32_t* __restrict__ thr_key,
+                                                     const uint2* __restrict__ cand, Sample sample,
+                                                     const float* __restrict__ qmul, uint32_t first,
                                                      uint64_t* __restrict__ out_key, uint32_t* __restrict__ out_slot,
                                                      uint32_t* __restrict__ redo, uint32_t redo_end,
                                                      uint32_t* __restrict__ nredo) {
@@ -1078,9 +1095,9 @@ __global__ void __launch_bounds__(256, 6) k_tile_finish(const float* __restrict_
     float* ub = reinterpret_cast<float*>(list + cap);
     const uint2* mine = cand + static_cast<size_t>(qi) * cap;
     if (cnt > static_cast<uint32_t>(cap)) {   // to the front of redo[] to be swept, to its end where that would not help
-        const uint32_t was = thr_key[qi];
-        const bool sweep = cnt != kGivenUp && (was == kClosedKey || worth_a_sweep(mine, cnt, 1.0f, from, was, list, ub, cap,
-                                                                                  k, sq, c2, qslack[qi], s));
+        const bool sweep =
+            cnt != kGivenUp && worth_a_sweep(mine, cnt, thr_key[qi], sample.acc + static_cast<size_t>(qi) * sample.ld,
+                                             sample, qmul[qi], qslack[qi], list, ub, cap, k, sq, c2, s);
         if (threadIdx.x == 0) {
             if (sweep) redo[atomicAdd(nredo, 1u)] = first + qi;
             else redo[redo_end - 1 - atomicAdd(nredo + 1, 1u)] = first + qi;
@@ -1170,11 +1187,12 @@ EncodeTiled encode_fn() {
     return fn;
 }
 
-// f16 rows (dpad elements, row stride dpad * 2 bytes) read as boxes of 64 x box_rows, 128-byte swizzle.
-CUtensorMap make_map(const void* ptr, size_t rows, int dpad, int box_rows) {
+// f16 rows (dpad elements, row stride dpad * 2 bytes, or `step` such rows) read as boxes of 64 x box_rows,
+// 128-byte swizzle.
+CUtensorMap make_map(const void* ptr, size_t rows, int dpad, int box_rows, size_t step = 1) {
     CUtensorMap m;
     const cuuint64_t dims[2] = {static_cast<cuuint64_t>(dpad), static_cast<cuuint64_t>(rows)};
-    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(dpad) * 2};
+    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(dpad) * 2 * step};
     const cuuint32_t box[2] = {static_cast<cuuint32_t>(KA), static_cast<cuuint32_t>(box_rows)};
     const cuuint32_t estr[2] = {1, 1};
     const CUresult r = encode_fn()(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(ptr), dims, strides, box,
@@ -1352,7 +1370,7 @@ size_t tile_nearest(const float* q, const TileQueries& qs, const float* base_row
     const size_t npad = ceil_div(n, BN) * BN;
     DevBuf<float> xterm(npad, st), run_slack(npad / 32, st);
     k_tile_terms<<<blocks_of(npad), 256, 0, st>>>(base.sq.get(), n, npad, bound, nullptr, nullptr,
-                                                   xterm.get(), run_slack.get());
+                                                   xterm.get(), run_slack.get(), 1, 0, false, nullptr, nullptr);
     QG_LAUNCH_CHECK();
     const size_t QB = 131072;   // queries per block: 268 MB of candidate lists
     const size_t qb = std::min(QB, nq);
@@ -1431,17 +1449,21 @@ TileRedo tile_topk(const float* q, const TileQueries& qs, const float* base_rows
     require(n >= 1 && n < (size_t{1} << 31) && nq < (size_t{1} << 31), "too many rows for the tensor-core path",
             kUnsupported);
     require(k <= kTileMaxK, "k too large for the tensor-core path", kUnsupported);
-    const TileBound bound(d, ip);
-    const size_t npad = ceil_div(n, BN) * BN;
-    DevBuf<float> xterm(npad, st), run_slack(npad / 32, st);
-    k_tile_terms<<<blocks_of(npad), 256, 0, st>>>(base.sq.get(), n, npad, bound, allow, deny, xterm.get(),
-                                                   run_slack.get());
-    QG_LAUNCH_CHECK();
     // the candidate list: about 8 times what is wanted, so that a chunk of rows
     // far from their average order does not overflow it
-    const int cap = sweep ? kMaxCap : std::clamp(next_pow2(static_cast<int>(8 * k)), 2048, kMaxCap);
-    // the seed: enough rows that the first chunk's threshold lets few pass
+    // (few queries take the most there is: rows stored in an order overflow it less)
+    const int cap = sweep || nq <= 64 ? kMaxCap : std::clamp(next_pow2(static_cast<int>(8 * k)), 2048, kMaxCap);
+    // the sample: enough rows that the first chunk's threshold lets few pass
     const size_t seed = std::min<size_t>(n, std::clamp<size_t>(ceil_div(16 * k, BN) * BN, 2048, 8192));
+    const size_t step = n / seed;
+    const TileBound bound(d, ip);
+    const size_t npad = ceil_div(n, BN) * BN;
+    DevBuf<float> xterm(npad, st), run_slack(npad / 32, st), sample_term(seed, st), sample_sq(seed, st);
+    k_tile_terms<<<blocks_of(npad), 256, 0, st>>>(base.sq.get(), n, npad, bound, allow, deny, xterm.get(),
+                                                   run_slack.get(), static_cast<uint32_t>(step),
+                                                   static_cast<uint32_t>(seed), !sweep, sample_term.get(),
+                                                   sample_sq.get());
+    QG_LAUNCH_CHECK();
     const size_t ld = ceil_div(seed, 4) * 4;
     // queries per block: the lists within 512 MB, the stored products within 256 MB
     const size_t QB = std::min<size_t>({(size_t{512} << 20) / (cap * 8), (size_t{256} << 20) / (ld * 4), nq});
@@ -1467,6 +1489,7 @@ TileRedo tile_topk(const float* q, const TileQueries& qs, const float* base_rows
     a.store = acc.get();
     a.ld = ld;
     const CUtensorMap tmB = make_map(base.f16.get(), n, base.dpad, BN);
+    const CUtensorMap tmS = make_map(base.f16.get(), seed, base.dpad, BN, step);
     const size_t seed_smem = seed * 8, cut_smem = static_cast<size_t>(cap) * 12;
     allow_large_smem<k_tile_seed>();
     allow_large_smem<k_tile_cut>();
@@ -1497,11 +1520,11 @@ TileRedo tile_topk(const float* q, const TileQueries& qs, const float* base_rows
         a.group_n = a.ntiles;
         {
             KernelTimer kt("mm_filter", st);
-            launch_tile<kStore>(tmA, tmB, a, st, /*may_tune=*/false, [] {}, [] {});
+            launch_tile<kStore>(tmA, tmS, a, st, /*may_tune=*/false, [] {}, [] {});
         }
-        k_tile_seed<<<nb, 256, seed_smem, st>>>(acc.get(), ld, static_cast<int>(seed), xterm.get(), base.sq.get(),
-                                                bound.c2, qmul.get(), qslack.get(), static_cast<int>(k), cap, sweep,
-                                                thr.get(), count.get(), cand.get());
+        k_tile_seed<<<nb, 256, seed_smem, st>>>(acc.get(), ld, static_cast<int>(seed), sample_term.get(), sample_sq.get(),
+                                                bound.c2, qmul.get(), qslack.get(), static_cast<int>(k), cap,
+                                                sweep ? 0u : static_cast<uint32_t>(step), thr.get(), count.get(), cand.get());
         QG_LAUNCH_CHECK();
         for (int left = kSweeps; sweep && left > 0; --left) {
             for (size_t n0 = 0; n0 < n; n0 += kMaxChunkRows) {
@@ -1520,8 +1543,8 @@ TileRedo tile_topk(const float* q, const TileQueries& qs, const float* base_rows
             QG_CUDA(cudaStreamSynchronize(st));
             if (open == 0) break;
         }
-        for (size_t n0 = sweep ? n : seed; n0 < n;) {
-            const size_t n1 = std::min(n, std::min(n0 * growth, n0 + kMaxChunkRows));
+        for (size_t n0 = sweep || seed == n ? n : 0; n0 < n;) {
+            const size_t n1 = std::min({n, (n0 + seed) * growth - seed, n0 + kMaxChunkRows});   // (the sample counts)
             a.n0 = static_cast<int>(n0);
             a.ntiles = static_cast<int>(ceil_div(n1 - n0, BN));
             a.group_n = 16;
@@ -1540,14 +1563,15 @@ TileRedo tile_topk(const float* q, const TileQueries& qs, const float* base_rows
             n0 = n1;
             if (n0 == n) break;
             k_tile_cut<<<nb, 128, cut_smem, st>>>(base.sq.get(), bound.c2, qslack.get(), static_cast<int>(k), cap,
-                                                  static_cast<float>(n) / static_cast<float>(n0), static_cast<uint32_t>(a.n0),
                                                   thr.get(), count.get(), cand.get());
             QG_LAUNCH_CHECK();
         }
         auto finish = [&](auto kernel) {
             kernel<<<nb, 256, cut_smem, st>>>(q + q0 * d, d, base_rows, ip, base.sq.get(), bound.c2, qslack.get(),
-                                              static_cast<int>(k), cap, count.get(), thr.get(), static_cast<uint32_t>(a.n0),
-                                              cand.get(), static_cast<uint32_t>(q0), out_key + q0 * k, out_slot + q0 * k, redo.get(),
+                                              static_cast<int>(k), cap, count.get(), thr.get(), cand.get(),
+                                              Sample{acc.get(), ld, static_cast<int>(seed), sample_term.get(),
+                                                     sample_sq.get()},
+                                              qmul.get(), static_cast<uint32_t>(q0), out_key + q0 * k, out_slot + q0 * k, redo.get(),
                                               static_cast<uint32_t>(nq), nredo);
             QG_LAUNCH_CHECK();
         };

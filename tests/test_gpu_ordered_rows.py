@@ -101,3 +101,20 @@ def test_rows_past_one_launch():
     idx.add(x)
     q = rng.normal(size=(3, d)).astype(np.float32)
     both(lambda: idx.batch_query(q, 30))
+
+
+@pytest.mark.parametrize("k,seed", [(10, 2048), (200, 3200), (700, 8192)])
+@pytest.mark.parametrize("d", [20, 136])
+def test_around_the_sample(k, seed, d):
+    """Row counts around one, two and three times the sample, whose step changes there."""
+    rng = np.random.default_rng(seed + d)
+    for n in [m * seed + e for m in (1, 2, 3) for e in (-1, 0, 1, 129)]:
+        x = rng.normal(size=(n, d)).astype(np.float32)
+        x = x[np.argsort(x[:, 0])]
+        q = rng.normal(size=(67, d)).astype(np.float32)
+        for metric in (qb.Metric.L2, qb.Metric.InnerProduct):
+            idx = qb.FlatIndex(d, metric=metric)
+            idx.add(x)
+            idx.remove(np.arange(0, n, 7))
+            for nq in (1, 67):
+                both(lambda: idx.batch_query(q[:nq], k))
