@@ -614,7 +614,7 @@ bool cosine_ip_wins(const float* x, size_t n, int dim, const uint32_t* assign, c
     const size_t smem = static_cast<size_t>(m_pad) * 16 * (1 + kPickWarps) +
                         sizeof(float) * (static_cast<size_t>(dim) * (1 + kPickWarps) + static_cast<size_t>(m) * kPickWarps);
     require(smem <= 200 * 1024, "the cosine scoring decision supports dim and m up to about 4096", kUnsupported);
-    if (smem > 48 * 1024) allow_large_smem<k_pick_score>();
+    allow_large_smem<k_pick_score>();   // (its static arrays count towards the 48 KB that need no leave)
     k_pick_score<<<static_cast<unsigned>(nq), 32 * kPickWarps, smem, st>>>(
         x, n, dim, static_cast<int>(nq), centers, yt, m, sd, codes.get(), scores.get(), nlist, off.get(),
         members.get(), cut.get(), cap, ke.get(), kp.get(), kl.get(), count.get());

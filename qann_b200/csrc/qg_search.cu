@@ -398,8 +398,7 @@ void select_rows(const float* scores, size_t ld, int nrows, int ncols, int P, ui
     const size_t base = static_cast<size_t>(next_pow2(P)) * 16;
     const bool staged = few && base + static_cast<size_t>(ncols) * 4 <= 160 * 1024;
     const size_t smem = base + (staged ? static_cast<size_t>(ncols) * 4 : 0);
-    if (smem > 48 * 1024)
-        allow_large_smem<k_select_rows>();
+    allow_large_smem<k_select_rows>();   // (its static arrays count towards the 48 KB that need no leave)
     KernelTimer kt("select_rows", st);
     k_select_rows<<<nrows, few ? 1024 : 256, smem, st>>>(scores, ld, ncols, P, allow, deny, col_base, eq0, staged,
                                                           out_col, out_score);

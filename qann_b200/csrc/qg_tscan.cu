@@ -636,7 +636,7 @@ void tensor_scan_candidates(const IvfView& v, int nq, int P, int kp, const uint3
     DevBuf<uint32_t> redo(nq, st), nredo(1, st);
     QG_CUDA(cudaMemsetAsync(nredo.get(), 0, sizeof(uint32_t), st));
     const size_t fsmem = static_cast<size_t>(kp + cap) * 8;
-    if (fsmem > 48 * 1024) allow_large_smem<k_tscan_final>();
+    allow_large_smem<k_tscan_final>();   // (its static arrays count towards the 48 KB that need no leave)
     {
         KernelTimer kt("tscan_final", st);
         k_tscan_final<<<static_cast<unsigned>(nq), 256, fsmem, st>>>(v, P, probe, push.get(), key0, cand.get(),
